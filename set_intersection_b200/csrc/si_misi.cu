@@ -17,7 +17,8 @@
 //    smaller partners y are streamed from global memory against it.  The work
 //    is sum over pairs of min(|a|, |b|) probes instead of |a| + |b|.
 //  * Plan on the device: each side's sets are sorted by size, descending
-//    (radix sort of (size, index) keys), so the partners of a row form a
+//    (ranked by counting, or a radix sort of (size, index) keys for large
+//    collections), so the partners of a row form a
 //    suffix of the other side's sorted list; prefix sums of the sorted sizes
 //    number the partners' elements, and every row's suffix is cut into work
 //    items of equal element volume (a large partner may span items).
@@ -55,7 +56,10 @@ constexpr uint64_t kMinItemWork = 131072;  // partner elements per work item, at
 constexpr uint32_t kLaneCol = 64;          // partner pieces below this size are probed by one lane each
 constexpr uint64_t kMinSlice = 4096;       // partner elements per slice a warp takes, at least
 constexpr uint32_t kEmpty = 0xffffffffu;
-constexpr size_t kMisiHeader = 256;        // [0..16) error words, [16] u32 ticket
+constexpr size_t kMisiHeader = 256;        // [0..16) error words, then:
+constexpr size_t kMisiTicket = 16;         // u32 ticket of the probe kernel
+constexpr size_t kMisiPlanDone = 36;       // u32 CTAs of the order kernel that finished
+constexpr size_t kMisiTotals = 40;         // u64[2] elements of side A and of side B
 
 // Partner elements of one work item of a row whose set has `size` elements:
 // staging the set (rebuilt for every item of its row) costs at most 1/64 of
@@ -66,6 +70,14 @@ constexpr uint64_t kItemPerElement = 64;
 __host__ __device__ inline uint64_t item_unit(uint64_t size) {
     return kItemPerElement * size > kMinItemWork ? kItemPerElement * size : kMinItemWork;
 }
+
+// Up to this many sets the plan ranks them by comparing every two (two
+// kernels and a memset); more are sorted (CUB, 13 launches and more).  Plan of
+// 1000 sets: 15 us against 40, of 8192: 48-56 against 120-131, of 16384: 115
+// against 143.  The comparisons grow with the square of the sets.
+constexpr uint32_t kRankRows = 16384;
+constexpr int kRankBits = 15;  // rank in the low bits of an accumulator, sum of sizes above: 46 + 15 bits
+constexpr uint32_t kRankTile = 256;
 
 __host__ __device__ constexpr size_t misi_smem(int tech) {
     return tech == SI_TECH_BITMAP ? kBitmapBits / 8 : tech == SI_TECH_HI ? kHashTable * 4 : kSortedChunk * 4;
@@ -80,7 +92,7 @@ struct MisiLayout {
     uint32_t nA = 0, nB = 0, rows = 0;
     bool self = true;
     size_t off_keys_in = 0, off_keys = 0, off_sizes = 0, off_P = 0, off_cs = 0, off_nseg = 0, off_items = 0,
-           off_cub = 0, cub_bytes = 0, total = 0;
+           off_cub = 0, cub_bytes = 0, off_acc = 0, total = 0;
 };
 
 // Sort key of a set: size descending, then local index ascending.
@@ -117,11 +129,20 @@ MisiLayout misi_layout(si_set_range A, si_set_range B) {
     L.cub_bytes = align_up(std::max(sort_bytes, scan_bytes), 256);
     L.off_cub = o;
     o += L.cub_bytes;
+    L.off_acc = o;  // the ranks' accumulators
+    o = align_up(o + (n <= kRankRows ? n * 16 : 0), 256);
     L.total = o;
     return L;
 }
 
 // ------------------------------------------------------------------ plan --
+// Sum over the warp's active lanes (a prefix of the warp), in lane 0.
+__device__ __forceinline__ uint64_t warp_sum_active(uint32_t v) {
+    const uint32_t m = __activemask();
+    const uint64_t lo = __reduce_add_sync(m, v & 0xffffu), hi = __reduce_add_sync(m, v >> 16);
+    return lo + (hi << 16);
+}
+
 __global__ void misi_keys_kernel(const uint64_t* __restrict__ off, uint32_t a_start, uint32_t nA, uint32_t b_start,
                                  uint32_t nB, uint64_t* __restrict__ keys, uint32_t* err) {
     const uint32_t n = nA + nB;
@@ -196,6 +217,150 @@ __global__ void misi_rows_kernel(const uint64_t* __restrict__ keys, uint32_t nA,
         const uint64_t unit = item_unit(size);
         nseg[r] = work ? (work + unit - 1) / unit : 0;
     }
+}
+
+// The plan of small collections in two kernels.  Every set i compares itself
+// with all others: own[i] = (sets of its side before it in the sorted order,
+// the sum of their sizes), other[i] = the same over the other side's sets that
+// are no partners of row i.  Both halves travel in one 64-bit atomic add.
+// CTA (x, y): sets [256 x, 256 x + 256) against sets [256 y, 256 y + 256).
+__global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint64_t* __restrict__ off, uint32_t a_start,
+                                                              uint32_t nA, uint32_t b_start, uint32_t nB,
+                                                              unsigned long long* __restrict__ own,
+                                                              unsigned long long* __restrict__ other,
+                                                              unsigned char* header) {
+    __shared__ uint32_t s_size[kRankTile];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t n = nA + nB, tid = threadIdx.x;
+    auto set_id = [&](uint32_t i) { return i < nA ? a_start + i : b_start + (i - nA); };
+    auto size_of = [&](uint32_t i) {
+        const uint64_t size = off[set_id(i) + 1] - off[set_id(i)];
+        if (size > 0xffffffffull) record_error(reinterpret_cast<uint32_t*>(header), SI_ERR_INVALID_INPUT, 40, set_id(i));
+        return static_cast<uint32_t>(size);
+    };
+    const uint32_t j0 = blockIdx.y * kRankTile, tile = min(kRankTile, n - j0);
+    s_size[tid] = tid < tile ? size_of(j0 + tid) : 0u;
+    __syncthreads();
+    const uint32_t i = blockIdx.x * kRankTile + tid;
+    if (i >= n) return;
+    const uint32_t size = size_of(i);
+    const bool iA = i < nA;
+    uint32_t before = 0, larger = 0;
+    uint64_t before_sum = 0, larger_sum = 0;
+    if (j0 + tile <= nA || j0 >= nA) {  // one side's sets only
+        // sets as large come before it when they are earlier sets of its side, or when i is a B set
+        const bool same = (j0 < nA) == iA, earlier = j0 + kRankTile <= blockIdx.x * kRankTile;
+        uint32_t c = 0;
+        uint64_t sum = 0;
+        if (same && j0 == blockIdx.x * kRankTile) {
+            for (uint32_t t = 0; t < tile; ++t) {
+                const uint32_t sj = s_size[t];
+                const bool b = sj > size || (sj == size && t < tid);
+                c += b;
+                sum += b ? sj : 0u;
+            }
+        } else if (same ? earlier : !iA) {
+#pragma unroll 8
+            for (uint32_t t = 0; t < tile; ++t) {
+                const uint32_t sj = s_size[t];
+                c += sj >= size;
+                sum += sj >= size ? sj : 0u;
+            }
+        } else {
+#pragma unroll 8
+            for (uint32_t t = 0; t < tile; ++t) {
+                const uint32_t sj = s_size[t];
+                c += sj > size;
+                sum += sj > size ? sj : 0u;
+            }
+        }
+        (same ? before : larger) = c;
+        (same ? before_sum : larger_sum) = sum;
+    } else {
+        for (uint32_t t = 0; t < tile; ++t) {
+            const uint32_t j = j0 + t, sj = s_size[t];
+            const bool same = (j < nA) == iA, b = sj > size || (sj == size && (same ? j < i : !iA));
+            before += same && b;
+            before_sum += same && b ? sj : 0u;
+            larger += !same && b;
+            larger_sum += !same && b ? sj : 0u;
+        }
+    }
+    if (before) atomicAdd(own + i, (before_sum << kRankBits) | before);
+    if (larger) atomicAdd(other + i, (larger_sum << kRankBits) | larger);
+    if (blockIdx.y == 0) {
+        const uint64_t sumA = warp_sum_active(iA ? size : 0u), sumB = warp_sum_active(iA ? 0u : size);
+        if ((tid & 31) == 0) {
+            unsigned long long* totals = reinterpret_cast<unsigned long long*>(header + kMisiTotals);
+            if (sumA) atomicAdd(totals, sumA);
+            if (sumB) atomicAdd(totals + 1, sumB);
+        }
+    }
+}
+
+// Writes the sorted keys, the prefix sums, every row's first partner and its
+// number of work items; the last CTA to finish scans those into items.
+constexpr int kOrderThreads = 256;
+__global__ void __launch_bounds__(kOrderThreads) misi_order_kernel(
+    const uint64_t* __restrict__ off, uint32_t a_start, uint32_t nA, uint32_t b_start, uint32_t nB, bool self,
+    const unsigned long long* __restrict__ own, const unsigned long long* __restrict__ other,
+    uint64_t* __restrict__ keys, uint64_t* __restrict__ P, uint32_t* __restrict__ cs, uint64_t* __restrict__ nseg,
+    uint64_t* __restrict__ items, unsigned char* header) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the ranks
+    __shared__ uint64_t s_warp[kOrderThreads / 32];
+    __shared__ uint32_t s_last;
+    const uint32_t n = nA + nB, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t* totals = reinterpret_cast<const uint64_t*>(header + kMisiTotals);
+    const uint32_t i = blockIdx.x * kOrderThreads + tid;
+    if (i < n) {
+        const bool iA = i < nA;
+        const uint32_t local = iA ? i : i - nA, id = (iA ? a_start : b_start) + local;
+        const uint32_t size = static_cast<uint32_t>(off[id + 1] - off[id]);
+        const uint32_t mask = (1u << kRankBits) - 1;
+        const uint32_t rank = static_cast<uint32_t>(own[i]) & mask;
+        const uint64_t sum = own[i] >> kRankBits;
+        const uint32_t row = iA ? rank : nA + rank;
+        uint64_t* Ps = iA ? P : P + nA + 1;
+        keys[row] = size_key(size, local);
+        Ps[rank] = sum;
+        if (rank + 1 == (iA ? nA : nB)) Ps[rank + 1] = sum + size;
+        // partners: the sets after it of its own side, or the other side's from the first no larger one
+        const uint32_t c = self ? rank + 1 : static_cast<uint32_t>(other[i]) & mask;
+        const uint64_t work = self ? totals[0] - sum - size : totals[iA ? 1 : 0] - (other[i] >> kRankBits);
+        cs[row] = c;
+        const uint64_t unit = item_unit(size);
+        nseg[row] = work ? (work + unit - 1) / unit : 0;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        __threadfence();
+        s_last = atomicAdd(reinterpret_cast<uint32_t*>(header + kMisiPlanDone), 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const uint32_t per = (n + kOrderThreads - 1) / kOrderThreads;
+    const uint32_t r0 = min(n, tid * per), r1 = min(n, r0 + per);
+    uint64_t sum = 0;
+    for (uint32_t r = r0; r < r1; ++r) sum += __ldcg(nseg + r);
+    uint64_t incl = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint64_t t = __shfl_up_sync(kFullMask, incl, d);
+        if (static_cast<int>(lane) >= d) incl += t;
+    }
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint64_t o = incl - sum, all = 0;
+    for (uint32_t w = 0; w < kOrderThreads / 32; ++w) {
+        o += w < warp ? s_warp[w] : 0ull;
+        all += s_warp[w];
+    }
+    for (uint32_t r = r0; r < r1; ++r) {
+        items[r] = o;
+        o += __ldcg(nseg + r);
+    }
+    if (tid == 0) items[n] = all;
 }
 
 // ---------------------------------------------------------------- probes --
@@ -497,7 +662,6 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     const MisiLayout L = misi_layout(A, B);
     if (ws_bytes < L.total) return SI_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* w = static_cast<unsigned char*>(ws);
-    uint32_t* err = reinterpret_cast<uint32_t*>(w);
     SI_CUDA_TRY(cudaMemsetAsync(w, 0, kMisiHeader, stream));
     // every count of the tile starts at zero (pairs with an empty set are never visited)
     const uint64_t n_counts = L.self ? (L.nA < 2 ? 0 : tri_idx(stride, L.nA - 2, L.nA - 1) + 1)
@@ -513,10 +677,25 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     uint64_t* nseg = reinterpret_cast<uint64_t*>(w + L.off_nseg);
     uint64_t* items = reinterpret_cast<uint64_t*>(w + L.off_items);
     void* cub_tmp = w + L.off_cub;
-    const unsigned g = static_cast<unsigned>(std::min<uint64_t>((L.rows + 255) / 256 + 1, uint64_t(sm_count()) * 8));
-    {
+    if (L.rows <= kRankRows) {
         PhaseTimer timer("misi_plan", stream);
-        misi_keys_kernel<<<g, 256, 0, stream>>>(d_offsets, A.start, L.nA, B.start, L.nB, keys_in, err);
+        unsigned long long* own = reinterpret_cast<unsigned long long*>(w + L.off_acc);
+        unsigned long long* other = own + L.rows;
+        SI_CUDA_TRY(cudaMemsetAsync(own, 0, size_t(L.rows) * 16, stream));
+        const unsigned tiles = (L.rows + kRankTile - 1) / kRankTile;
+        misi_rank_kernel<<<dim3(tiles, tiles), kRankTile, 0, stream>>>(d_offsets, A.start, L.nA, B.start, L.nB, own,
+                                                                       other, w);
+        SI_LAUNCH_CHECK("misi_rank_kernel");
+        const si_status st = launch_dependent(
+            misi_order_kernel, dim3((L.rows + kOrderThreads - 1) / kOrderThreads), dim3(kOrderThreads), 0, stream,
+            d_offsets, A.start, L.nA, B.start, L.nB, L.self, static_cast<const unsigned long long*>(own),
+            static_cast<const unsigned long long*>(other), keys, P, cs, nseg, items, w);
+        if (st != SI_OK) return st;
+    } else {
+        const unsigned g = static_cast<unsigned>(std::min<uint64_t>((L.rows + 255) / 256 + 1, uint64_t(sm_count()) * 8));
+        PhaseTimer timer("misi_plan", stream);
+        misi_keys_kernel<<<g, 256, 0, stream>>>(d_offsets, A.start, L.nA, B.start, L.nB, keys_in,
+                                                reinterpret_cast<uint32_t*>(w));
         SI_LAUNCH_CHECK("misi_keys_kernel");
         size_t tmp = L.cub_bytes;
         SI_CUDA_TRY(cub::DeviceRadixSort::SortKeys(cub_tmp, tmp, keys_in, keys, static_cast<int>(L.nA), 0, 64, stream));
@@ -557,7 +736,7 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     prm.cs = cs;
     prm.items = items;
     prm.counts = d_counts;
-    prm.ticket = reinterpret_cast<uint32_t*>(w + 16);
+    prm.ticket = reinterpret_cast<uint32_t*>(w + kMisiTicket);
 
     auto launch = [&](auto kernel, int tech) -> si_status {
         const size_t smem = misi_smem(tech);

@@ -143,3 +143,32 @@ def test_powerlaw_config_8192_sets(cuda):
     want = oracle.all_pairs(el, off, k, 1 << 20, "std", threads=os.cpu_count() or 1)
     assert want.size == k * (k - 1) // 2
     np.testing.assert_array_equal(ref, want)
+
+@pytest.mark.parametrize("k", [2, 31, 255, 256, 257, 511, 513])
+@pytest.mark.parametrize("sizes", ["equal", "mixed", "tiny"])
+def test_plan_orders_ties_and_tiles(cuda, k, sizes):
+    """The plan's ranks at the edges of its 256-set tiles: sets of equal sizes,
+    empty sets, self-join tiles and cross tiles cut at and off tile edges."""
+    rng = np.random.default_rng(k)
+    n = {"equal": np.full(k, 20), "mixed": rng.integers(0, 60, k), "tiny": rng.integers(0, 3, k)}[sizes]
+    sets = [np.sort(rng.choice(500, size=s, replace=False)).astype(np.uint32) for s in n]
+    ds, col = from_sets(sets, universe=500)
+    want = oracle.all_pairs(ds.elements, ds.offsets, k, 500, "std")
+    full = np.zeros((k, k), np.uint32)
+    full[np.triu_indices(k, 1)] = want
+    for tech in ("bitmap", "hi"):
+        np.testing.assert_array_equal(run(col, tech), want)
+        for h in sorted({1, k // 2, min(256, k - 1), k - 1}):
+            np.testing.assert_array_equal(run(col, tech, (0, h), (h, k)).reshape(h, k - h), full[:h, h:])
+
+
+@pytest.mark.parametrize("rows", [16384, 16385])
+def test_plan_of_the_most_ranked_sets(cuda, rows):
+    """A cross tile of one set against many, at and past the ranked plan's limit."""
+    rng = np.random.default_rng(rows)
+    sets = [np.arange(0, 300, 2, dtype=np.uint32)]
+    sets += [np.unique(rng.integers(0, 300, 1 + i % 7)).astype(np.uint32) for i in range(rows - 1)]
+    ds, col = from_sets(sets, universe=300)
+    want = np.array([np.count_nonzero(s % 2 == 0) for s in sets[1:]], np.uint32)
+    for tech in ("bitmap", "obs"):
+        np.testing.assert_array_equal(run(col, tech, (0, 1), (1, rows)), want)
