@@ -206,6 +206,10 @@ si_status si_validate_sorted(const uint32_t* d_x, uint64_t n, uint32_t* d_flag, 
  * src/hi.cu:295-420 (warpBasedHI / blockBasedHI) and
  * src/bitmap_dynamic.cu:240-319.  t: IP, OBS, HI, BITMAP or AUTO (= BITMAP).
  * MM and BITMAP_NAIVE are served by si_misi_dense (single-tile run only).
+ * BITMAP on 32 sets or more keeps a value-major bit matrix of up to 512 sets
+ * in the workspace (64 MiB of it) and counts each partner against all of them
+ * at once, when the values of the tile's sets span at most 2^20 (512 sets at a
+ * time), 2^21 (256) or 2^22 (128); wider collections are probed pair by pair.
  */
 typedef struct si_set_range { uint32_t start, end; } si_set_range;
 size_t si_misi_workspace_size(si_set_range A, si_set_range B, si_technique t);
@@ -316,7 +320,7 @@ si_status si_misi_dense(const uint32_t* d_elements, const uint64_t* d_offsets, u
  * "sisi_split", "sisi_tile", and for BITMAP with elements "sisi_scan",
  * "sisi_copy"; dense all pairs "mm_incidence", "mm_gemm",
  * "naive_bitmaps", "naive_popcount"; all pairs of a tile "misi_plan",
- * "misi_probe"; single pair by search "obs_sample", "obs_search" (with the
+ * "misi_slab" (bitmap), "misi_probe"; single pair by search "obs_sample", "obs_search" (with the
  * offsets scan when elements are written), "obs_compact"; batched pairs
  * "batch_plan", "batch_count".  The events come from a pool that
  * si_timer_reset refills, so a timed launch costs two event records.

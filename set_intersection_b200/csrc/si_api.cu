@@ -205,7 +205,7 @@ si_status si_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t 
 size_t si_misi_workspace_size(si_set_range A, si_set_range B, si_technique t) {
     if (t != SI_TECH_IP && t != SI_TECH_OBS && t != SI_TECH_HI && t != SI_TECH_BITMAP && t != SI_TECH_AUTO) return 0;
     if (A.end < A.start || B.end < B.start) return 0;
-    return si::misi_workspace_size(A, B);
+    return si::misi_workspace_size(A, B, t == SI_TECH_AUTO ? SI_TECH_BITMAP : t);
 }
 
 si_status si_misi(const uint32_t* d_elements, const uint64_t* d_offsets, si_set_range A, si_set_range B,

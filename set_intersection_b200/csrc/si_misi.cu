@@ -39,6 +39,7 @@
 
 #include "si_device.cuh"
 #include "si_internal.h"
+#include "si_misi_slab.cuh"
 #include "si_stream.cuh"
 
 namespace si {
@@ -56,10 +57,7 @@ constexpr uint64_t kMinItemWork = 131072;  // partner elements per work item, at
 constexpr uint32_t kLaneCol = 64;          // partner pieces below this size are probed by one lane each
 constexpr uint64_t kMinSlice = 4096;       // partner elements per slice a warp takes, at least
 constexpr uint32_t kEmpty = 0xffffffffu;
-constexpr size_t kMisiHeader = 256;        // [0..16) error words, then:
-constexpr size_t kMisiTicket = 16;         // u32 ticket of the probe kernel
-constexpr size_t kMisiPlanDone = 36;       // u32 CTAs of the order kernel that finished
-constexpr size_t kMisiTotals = 40;         // u64[2] elements of side A and of side B
+constexpr size_t kMisiHeader = 256;        // [0..16) error words, then the words of si_misi_slab.cuh
 
 // Partner elements of one work item of a row whose set has `size` elements:
 // staging the set (rebuilt for every item of its row) costs at most 1/64 of
@@ -92,7 +90,7 @@ struct MisiLayout {
     uint32_t nA = 0, nB = 0, rows = 0;
     bool self = true;
     size_t off_keys_in = 0, off_keys = 0, off_sizes = 0, off_P = 0, off_cs = 0, off_nseg = 0, off_items = 0,
-           off_cub = 0, cub_bytes = 0, off_acc = 0, total = 0;
+           off_cub = 0, cub_bytes = 0, off_acc = 0, off_slab = 0, total = 0;
 };
 
 // Sort key of a set: size descending, then local index ascending.
@@ -100,7 +98,7 @@ __host__ __device__ inline uint64_t size_key(uint32_t size, uint32_t local) {
     return (uint64_t(0xffffffffu - size) << 32) | local;
 }
 
-MisiLayout misi_layout(si_set_range A, si_set_range B) {
+MisiLayout misi_layout(si_set_range A, si_set_range B, si_technique t) {
     MisiLayout L;
     L.self = A.start == B.start && A.end == B.end;
     L.nA = A.end - A.start;
@@ -131,6 +129,8 @@ MisiLayout misi_layout(si_set_range A, si_set_range B) {
     o += L.cub_bytes;
     L.off_acc = o;  // the ranks' accumulators
     o = align_up(o + (n <= kRankRows ? n * 16 : 0), 256);
+    L.off_slab = o;  // the bitmap technique's value-major matrix
+    if (t == SI_TECH_BITMAP && L.rows >= kSlabMinRows) o += kSlabBytes;
     L.total = o;
     return L;
 }
@@ -143,8 +143,11 @@ __device__ __forceinline__ uint64_t warp_sum_active(uint32_t v) {
     return lo + (hi << 16);
 }
 
-__global__ void misi_keys_kernel(const uint64_t* __restrict__ off, uint32_t a_start, uint32_t nA, uint32_t b_start,
-                                 uint32_t nB, uint64_t* __restrict__ keys, uint32_t* err) {
+// Sort keys of the sets, and the smallest and the largest value of all of them.
+__global__ void misi_keys_kernel(const uint32_t* __restrict__ el, const uint64_t* __restrict__ off, uint32_t a_start,
+                                 uint32_t nA, uint32_t b_start, uint32_t nB, uint64_t* __restrict__ keys,
+                                 unsigned char* header) {
+    uint32_t* err = reinterpret_cast<uint32_t*>(header);
     const uint32_t n = nA + nB;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const bool isA = i < nA;
@@ -153,6 +156,10 @@ __global__ void misi_keys_kernel(const uint64_t* __restrict__ off, uint32_t a_st
         const uint64_t size = off[id + 1] - off[id];
         if (size > 0xffffffffull) record_error(err, SI_ERR_INVALID_INPUT, 40, id);
         keys[i] = size_key(static_cast<uint32_t>(size), local);
+        if (size) {
+            atomicMax(reinterpret_cast<uint32_t*>(header + kMisiValueMin), ~__ldg(el + off[id]));
+            atomicMax(reinterpret_cast<uint32_t*>(header + kMisiValueMax), __ldg(el + off[id + 1] - 1));
+        }
     }
 }
 
@@ -224,7 +231,8 @@ __global__ void misi_rows_kernel(const uint64_t* __restrict__ keys, uint32_t nA,
 // the sum of their sizes), other[i] = the same over the other side's sets that
 // are no partners of row i.  Both halves travel in one 64-bit atomic add.
 // CTA (x, y): sets [256 x, 256 x + 256) against sets [256 y, 256 y + 256).
-__global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint64_t* __restrict__ off, uint32_t a_start,
+__global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint32_t* __restrict__ el,
+                                                              const uint64_t* __restrict__ off, uint32_t a_start,
                                                               uint32_t nA, uint32_t b_start, uint32_t nB,
                                                               unsigned long long* __restrict__ own,
                                                               unsigned long long* __restrict__ other,
@@ -290,10 +298,20 @@ __global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint64_t* __
     if (larger) atomicAdd(other + i, (larger_sum << kRankBits) | larger);
     if (blockIdx.y == 0) {
         const uint64_t sumA = warp_sum_active(iA ? size : 0u), sumB = warp_sum_active(iA ? 0u : size);
+        uint32_t vmin = 0, vmax = 0;
+        if (size) {
+            vmin = ~__ldg(el + off[set_id(i)]);
+            vmax = __ldg(el + off[set_id(i) + 1] - 1);
+        }
+        const uint32_t m = __activemask();
+        vmin = __reduce_max_sync(m, vmin);
+        vmax = __reduce_max_sync(m, vmax);
         if ((tid & 31) == 0) {
             unsigned long long* totals = reinterpret_cast<unsigned long long*>(header + kMisiTotals);
             if (sumA) atomicAdd(totals, sumA);
             if (sumB) atomicAdd(totals + 1, sumB);
+            atomicMax(reinterpret_cast<uint32_t*>(header + kMisiValueMin), vmin);
+            atomicMax(reinterpret_cast<uint32_t*>(header + kMisiValueMax), vmax);
         }
     }
 }
@@ -376,6 +394,7 @@ struct MisiParams {
     const uint64_t* items;  // exclusive scan of nseg, rows + 1 entries
     uint32_t* counts;
     uint32_t* ticket;
+    const unsigned char* header;
 };
 
 __device__ __forceinline__ uint64_t lower_bound_u64(const uint64_t* x, uint64_t lo, uint64_t hi, uint64_t v) {
@@ -433,6 +452,12 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
     __shared__ uint32_t s_has_max;
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t rows = p.nA + p.nB;
+    if constexpr (kTech == SI_TECH_BITMAP) {
+        // counted by misi_slab_kernel when the values fit its matrix
+        const uint32_t vmin = ~*reinterpret_cast<const uint32_t*>(p.header + kMisiValueMin);
+        const uint32_t vmax = *reinterpret_cast<const uint32_t*>(p.header + kMisiValueMax);
+        if (vmax >= vmin && slab_words(rows, vmax - vmin)) return;
+    }
     const uint64_t n_items = p.items[rows];
 
     for (;;) {
@@ -654,12 +679,12 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
 
 }  // namespace
 
-size_t misi_workspace_size(si_set_range A, si_set_range B) { return misi_layout(A, B).total; }
+size_t misi_workspace_size(si_set_range A, si_set_range B, si_technique t) { return misi_layout(A, B, t).total; }
 
 si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_technique t, si_set_range A,
                     si_set_range B, uint64_t stride, uint32_t* d_counts, void* ws, size_t ws_bytes,
                     cudaStream_t stream) {
-    const MisiLayout L = misi_layout(A, B);
+    const MisiLayout L = misi_layout(A, B, t);
     if (ws_bytes < L.total) return SI_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* w = static_cast<unsigned char*>(ws);
     SI_CUDA_TRY(cudaMemsetAsync(w, 0, kMisiHeader, stream));
@@ -683,8 +708,8 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
         unsigned long long* other = own + L.rows;
         SI_CUDA_TRY(cudaMemsetAsync(own, 0, size_t(L.rows) * 16, stream));
         const unsigned tiles = (L.rows + kRankTile - 1) / kRankTile;
-        misi_rank_kernel<<<dim3(tiles, tiles), kRankTile, 0, stream>>>(d_offsets, A.start, L.nA, B.start, L.nB, own,
-                                                                       other, w);
+        misi_rank_kernel<<<dim3(tiles, tiles), kRankTile, 0, stream>>>(d_elements, d_offsets, A.start, L.nA, B.start,
+                                                                       L.nB, own, other, w);
         SI_LAUNCH_CHECK("misi_rank_kernel");
         const si_status st = launch_dependent(
             misi_order_kernel, dim3((L.rows + kOrderThreads - 1) / kOrderThreads), dim3(kOrderThreads), 0, stream,
@@ -694,8 +719,7 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     } else {
         const unsigned g = static_cast<unsigned>(std::min<uint64_t>((L.rows + 255) / 256 + 1, uint64_t(sm_count()) * 8));
         PhaseTimer timer("misi_plan", stream);
-        misi_keys_kernel<<<g, 256, 0, stream>>>(d_offsets, A.start, L.nA, B.start, L.nB, keys_in,
-                                                reinterpret_cast<uint32_t*>(w));
+        misi_keys_kernel<<<g, 256, 0, stream>>>(d_elements, d_offsets, A.start, L.nA, B.start, L.nB, keys_in, w);
         SI_LAUNCH_CHECK("misi_keys_kernel");
         size_t tmp = L.cub_bytes;
         SI_CUDA_TRY(cub::DeviceRadixSort::SortKeys(cub_tmp, tmp, keys_in, keys, static_cast<int>(L.nA), 0, 64, stream));
@@ -737,6 +761,27 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     prm.items = items;
     prm.counts = d_counts;
     prm.ticket = reinterpret_cast<uint32_t*>(w + kMisiTicket);
+    prm.header = w;
+
+    if (t == SI_TECH_BITMAP && L.rows >= kSlabMinRows) {
+        SlabParams sp;
+        sp.el = d_elements;
+        sp.off = d_offsets;
+        sp.a_start = A.start;
+        sp.b_start = B.start;
+        sp.nA = L.nA;
+        sp.nB = L.nB;
+        sp.self = L.self;
+        sp.stride = stride;
+        sp.keys = keys;
+        sp.P = P;
+        sp.cs = cs;
+        sp.counts = d_counts;
+        sp.header = w;
+        sp.table = reinterpret_cast<uint32_t*>(w + L.off_slab);
+        const si_status st = misi_slab(sp, stream);
+        if (st != SI_OK) return st;
+    }
 
     auto launch = [&](auto kernel, int tech) -> si_status {
         const size_t smem = misi_smem(tech);

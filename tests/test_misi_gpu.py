@@ -172,3 +172,54 @@ def test_plan_of_the_most_ranked_sets(cuda, rows):
     want = np.array([np.count_nonzero(s % 2 == 0) for s in sets[1:]], np.uint32)
     for tech in ("bitmap", "obs"):
         np.testing.assert_array_equal(run(col, tech, (0, 1), (1, rows)), want)
+
+
+@pytest.mark.parametrize("k,span", [
+    (32, 1000), (128, 1), (129, (1 << 21) + 30), (256, 4095), (257, (1 << 20) + 14), (257, (1 << 20) + 15),
+    (300, (1 << 21) + 30), (300, (1 << 21) + 31), (512, 40000), (513, 100), (600, (1 << 22) + 62),
+    (600, (1 << 22) + 63), (1100, 70000),
+])
+def test_value_matrix_edges(cuda, k, span):
+    """The bitmap technique's value-major matrix: row counts at the edges of
+    its entries and groups, value spans at the limits of each entry width (past
+    the last the probe kernel counts), values up to 2^32 - 1, partners longer
+    than a slice; self-join, cross tiles with few and many rows, a replayed graph."""
+    import torch
+    from set_intersection_b200 import api
+    rng = np.random.default_rng(k * 31 + span % 1000)
+    base = (1 << 32) - 1 - span
+    sizes = np.minimum(rng.integers(0, 40, k) * rng.integers(1, 12, k), span // 2 + 1)
+    sizes[:3] = [min(span // 3 + 1, 9001), 0, min(span // 2 + 1, 4097)]
+    sets = [np.unique(rng.integers(0, span + 1, n)) if n else np.zeros(0, np.int64) for n in sizes]
+    sets[0] = np.union1d(sets[0], [0, span])  # the span is exact
+    sets = [(s + base).astype(np.uint32) for s in sets]
+    ds, col = from_sets(sets)
+    want = oracle.all_pairs(ds.elements, ds.offsets, k, ds.universe, "std")
+    ws = api.Workspace()
+    np.testing.assert_array_equal(run(col, "bitmap", ws=ws), want)
+    full = np.zeros((k, k), np.uint32)
+    full[np.triu_indices(k, 1)] = want
+    for h in (1, k // 2):
+        np.testing.assert_array_equal(run(col, "auto", (0, h), (h, k), ws=ws).reshape(h, k - h), full[:h, h:])
+    counts = torch.zeros(want.size, dtype=torch.int32, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        api.misi_into(col, counts, "bitmap", workspace=ws)
+    for _ in range(2):
+        counts.fill_(7)
+        g.replay()
+        np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint32), want)
+
+
+def test_cross_tile_with_many_groups_on_both_sides(cuda):
+    """Rows on both sides (more than eight 512-row groups each)."""
+    from set_intersection_b200 import api, generate
+    k, h = 9000, 4500
+    el, off = generate.powerlaw(41, k, 1, 300, 1.1, 1 << 14, 0.8)
+    col = collection(el, off, 1 << 14)
+    ws = api.Workspace()
+    got, want = run(col, "bitmap", (0, h), (h, k), ws=ws), run(col, "hi", (0, h), (h, k), ws=ws)
+    np.testing.assert_array_equal(got, want)
+    rows = np.random.default_rng(1).integers(0, h, 50)
+    ref = oracle.pairs(el, off, k, np.array([(a, h + b) for a in rows for b in range(0, k - h, 97)], np.uint32))
+    np.testing.assert_array_equal(got.reshape(h, k - h)[rows][:, ::97].ravel(), ref)
