@@ -206,10 +206,13 @@ si_status si_validate_sorted(const uint32_t* d_x, uint64_t n, uint32_t* d_flag, 
  * src/hi.cu:295-420 (warpBasedHI / blockBasedHI) and
  * src/bitmap_dynamic.cu:240-319.  t: IP, OBS, HI, BITMAP or AUTO (= BITMAP).
  * MM and BITMAP_NAIVE are served by si_misi_dense (single-tile run only).
- * BITMAP on 32 sets or more keeps a value-major bit matrix of up to 512 sets
- * in the workspace (64 MiB of it) and counts each partner against all of them
- * at once, when the values of the tile's sets span at most 2^20 (512 sets at a
- * time), 2^21 (256) or 2^22 (128); wider collections are probed pair by pair.
+ * BITMAP and HI on 32 sets or more keep a value-major bit matrix of up to 512
+ * sets in the workspace (64 MiB, HI 72) and count each partner against all of
+ * them at once: BITMAP when the values of the tile's sets span at most 2^20
+ * (512 sets at a time), 2^21 (256) or 2^22 (128); HI, whose matrix is indexed
+ * by a hash table, unless a set holds more than 2^20 elements of a wider span.
+ * Other tiles, and up to 128 (HI: 1024) sets of at most 64 elements, are probed
+ * pair by pair.
  */
 typedef struct si_set_range { uint32_t start, end; } si_set_range;
 size_t si_misi_workspace_size(si_set_range A, si_set_range B, si_technique t);

@@ -129,8 +129,9 @@ MisiLayout misi_layout(si_set_range A, si_set_range B, si_technique t) {
     o += L.cub_bytes;
     L.off_acc = o;  // the ranks' accumulators
     o = align_up(o + (n <= kRankRows ? n * 16 : 0), 256);
-    L.off_slab = o;  // the bitmap technique's value-major matrix
-    if (t == SI_TECH_BITMAP && L.rows >= kSlabMinRows) o += kSlabBytes;
+    L.off_slab = o;  // the value-major matrix of techniques bitmap and hi
+    if ((t == SI_TECH_BITMAP || t == SI_TECH_HI) && L.rows >= kSlabMinRows) o += kSlabBytes;
+    if (t == SI_TECH_HI && L.rows >= kSlabMinRows) o += kSlabKeyBytes;
     L.total = o;
     return L;
 }
@@ -452,11 +453,9 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
     __shared__ uint32_t s_has_max;
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t rows = p.nA + p.nB;
-    if constexpr (kTech == SI_TECH_BITMAP) {
-        // counted by misi_slab_kernel when the values fit its matrix
-        const uint32_t vmin = ~*reinterpret_cast<const uint32_t*>(p.header + kMisiValueMin);
-        const uint32_t vmax = *reinterpret_cast<const uint32_t*>(p.header + kMisiValueMax);
-        if (vmax >= vmin && slab_words(rows, vmax - vmin)) return;
+    if constexpr (kTech == SI_TECH_BITMAP || kTech == SI_TECH_HI) {
+        // counted by misi_slab_kernel when its matrix holds the values
+        if (slab_plan_of(kTech == SI_TECH_HI, p.nA, p.nB, p.header, p.P).words) return;
     }
     const uint64_t n_items = p.items[rows];
 
@@ -763,7 +762,7 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     prm.ticket = reinterpret_cast<uint32_t*>(w + kMisiTicket);
     prm.header = w;
 
-    if (t == SI_TECH_BITMAP && L.rows >= kSlabMinRows) {
+    if ((t == SI_TECH_BITMAP || t == SI_TECH_HI) && L.rows >= kSlabMinRows) {
         SlabParams sp;
         sp.el = d_elements;
         sp.off = d_offsets;
@@ -779,7 +778,8 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
         sp.counts = d_counts;
         sp.header = w;
         sp.table = reinterpret_cast<uint32_t*>(w + L.off_slab);
-        const si_status st = misi_slab(sp, stream);
+        sp.slots = reinterpret_cast<uint32_t*>(w + L.off_slab + kSlabBytes);
+        const si_status st = misi_slab(sp, t, stream);
         if (st != SI_OK) return st;
     }
 

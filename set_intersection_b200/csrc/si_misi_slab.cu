@@ -1,12 +1,16 @@
-// si_misi_slab.cu -- all pairs of a collection by bitmap, many rows at a time.
+// si_misi_slab.cu -- all pairs of a collection by bitmap or by hash, many rows
+// at a time.
 //
-// The reference gives a block one set's bitmap and probes it with one partner
-// after another (src/bitmap_dynamic.cu:279-319): one probe per element and
-// pair.  Here the bitmap of up to 512 rows (sets) is turned over: entry v of
-// the matrix holds one bit per row, set when the row's set holds value v.  One
-// 64-byte gather then probes an element of a partner against 512 rows at once,
-// and the hits of all rows are summed in vertical counters (bit planes, one
-// LOP3 sum and one LOP3 carry per adder for 32 rows).
+// The reference gives a block one set's bitmap or hash table and probes it
+// with one partner after another (src/bitmap_dynamic.cu:279-319, src/hi.cu:
+// 295-420): one probe per element and pair.  Here the bitmap of up to 512 rows
+// (sets) is turned over: entry v of the matrix holds one bit per row, set when
+// the row's set holds value v.  One 64-byte gather then probes an element of a
+// partner against 512 rows at once, and the hits of all rows are summed in
+// vertical counters (bit planes, one LOP3 sum and one LOP3 carry per adder for
+// 32 rows).  Technique hi finds a value's entry by hashing: one open-addressing
+// table holds the values of all the rows, a slot's entry their bits, so any
+// range of values fits and an element costs one lookup for all the rows.
 //
 // One cooperative launch walks the row groups, largest sets first.  Per group:
 //   build   every element of the group's rows sets its row's bit (red.or)
@@ -20,11 +24,12 @@
 // counts only against rows at least as large, so the elements read are the
 // smaller sets', as in the probe kernel.
 //
-// Power-law collection (8192 sets, 45.6 M elements, 2^20 values): the launch
-// takes 1.77 ms where the probe kernel takes 35.2 ms (builds 0.40 ms, bound by
-// the L2's atomics at 1.4e11 a second; probes 1.23 ms, bound by L2 gathers in
-// the first groups and by latency in the last; clears 0.14 ms).  64 sets of up
-// to 512 elements: 42 us a call against 62.
+// Power-law collection (8192 sets, 45.6 M elements, 2^20 values), bitmap: the
+// launch takes 1.88 ms where the probe kernel takes 35.2 ms (builds 0.38 ms,
+// bound by the L2's atomics at 1.4e11 a second; probes 1.35 ms, bound by L2
+// gathers in the first groups and by latency in the last; clears 0.15 ms).
+// Hash, a cross tile of 1500 x 1500 of such sets: 0.94 ms against 8.05 ms.
+// 64 sets of up to 512 elements: bitmap 46 us a call against 62, hash 60 and 62.
 #include <algorithm>
 
 #include "si_device.cuh"
@@ -90,12 +95,40 @@ __device__ __forceinline__ bool grid_barrier(uint32_t* arrived, uint32_t target,
     return *s_ok != 0;
 }
 
+// Where a value's entry is.  Bitmap: at the value's offset in the span.  Hash:
+// in the slot that linear probing finds it in.
+template <bool kHash>
+struct Entries {
+    uint32_t* slots;
+    uint32_t vmin, span, mask, shift;
+    __device__ __forceinline__ explicit Entries(const SlabParams& p, const SlabPlan& pl)
+        : slots(p.slots), vmin(pl.vmin), span(pl.span), mask(pl.slots - 1), shift(pl.shift) {}
+    __device__ __forceinline__ uint32_t zero() const { return kHash ? mask + 1 : span + 1; }
+    __device__ __forceinline__ uint32_t total() const { return kHash ? mask + 3 : span + 2; }
+    __device__ __forceinline__ uint32_t slot(uint32_t v) const { return (v * 0x9e3779b1u) >> shift; }
+    // What can be loaded ahead of find(): the value in v's first slot.
+    __device__ __forceinline__ uint32_t first(uint32_t v) const { return kHash ? slots[slot(v)] : 0u; }
+    // v's entry, the zero entry when it has none.
+    __device__ __forceinline__ uint32_t find(uint32_t v, uint32_t k) const {
+        if constexpr (!kHash) return min(v - vmin, span + 1);
+        if (v == kSlabEmpty) return mask + 2;
+        uint32_t h = slot(v);
+        while (k != v) {
+            if (k == kSlabEmpty) return mask + 1;
+            h = (h + 1) & mask;
+            k = slots[h];
+        }
+        return h;
+    }
+};
+
 // The group's rows [r0, r1) of one side: every element sets (kSet) or zeroes
 // its row's word in the matrix.  P: prefix sums of the side's sorted sizes.
-template <int E, bool kSet>
-__device__ __forceinline__ void group_elements(const SlabParams& p, const uint64_t* keys, const uint64_t* P,
-                                               uint32_t start, uint32_t r0, uint32_t r1, uint32_t vmin,
-                                               uint32_t span) {
+// Values outside the span, which only an unsorted set has, are left out (the
+// table's slots are as many as distinct values of the span could need).
+template <int E, bool kHash, bool kSet>
+__device__ __forceinline__ void group_elements(const SlabParams& p, const Entries<kHash>& en, const uint64_t* keys,
+                                               const uint64_t* P, uint32_t start, uint32_t r0, uint32_t r1) {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t e0 = P[r0], e1 = P[r1];
     const uint64_t nwarps = uint64_t(gridDim.x) * kSlabWarps;
@@ -111,11 +144,44 @@ __device__ __forceinline__ void group_elements(const SlabParams& p, const uint64
             constexpr uint32_t kLd = 8;  // loads in flight per lane
             for (uint32_t i = lane; i < n; i += 32 * kLd) {
                 uint32_t o[kLd];
-#pragma unroll
-                for (uint32_t u = 0; u < kLd; ++u) o[u] = i + 32 * u < n ? __ldg(x + i + 32 * u) - vmin : ~0u;
+                bool on[kLd];
 #pragma unroll
                 for (uint32_t u = 0; u < kLd; ++u) {
-                    if (o[u] > span) continue;  // past the end, or an unsorted set
+                    const uint32_t v = i + 32 * u < n ? __ldg(x + i + 32 * u) : en.vmin - 1;
+                    on[u] = i + 32 * u < n && v - en.vmin <= en.span;
+                    o[u] = kHash ? v : v - en.vmin;
+                }
+                if constexpr (kHash) {
+                    // every element's first slot is read, then claimed, before any goes on to its next
+                    uint32_t h[kLd], k[kLd];
+#pragma unroll
+                    for (uint32_t u = 0; u < kLd; ++u) {
+                        h[u] = en.slot(o[u]);
+                        k[u] = on[u] ? __ldcg(en.slots + h[u]) : 0u;
+                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < kLd; ++u)
+                        if (kSet && on[u] && k[u] == kSlabEmpty && o[u] != kSlabEmpty) {
+                            k[u] = atomicCAS(en.slots + h[u], kSlabEmpty, o[u]);
+                            if (k[u] == kSlabEmpty) k[u] = o[u];
+                        }
+#pragma unroll
+                    for (uint32_t u = 0; u < kLd; ++u) {
+                        while (on[u] && o[u] != kSlabEmpty && k[u] != o[u]) {
+                            if (!kSet && k[u] == kSlabEmpty) break;
+                            h[u] = (h[u] + 1) & en.mask;
+                            k[u] = __ldcg(en.slots + h[u]);
+                            if (kSet && k[u] == kSlabEmpty) {
+                                k[u] = atomicCAS(en.slots + h[u], kSlabEmpty, o[u]);
+                                if (k[u] == kSlabEmpty) k[u] = o[u];
+                            }
+                        }
+                        o[u] = o[u] == kSlabEmpty ? en.mask + 2 : h[u];
+                    }
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < kLd; ++u) {
+                    if (!on[u]) continue;
                     uint32_t* word = p.table + uint64_t(o[u]) * E + (bit >> 5);
                     if constexpr (kSet)
                         asm volatile("red.global.or.b32 [%0], %1;" ::"l"(word), "r"(1u << (bit & 31)) : "memory");
@@ -134,6 +200,13 @@ __device__ __forceinline__ void clear_table(const SlabParams& p, uint64_t entrie
     const uint64_t n = entries * (E / 4), stride = uint64_t(gridDim.x) * kSlabThreads;
     for (uint64_t i = uint64_t(blockIdx.x) * kSlabThreads + threadIdx.x; i < n; i += stride)
         t[i] = make_uint4(0u, 0u, 0u, 0u);
+}
+
+__device__ __forceinline__ void clear_slots(const SlabParams& p, uint32_t slots) {
+    uint4* t = reinterpret_cast<uint4*>(p.slots);
+    const uint32_t stride = gridDim.x * kSlabThreads;
+    for (uint32_t i = blockIdx.x * kSlabThreads + threadIdx.x; i < slots / 4; i += stride)
+        t[i] = make_uint4(kSlabEmpty, kSlabEmpty, kSlabEmpty, kSlabEmpty);
 }
 
 // (sum, carry) of three bits in every position.
@@ -175,9 +248,9 @@ __device__ __forceinline__ void add8(uint32_t (&pl)[NP][4], int w, const uint4 (
 // rounds ahead (2.5 and 2.7 ms), 24 warps per SM at 80 registers (1.74 ms:
 // spills), entries of 256 rows (1.72 against 1.59 ms) or of 128 rows, elements
 // loaded two rounds ahead (no change).
-template <int E, class Sink>
+template <int E, bool kHash, class Sink>
 __device__ __forceinline__ void count_partner(const uint32_t* __restrict__ y, uint32_t n, const uint32_t* table,
-                                              uint32_t vmin, uint32_t span, Sink sink) {
+                                              const Entries<kHash>& en, Sink sink) {
     constexpr int LPE = E / 4;        // lanes per element
     constexpr int NG = 32 / LPE;      // elements per step
     constexpr int kRound = 8 * NG;
@@ -192,26 +265,45 @@ __device__ __forceinline__ void count_partner(const uint32_t* __restrict__ y, ui
     for (int j = 0; j < NP; ++j)
 #pragma unroll
         for (int w = 0; w < 4; ++w) pl[j][w] = 0u;
-    // a round's elements, 32 to a load, as matrix entries; past the end the zero entry span + 1
-    uint32_t o[kLoads];
-    auto load = [&](uint32_t b) {
+    // a round's elements, 32 to a load: as entries (bitmap), or as values of
+    // which the first slots are read next (hash); past the end the zero entry
+    uint32_t v[kLoads], k1[kLoads], next[kLoads];
+    auto load = [&](uint32_t b, uint32_t (&r)[kLoads]) {
 #pragma unroll
         for (int k = 0; k < kLoads; ++k) {
             const uint32_t i = b + 32 * k + lane;
-            o[k] = i < n ? min(__ldg(y + i) - vmin, span + 1) : span + 1;
+            if constexpr (kHash) r[k] = i < n ? __ldg(y + i) : 0u;
+            else r[k] = i < n ? en.find(__ldg(y + i), 0u) : en.zero();
         }
     };
-    load(0);
+    auto look = [&]() {
+        if constexpr (kHash) {
+#pragma unroll
+            for (int k = 0; k < kLoads; ++k) k1[k] = en.first(v[k]);
+        }
+    };
+    load(0, v);
+    look();
+    if constexpr (kHash) load(kRound, next);
     for (uint32_t b = 0; b < n; b += kRound) {
         uint4 x[8];
 #pragma unroll
-        for (int k = 0; k < kLoads; ++k)
+        for (int k = 0; k < kLoads; ++k) {
+            const uint32_t o = !kHash ? v[k] : b + 32 * k + lane < n ? en.find(v[k], k1[k]) : en.zero();
 #pragma unroll
             for (int st = 0; st < LPE; ++st) {  // 32 elements, one per lane: LPE steps of NG of them
-                const uint32_t oe = LPE == 1 ? o[k] : __shfl_sync(kFullMask, o[k], st * NG + gi);
+                const uint32_t oe = LPE == 1 ? o : __shfl_sync(kFullMask, o, st * NG + gi);
                 x[k * LPE + st] = t4[uint64_t(oe) * LPE];
             }
-        load(b + kRound);
+        }
+        if constexpr (kHash) {  // the slots a round ahead, the elements two
+#pragma unroll
+            for (int k = 0; k < kLoads; ++k) v[k] = next[k];
+            look();
+            load(b + 2 * kRound, next);
+        } else {
+            load(b + kRound, v);
+        }
 #pragma unroll
         for (int w = 0; w < 4; ++w) add8<NP>(pl, w, x);
     }
@@ -282,20 +374,35 @@ __device__ __forceinline__ void count_partner(const uint32_t* __restrict__ y, ui
     }
 }
 
-template <int E>
-__device__ void slab_run(const SlabParams& p, uint32_t vmin, uint32_t span, GroupRows& rows, uint32_t* s_ok) {
+template <int E, bool kHash>
+__device__ void slab_run(const SlabParams& p, const SlabPlan& plan, GroupRows& rows, uint32_t* s_ok) {
     uint32_t* err = reinterpret_cast<uint32_t*>(p.header);
     uint32_t* ticket = reinterpret_cast<uint32_t*>(p.header + kMisiSlabTicket);
     uint32_t* arrived = reinterpret_cast<uint32_t*>(p.header + kMisiSlabBarrier);
     const uint32_t lane = threadIdx.x & 31;
     constexpr uint32_t R = 32 * E;
+    const Entries<kHash> en(p, plan);
+    // Hash: at most this many distinct values are in the slots at once.  With
+    // fewer in the whole span the slots are never emptied; otherwise they are
+    // when the groups since then could fill half of them.
+    const uint64_t cap = plan.slots / 2;
+    const bool bounded = !kHash || uint64_t(plan.span) + 1 <= cap;
+    uint64_t held = 0;  // elements inserted since the slots were emptied
     uint32_t epoch = 0;
-    clear_table<E>(p, uint64_t(span) + 2);
+    clear_table<E>(p, en.total());
+    if constexpr (kHash) clear_slots(p, plan.slots);
     if (!grid_barrier(arrived, gridDim.x * ++epoch, err, s_ok)) return;
     // Cross tile: with few groups on one side, only that side's sets are rows,
     // and all of the other side's sets partners
-    const uint32_t groupsA = (p.nA + R - 1) / R, groupsB = (p.nB + R - 1) / R;
+    auto groups = [&](uint32_t n, const uint64_t* P) {
+        const uint64_t g = (uint64_t(n) + R - 1) / R, h = bounded || n == 0 ? 0 : (P[n] + cap - 1) / cap;
+        return g > h ? g : h;
+    };
+    const uint64_t groupsA = groups(p.nA, p.P), groupsB = groups(p.nB, p.P + p.nA + 1);
     const bool all = !p.self && min(groupsA, groupsB) <= kSlabAllGroups;
+    bool dirty = false;  // the last group's bits are in the matrix: its rows [q0, q1) of the side before or this one
+    uint32_t q0 = 0, q1 = 0, q_start = 0;
+    const uint64_t *Kq = nullptr, *Pq = nullptr;
     for (int side = 0; side < (p.self ? 1 : 2); ++side) {
         const bool rowA = side == 0;
         if (all && rowA != (groupsA <= groupsB)) continue;
@@ -307,14 +414,37 @@ __device__ void slab_run(const SlabParams& p, uint32_t vmin, uint32_t span, Grou
         const uint32_t nt = partnersA ? p.nA : p.nB, t_start = partnersA ? p.a_start : p.b_start;
         const uint64_t* Kt = partnersA ? p.keys : p.keys + p.nA;
         const uint64_t* Pt = partnersA ? p.P : p.P + p.nA + 1;
-        for (uint32_t r0 = 0; r0 < nrows; r0 += R) {
-            const uint32_t r1 = min(r0 + R, nrows);
+        for (uint32_t r0 = 0, r1; r0 < nrows; r0 = r1) {
+            r1 = min(r0 + R, nrows);
+            if (!bounded) {  // the rows that fill half of the slots (one set does not)
+                const uint64_t full = Pr[r0] + cap;
+                r1 = static_cast<uint32_t>(warp_first_true(r0 + 1, r1 + 1, [&](uint64_t q) { return Pr[q] > full; })) - 1;
+                r1 = max(r1, r0 + 1);
+            }
             const uint32_t c0 = all ? 0u : cs[r0];
             // partner c takes [cost(c), cost(c + 1)): its elements, then kSlabOver
             auto cost = [&](uint64_t c) { return Pt[c] + uint64_t(kSlabOver) * c; };
             const uint64_t w0 = cost(c0), w1 = cost(nt);
             if (c0 >= nt || Pt[nt] == Pt[c0] || Pr[r1] == Pr[r0]) break;  // nor has any later group partners
-            group_elements<E, true>(p, Kr, Pr, row_start, r0, r1, vmin, span);
+            const uint64_t n_group = Pr[r1] - Pr[r0];
+            const bool empty_slots = !bounded && held + n_group > cap;
+            if (dirty) {  // back to zero: the group's words, unless the whole matrix is fewer stores
+                if (!empty_slots && (Pq[q1] - Pq[q0]) * 24 < uint64_t(en.total()) * E) {
+                    group_elements<E, kHash, false>(p, en, Kq, Pq, q_start, q0, q1);
+                } else {
+                    clear_table<E>(p, en.total());
+                    if (empty_slots) clear_slots(p, plan.slots);
+                }
+                if (!grid_barrier(arrived, gridDim.x * ++epoch, err, s_ok)) return;
+            }
+            held = empty_slots ? n_group : held + n_group;
+            group_elements<E, kHash, true>(p, en, Kr, Pr, row_start, r0, r1);
+            dirty = true;
+            q0 = r0;
+            q1 = r1;
+            q_start = row_start;
+            Kq = Kr;
+            Pq = Pr;
             if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
             for (uint32_t i = threadIdx.x; i < r1 - r0; i += kSlabThreads) {
                 const uint32_t id = static_cast<uint32_t>(Kr[r0 + i] & 0xffffffffu);
@@ -361,7 +491,7 @@ __device__ void slab_run(const SlabParams& p, uint32_t vmin, uint32_t span, Grou
                         const bool y_whole = (whole_mask >> l) & 1u;
                         const uint32_t cy = c + l;
                         count_partner<E>(p.el + __shfl_sync(kFullMask, y0, l), __shfl_sync(kFullMask, n, l), p.table,
-                                         vmin, span, [&](uint32_t row, uint32_t cnt) {
+                                         en, [&](uint32_t row, uint32_t cnt) {
                                              if (row >= r1 - r0 || rows.cs[row] > cy) return;  // a row smaller than y
                                              const uint32_t id = rows.id[row];
                                              const uint64_t idx = !p.self     ? rows.base[row] + ybase
@@ -375,43 +505,34 @@ __device__ void slab_run(const SlabParams& p, uint32_t vmin, uint32_t span, Grou
                 }
             }
             if (!grid_barrier(arrived, gridDim.x * ++epoch, err, s_ok)) return;
-            // back to zero: the group's words, unless the whole matrix is fewer stores
-            if (r1 < nrows || (!p.self && !all && rowA)) {
-                const uint64_t entries = uint64_t(span) + 2;
-                if ((Pr[r1] - Pr[r0]) * 24 < entries * E) group_elements<E, false>(p, Kr, Pr, row_start, r0, r1, vmin, span);
-                else clear_table<E>(p, entries);
-                if (!grid_barrier(arrived, gridDim.x * ++epoch, err, s_ok)) return;
-            }
         }
     }
 }
 
+template <bool kHash>
 __global__ void __launch_bounds__(kSlabThreads, kSlabCtasPerSm) misi_slab_kernel(SlabParams p) {
     __shared__ GroupRows rows;
     __shared__ uint32_t s_ok;
-    const uint32_t nmin = *reinterpret_cast<const uint32_t*>(p.header + kMisiValueMin);
-    const uint32_t vmax = *reinterpret_cast<const uint32_t*>(p.header + kMisiValueMax);
-    const uint32_t vmin = ~nmin;
-    if (vmax < vmin) return;  // every set is empty (or none is sorted): the probe kernel's part
-    const uint32_t span = vmax - vmin;
-    switch (slab_words(p.nA + p.nB, span)) {
-        case 16: slab_run<16>(p, vmin, span, rows, &s_ok); break;
-        case 8: slab_run<8>(p, vmin, span, rows, &s_ok); break;
-        case 4: slab_run<4>(p, vmin, span, rows, &s_ok); break;
+    const SlabPlan plan = slab_plan_of(kHash, p.nA, p.nB, p.header, p.P);
+    switch (plan.words) {
+        case 16: slab_run<16, kHash>(p, plan, rows, &s_ok); break;
+        case 8: slab_run<8, kHash>(p, plan, rows, &s_ok); break;
+        case 4: slab_run<4, kHash>(p, plan, rows, &s_ok); break;
         default: break;
     }
 }
 
 }  // namespace
 
-si_status misi_slab(const SlabParams& p, cudaStream_t stream) {
+si_status misi_slab(const SlabParams& p, si_technique t, cudaStream_t stream) {
+    const auto kernel = t == SI_TECH_HI ? misi_slab_kernel<true> : misi_slab_kernel<false>;
     int per_sm = 0;
-    SI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, misi_slab_kernel, kSlabThreads, 0));
+    SI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSlabThreads, 0));
     if (per_sm < 1) return SI_ERR_UNSUPPORTED;
     SlabParams prm = p;
     void* args[] = {&prm};
     PhaseTimer timer("misi_slab", stream);
-    SI_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(misi_slab_kernel),
+    SI_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel),
                                             dim3(static_cast<unsigned>(sm_count() * per_sm)), dim3(kSlabThreads), args,
                                             0, stream));
     return SI_OK;

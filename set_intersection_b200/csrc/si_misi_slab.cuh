@@ -21,6 +21,13 @@ constexpr size_t kSlabBytes = (kSlabValues + 16) * kSlabMaxWords * 4;
 // Collections of fewer rows keep the probe kernel: a group of rows fills less
 // than a quarter of the narrowest entry.
 constexpr uint32_t kSlabMinRows = 32;
+// So do small collections of small sets, where the matrix' clears and grid
+// barriers cost more than the probes: with sets of up to 32 elements, hash,
+// 32 sets 32 us a call by the probe kernel and 53 by the matrix, 200 sets 48 and
+// 62, 1000 sets 119 and 118-125; bitmap, 32 sets 32 and 42, 200 sets 48 and 48.
+constexpr uint32_t kSlabSmallSet = 64;
+constexpr uint32_t kSlabSmallRows = 128;
+constexpr uint32_t kSlabSmallRowsHash = 1024;
 
 // Words of the all-pairs header that the plan and both kernels use.
 constexpr size_t kMisiTicket = 16;      // u32 ticket of the probe kernel
@@ -31,15 +38,44 @@ constexpr size_t kMisiSlabBarrier = 32;  // u32 arrivals at the grid barrier
 constexpr size_t kMisiPlanDone = 36;     // u32 CTAs of the order kernel that finished
 constexpr size_t kMisiTotals = 40;       // u64[2] elements of side A and of side B
 
-// Words per entry for a collection of `rows` rows whose values lie in
-// [vmin, vmin + span], or 0 when the narrowest entries do not fit: then the
-// probe kernel counts.  Entry span + 1 is always zero (values out of range,
-// which only an unsorted set has, read it).
-__host__ __device__ inline uint32_t slab_words(uint32_t rows, uint32_t span) {
-    if (rows < kSlabMinRows) return 0;
+// Technique hi: the entries are the slots of an open-addressing hash table of
+// the values, twice as many as it can come to hold.
+constexpr uint32_t kSlabMaxSlots = 1u << 21;
+constexpr uint32_t kSlabMinSlots = 1u << 10;  // (slab_plan starts from it)
+constexpr size_t kSlabKeyBytes = size_t(kSlabMaxSlots) * 4;
+constexpr uint32_t kSlabEmpty = 0xffffffffu;  // an empty slot; that value has an entry of its own
+
+// How a tile is counted: words per entry (0: the probe kernel counts) and, for
+// technique hi, the table's slots.
+struct SlabPlan {
+    uint32_t words, slots, shift;  // slots = 2^(32 - shift)
+    uint32_t vmin, span;  // the values lie in [vmin, vmin + span]
+};
+
+// rows: of the tile; vmin, vmax: its smallest and largest value; largest: the
+// elements of its largest set; total: of its larger side.  A bitmap has an
+// entry per value of the span and one that is always zero (values out of
+// range, which only an unsorted set has, read it); a table of n slots has the
+// zero entry n and entry n + 1 for the value that marks empty slots.
+__host__ __device__ inline SlabPlan slab_plan(bool hash, uint32_t rows, uint32_t vmin, uint32_t vmax,
+                                              uint64_t largest, uint64_t total) {
+    SlabPlan pl = {0, 0, 0, vmin, vmax - vmin};
+    if (rows < kSlabMinRows || vmax < vmin) return pl;  // (vmax < vmin: every set is empty)
+    if (largest <= kSlabSmallSet && rows <= (hash ? kSlabSmallRowsHash : kSlabSmallRows)) return pl;
+    uint64_t entries = uint64_t(pl.span) + 2;
+    if (hash) {
+        // distinct values at once: all of them, or a group's (whose rows end before half of the slots is full)
+        const uint64_t distinct = total < uint64_t(pl.span) + 1 ? total : uint64_t(pl.span) + 1;
+        pl.slots = kSlabMinSlots;
+        pl.shift = 22;
+        for (; pl.slots < kSlabMaxSlots && pl.slots < 2 * distinct; --pl.shift) pl.slots *= 2;
+        if (pl.slots < 2 * distinct && largest > pl.slots / 2) return pl;
+        entries = uint64_t(pl.slots) + 2;
+    }
     uint32_t e = rows <= 128 ? 4u : rows <= 256 ? 8u : kSlabMaxWords;
-    while (e >= kSlabMinWords && (uint64_t(span) + 2) * e * 4 > kSlabBytes) e /= 2;
-    return e >= kSlabMinWords ? e : 0u;
+    while (e >= kSlabMinWords && entries * e * 4 > kSlabBytes) e /= 2;
+    if (e >= kSlabMinWords) pl.words = e;
+    return pl;
 }
 
 struct SlabParams {
@@ -54,8 +90,23 @@ struct SlabParams {
     uint32_t* counts;
     unsigned char* header;
     uint32_t* table;
+    uint32_t* slots;  // technique hi: the values in the slots
 };
 
-si_status misi_slab(const SlabParams& p, cudaStream_t stream);
+#ifdef __CUDACC__
+// The plan of a tile, from the all-pairs header and the sorted prefix sums.
+__device__ __forceinline__ SlabPlan slab_plan_of(bool hash, uint32_t nA, uint32_t nB, const unsigned char* header,
+                                                 const uint64_t* P) {
+    const uint64_t* PB = P + nA + 1;
+    const uint64_t largestA = nA ? P[1] : 0, largestB = nB ? PB[1] : 0;
+    const uint64_t totalA = nA ? P[nA] : 0, totalB = nB ? PB[nB] : 0;
+    return slab_plan(hash, nA + nB, ~*reinterpret_cast<const uint32_t*>(header + kMisiValueMin),
+                     *reinterpret_cast<const uint32_t*>(header + kMisiValueMax),
+                     largestA > largestB ? largestA : largestB, totalA > totalB ? totalA : totalB);
+}
+#endif
+
+// t: SI_TECH_BITMAP or SI_TECH_HI.
+si_status misi_slab(const SlabParams& p, si_technique t, cudaStream_t stream);
 
 }  // namespace si

@@ -223,3 +223,55 @@ def test_cross_tile_with_many_groups_on_both_sides(cuda):
     rows = np.random.default_rng(1).integers(0, h, 50)
     ref = oracle.pairs(el, off, k, np.array([(a, h + b) for a in rows for b in range(0, k - h, 97)], np.uint32))
     np.testing.assert_array_equal(got.reshape(h, k - h)[rows][:, ::97].ravel(), ref)
+
+
+@pytest.mark.parametrize("k,n_max,span", [
+    (32, 300, 1000), (128, 400, 1 << 31), (129, 3000, 5000), (257, 9000, (1 << 20) + 7), (300, 5000, 1 << 22),
+    (513, 70, 1 << 24), (1100, 600, 1 << 16),
+])
+def test_hash_matrix_edges(cuda, k, n_max, span):
+    """Technique hi's matrix: row counts at the edges of its entries and
+    groups, tables bounded by the elements and by the span, the value that
+    marks empty slots, partners longer than a slice; cross tiles; a replayed graph."""
+    import torch
+    from set_intersection_b200 import api
+    rng = np.random.default_rng(k)
+    sizes = rng.integers(0, n_max + 1, k)
+    sizes[:3] = [n_max, 0, max(1, n_max - 1)]
+    common = rng.integers(0, span, 50)
+    sets = [np.unique(np.concatenate([rng.integers(0, span, n), common[:n]])) for n in sizes]
+    sets = [np.union1d(s, [span]) if i % 3 == 0 else s for i, s in enumerate(sets)]
+    sets = [(s + ((1 << 32) - 1 - span)).astype(np.uint32) for s in sets]
+    ds, col = from_sets(sets)
+    want = oracle.all_pairs(ds.elements, ds.offsets, k, ds.universe, "std")
+    ws = api.Workspace()
+    np.testing.assert_array_equal(run(col, "hi", ws=ws), want)
+    full = np.zeros((k, k), np.uint32)
+    full[np.triu_indices(k, 1)] = want
+    for h in (1, k // 2):
+        np.testing.assert_array_equal(run(col, "hi", (0, h), (h, k), ws=ws).reshape(h, k - h), full[:h, h:])
+    counts = torch.zeros(want.size, dtype=torch.int32, device="cuda")
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        api.misi_into(col, counts, "hi", workspace=ws)
+    for _ in range(2):
+        counts.fill_(7)
+        g.replay()
+        np.testing.assert_array_equal(counts.cpu().numpy().view(np.uint32), want)
+
+
+@pytest.mark.parametrize("big", [0, 1 << 20, (1 << 20) + 5])
+def test_hash_groups_that_fill_the_slots(cuda, big):
+    """Sets over the whole 32-bit range, so many elements that a group's rows
+    end where half of the slots is full and the table is emptied between
+    groups; a set of half the slots, and one larger, which the probe kernel counts."""
+    rng = np.random.default_rng(big)
+    sets = [np.unique(rng.integers(0, 1 << 32, 60000, dtype=np.uint64)) for _ in range(48)]
+    sets = [np.union1d(s, sets[0][i:500 + i]) for i, s in enumerate(sets)]
+    sets = [np.union1d(s, [0xffffffff]) if i % 2 else s for i, s in enumerate(sets)]
+    if big:
+        s = np.unique(rng.integers(0, 1 << 32, big + 5000, dtype=np.uint64))
+        sets.append(s[:big])
+    ds, col = from_sets([s.astype(np.uint32) for s in sets])
+    want = oracle.all_pairs(ds.elements, ds.offsets, ds.cardinality, ds.universe, "std")
+    np.testing.assert_array_equal(run(col, "hi"), want)
