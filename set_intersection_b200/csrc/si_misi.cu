@@ -13,7 +13,8 @@
 //  * Every pair is handled by its LARGER set (ties: the A side, then the lower
 //    index): the larger set x is staged into shared memory once per work item
 //    -- as a bitmap of its values (bitmap), an open-addressing hash table (hi),
-//    or as the sorted array itself (obs: binary search; ip: merge) -- and the
+//    or as the sorted array itself with a table of value buckets (obs, ip:
+//    binary search of a bucket) -- and the
 //    smaller partners y are streamed from global memory against it.  The work
 //    is sum over pairs of min(|a|, |b|) probes instead of |a| + |b|.
 //  * Plan on the device: each side's sets are sorted by size, descending
@@ -45,28 +46,38 @@
 namespace si {
 namespace {
 
-constexpr int kMisiThreads = 1024;
-constexpr int kMisiWarps = kMisiThreads / 32;
+__host__ __device__ constexpr int misi_threads(int tech) { return tech == SI_TECH_OBS ? 512 : 1024; }
 constexpr uint32_t kBitmapBits = 1u << 20;             // bitmap: values per chunk (128 KiB)
 constexpr uint32_t kSortedChunk = 16384;               // obs / ip: elements per chunk (64 KiB)
+constexpr uint32_t kTopBuckets = 16384;                // obs / ip: buckets of the chunk's values, at most (32 KiB)
 constexpr uint32_t kHashChunk = 8192;                  // hi: elements per chunk
 constexpr uint32_t kHashTable = 2 * kHashChunk;        // slots (64 KiB), load factor <= 1/2
 constexpr uint32_t kHashBits = 14;
 static_assert(kHashTable == (1u << kHashBits), "hash table size");
-constexpr uint64_t kMinItemWork = 131072;  // partner elements per work item, at least
 constexpr uint32_t kLaneCol = 64;          // partner pieces below this size are probed by one lane each
-constexpr uint64_t kMinSlice = 4096;       // partner elements per slice a warp takes, at least
+// Partner elements per slice a warp takes, at least.  obs, ip: slices of 4096
+// leave warps idle on small rows (64 sets of up to 512 elements 78 us a call, 42
+// with slices of 512).
+__host__ __device__ constexpr uint64_t min_slice(int tech) { return tech == SI_TECH_OBS ? 512 : 4096; }
 constexpr uint32_t kEmpty = 0xffffffffu;
 constexpr size_t kMisiHeader = 256;        // [0..16) error words, then the words of si_misi_slab.cuh
 
-// Partner elements of one work item of a row whose set has `size` elements:
-// staging the set (rebuilt for every item of its row) costs at most 1/64 of
-// the item's probes.  Measured on the power-law collection (bitmap probe):
-// 62.8 ms with items of 4x the set, 43.6 with 16x, 39.1 with 32x, 36.8 with
-// 64x: the staging's inserts are shared atomics.
-constexpr uint64_t kItemPerElement = 64;
-__host__ __device__ inline uint64_t item_unit(uint64_t size) {
-    return kItemPerElement * size > kMinItemWork ? kItemPerElement * size : kMinItemWork;
+// Partner elements of one work item of a row whose set has `size` elements.
+// Bitmap, hi: staging the set (rebuilt for every item of its row) costs at most
+// 1/64 of the item's probes.  Measured on the power-law collection (bitmap
+// probe): 62.8 ms with items of 4x the set, 43.6 with 16x, 39.1 with 32x, 36.8
+// with 64x: the staging's inserts are shared atomics.  obs, ip: staging copies
+// the set and writes its bucket ends, and shorter items fill the tail: with
+// 8x (least 32768) / 16x / 32x, 1001 sets of up to 16384 elements over 2^18
+// values take 1.02 / 0.69 / 0.64 ms, 200 such sets over 2^20 167 / 180 / 271 us.
+struct ItemUnit {
+    uint32_t per_element, least;
+};
+__host__ __device__ constexpr ItemUnit item_rule(int tech) {
+    return tech == SI_TECH_OBS ? ItemUnit{16, 131072} : ItemUnit{64, 131072};
+}
+__host__ __device__ inline uint64_t item_unit(ItemUnit rule, uint64_t size) {
+    return max(rule.per_element * size, uint64_t(rule.least));
 }
 
 // Up to this many sets the plan ranks them by comparing every two (two
@@ -78,7 +89,9 @@ constexpr int kRankBits = 15;  // rank in the low bits of an accumulator, sum of
 constexpr uint32_t kRankTile = 256;
 
 __host__ __device__ constexpr size_t misi_smem(int tech) {
-    return tech == SI_TECH_BITMAP ? kBitmapBits / 8 : tech == SI_TECH_HI ? kHashTable * 4 : kSortedChunk * 4;
+    return tech == SI_TECH_BITMAP ? kBitmapBits / 8
+           : tech == SI_TECH_HI   ? kHashTable * 4
+                                  : (kSortedChunk + 4) * 4 + (kTopBuckets + 2) * 2;
 }
 __host__ __device__ constexpr int misi_ctas_per_sm(int tech) { return tech == SI_TECH_BITMAP ? 1 : 2; }
 
@@ -194,7 +207,7 @@ __device__ __forceinline__ uint32_t first_not_larger(const uint64_t* keys, uint3
 // Per row: where its partners start in the other side's sorted list, and how
 // many work items its partners' elements make.  P: exclusive prefix sums.
 __global__ void misi_rows_kernel(const uint64_t* __restrict__ keys, uint32_t nA, uint32_t nB, bool self,
-                                 const uint64_t* __restrict__ P, uint32_t* __restrict__ cs,
+                                 ItemUnit rule, const uint64_t* __restrict__ P, uint32_t* __restrict__ cs,
                                  uint64_t* __restrict__ nseg) {
     const uint32_t rows = nA + nB;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= rows; r += gridDim.x * blockDim.x) {
@@ -222,7 +235,7 @@ __global__ void misi_rows_kernel(const uint64_t* __restrict__ keys, uint32_t nA,
         }
         cs[r] = c;
         const uint64_t work = Pt[nt] - Pt[c];
-        const uint64_t unit = item_unit(size);
+        const uint64_t unit = item_unit(rule, size);
         nseg[r] = work ? (work + unit - 1) / unit : 0;
     }
 }
@@ -322,7 +335,7 @@ __global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint32_t* __
 constexpr int kOrderThreads = 256;
 __global__ void __launch_bounds__(kOrderThreads) misi_order_kernel(
     const uint64_t* __restrict__ off, uint32_t a_start, uint32_t nA, uint32_t b_start, uint32_t nB, bool self,
-    const unsigned long long* __restrict__ own, const unsigned long long* __restrict__ other,
+    ItemUnit rule, const unsigned long long* __restrict__ own, const unsigned long long* __restrict__ other,
     uint64_t* __restrict__ keys, uint64_t* __restrict__ P, uint32_t* __restrict__ cs, uint64_t* __restrict__ nseg,
     uint64_t* __restrict__ items, unsigned char* header) {
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the ranks
@@ -347,7 +360,7 @@ __global__ void __launch_bounds__(kOrderThreads) misi_order_kernel(
         const uint32_t c = self ? rank + 1 : static_cast<uint32_t>(other[i]) & mask;
         const uint64_t work = self ? totals[0] - sum - size : totals[iA ? 1 : 0] - (other[i] >> kRankBits);
         cs[row] = c;
-        const uint64_t unit = item_unit(size);
+        const uint64_t unit = item_unit(rule, size);
         nseg[row] = work ? (work + unit - 1) / unit : 0;
     }
     __syncthreads();
@@ -422,6 +435,47 @@ __device__ __forceinline__ uint64_t lower_bound_u32(const uint32_t* x, uint64_t 
 
 __device__ __forceinline__ uint32_t hslot(uint32_t v) { return (v * 0x9e3779b1u) >> (32 - kHashBits); }
 
+// obs, ip: the staged chunk sm[0, m) of sorted values, base .. base + span, and
+// behind it the ends of its buckets, top[b] = elements below bucket b (16 bits
+// each): bucket b holds the values with (v - base) >> shift == b.  A value
+// searches its bucket alone: the bucket's two ends are the cached top of the
+// search tree, one lookup in place of its first levels.
+// One to two buckets per element, at most kTopBuckets.
+__device__ __forceinline__ uint32_t top_shift(uint32_t span, uint32_t m) {
+    const uint32_t bits = 32 - __clz(span), want = min(14, 33 - __clz(m));  // span < 2^bits
+    return bits > want ? bits - want : 0u;
+}
+static_assert(kTopBuckets == 1u << 14 && kSortedChunk <= 65535, "bucket ends are 16 bits");
+__device__ __forceinline__ uint16_t* top_of(uint32_t* sm) { return reinterpret_cast<uint16_t*>(sm + kSortedChunk + 4); }
+
+// Adds to hits how many of the N values are in the chunk; the N searches are
+// interleaved, each step independent of the others'.
+template <int N>
+__device__ __forceinline__ void find_sorted(const uint32_t (&v)[N], const uint32_t* sm, uint32_t base, uint32_t span,
+                                            uint32_t m, uint32_t& hits) {
+    const uint16_t* top = top_of(const_cast<uint32_t*>(sm));
+    const uint32_t shift = top_shift(span, m), last = (span >> shift) + 1;
+    uint32_t lo[N], len[N], most = 0;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        const uint32_t b = min((v[u] - base) >> shift, last);  // bucket `last` is empty
+        lo[u] = top[b];
+        len[u] = top[b + 1] - lo[u];
+        most = max(most, len[u]);
+    }
+    // the last element <= v, or the bucket's first (a search of length 0 or 1 stays where it is)
+    for (; most > 1; most -= most >> 1) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            const uint32_t half = len[u] >> 1;
+            lo[u] = sm[lo[u] + half] <= v[u] ? lo[u] + half : lo[u];
+            len[u] -= half;
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) hits += len[u] != 0 && sm[lo[u]] == v[u] ? 1u : 0u;
+}
+
 template <int kTech>
 __device__ __forceinline__ uint32_t probe_one(uint32_t v, const uint32_t* sm, uint32_t base, uint32_t span, uint32_t m,
                                               bool has_max) {
@@ -433,24 +487,54 @@ __device__ __forceinline__ uint32_t probe_one(uint32_t v, const uint32_t* sm, ui
         uint32_t h = hslot(v), t;
         while ((t = sm[h]) != v && t != kEmpty) h = (h + 1) & (kHashTable - 1);
         return t == v ? 1u : 0u;
-    } else {  // obs: branch-free binary search of the staged sorted chunk
-        if (m == 0) return 0u;
-        uint32_t lo = 0, len = m;
-        while (len > 1) {
-            const uint32_t half = len >> 1;
-            lo = sm[lo + half] <= v ? lo + half : lo;
-            len -= half;
-        }
-        return sm[lo] == v ? 1u : 0u;
+    } else {
+        uint32_t h = 0;
+        const uint32_t vv[1] = {v};
+        find_sorted<1>(vv, sm, base, span, m, h);
+        return h;
     }
 }
 
+// Running maximum of top[0 .. nb], in place, by the CTA; top[nb + 1] = m (the
+// empty bucket past the last).  s: one word per warp.
+template <int kThreads>
+__device__ __forceinline__ void bucket_ends(uint16_t* top, uint32_t nb, uint32_t m, uint32_t* s) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t per = (nb + kThreads) / kThreads;  // of nb + 1 words
+    const uint32_t b0 = min(nb + 1, tid * per), b1 = min(nb + 1, b0 + per);
+    uint32_t mx = 0;
+    for (uint32_t b = b0; b < b1; ++b) mx = max(mx, static_cast<uint32_t>(top[b]));
+    uint32_t incl = mx;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(kFullMask, incl, d);
+        if (static_cast<int>(lane) >= d) incl = max(incl, t);
+    }
+    if (lane == 31) s[warp] = incl;
+    __syncthreads();
+    uint32_t run = __shfl_up_sync(kFullMask, incl, 1);
+    if (lane == 0) run = 0;
+    for (uint32_t w = 0; w < warp; ++w) run = max(run, s[w]);
+    for (uint32_t b = b0; b < b1; ++b) {
+        run = max(run, static_cast<uint32_t>(top[b]));
+        top[b] = static_cast<uint16_t>(run);
+    }
+    if (tid == 0) top[nb + 1] = static_cast<uint16_t>(m);
+}
+
+// kTech: BITMAP, HI or OBS, which also serves ip: merging a pair crosses the
+// larger set at every element of the smaller one, and each crossing is found by
+// the search of its bucket.  On 1001 sets of up to 16384 elements over 2^18
+// values this takes 0.67 ms, where a serial merge per lane of its piece of the
+// partner took 6.9 ms and a search of the whole chunk 1.6 ms.
 template <int kTech>
-__global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_probe_kernel(MisiParams p) {
+__global__ void __launch_bounds__(misi_threads(kTech), misi_ctas_per_sm(kTech)) misi_probe_kernel(MisiParams p) {
+    constexpr int kMisiThreads = misi_threads(kTech), kMisiWarps = kMisiThreads / 32;
     extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint64_t s_item;
     __shared__ unsigned long long s_next;  // the next slice of the item's partner elements
     __shared__ uint32_t s_has_max;
+    __shared__ uint32_t s_scan[kTech == SI_TECH_OBS ? kMisiWarps : 1];
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t rows = p.nA + p.nB;
     if constexpr (kTech == SI_TECH_BITMAP || kTech == SI_TECH_HI) {
@@ -486,11 +570,11 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
         // sizes); this item takes [it_lo, it_hi), and the warps take slices
         // of it from a shared counter (at least 4 per warp), so that a warp
         // whose slices probe faster takes more of them
-        const uint64_t unit = item_unit(nx);
+        const uint64_t unit = item_unit(item_rule(kTech), nx);
         const uint64_t it_lo = Pt[c_row] + seg * unit;
         const uint64_t it_hi = min(it_lo + unit, Pt[nt]);
         const uint64_t span_e = it_hi - it_lo;
-        const uint64_t slice = max(kMinSlice, span_e / (4 * kMisiWarps));
+        const uint64_t slice = max(min_slice(kTech), span_e / (4 * kMisiWarps));
 
         // ---- chunks of x ----
         uint64_t i0 = 0;
@@ -526,9 +610,25 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
                     uint32_t h = hslot(v);
                     while (atomicCAS(sm + h, kEmpty, v) != kEmpty) h = (h + 1) & (kHashTable - 1);
                 }
-            } else {  // obs, ip: the chunk itself
+            } else {  // obs, ip: the chunk itself, and the ends of its buckets
                 i1 = min(nx, i0 + kSortedChunk);
-                for (uint64_t e = i0 + tid; e < i1; e += kMisiThreads) sm[e - i0] = __ldg(x + e);
+                const uint32_t mm = static_cast<uint32_t>(i1 - i0);
+                span = __ldg(x + i1 - 1) - base;
+                const uint32_t shift = top_shift(span, mm), nb = (span >> shift) + 1;  // nb <= kTopBuckets
+                uint16_t* top = top_of(sm);
+                for (uint32_t e = tid; e < mm; e += kMisiThreads) sm[e] = __ldg(x + i0 + e);
+                for (uint32_t b = tid; b <= nb + 1; b += kMisiThreads) top[b] = 0;
+                __syncthreads();
+                // the last element of every bucket writes its end, a running
+                // maximum fills the empty buckets; an unsorted set may write
+                // any bucket, which the search survives (lo + len <= m there too)
+                for (uint32_t e = tid; e < mm; e += kMisiThreads) {
+                    const uint32_t b = min((sm[e] - base) >> shift, nb - 1);
+                    if (e + 1 == mm || min((sm[e + 1] - base) >> shift, nb - 1) != b)
+                        top[b + 1] = static_cast<uint16_t>(e + 1);
+                }
+                __syncthreads();
+                bucket_ends<kMisiThreads>(top, nb, mm, s_scan);
             }
             const uint32_t m = static_cast<uint32_t>(i1 - i0);
             const uint32_t vlast = __ldg(x + i1 - 1);
@@ -575,72 +675,61 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
                 }
                 const uint32_t nb = __popc(__ballot_sync(kFullMask, valid));  // valid lanes are a prefix
                 uint32_t my_hits = 0;
-                if constexpr (kTech == SI_TECH_IP) {
-                    for (uint32_t q = 0; q < nb; ++q) {
-                        const uint32_t ny = __shfl_sync(kFullMask, n, q);
-                        const uint32_t* y = p.el + __shfl_sync(kFullMask, y0, q);
-                        uint32_t hits = 0;
-                        // merge: lane takes y[j0, j1), finds its start in the chunk, walks forward
-                        const uint32_t vt = (ny + 31) / 32;
-                        const uint32_t j0 = min(ny, lane * vt), j1 = min(ny, j0 + vt);
-                        if (j0 < j1) {
-                            const uint32_t v0 = __ldg(y + j0);
-                            uint32_t qq = 0, len = m;
-                            while (len > 0) {
-                                const uint32_t half = len >> 1;
-                                const bool lt = sm[qq + half] < v0;
-                                qq = lt ? qq + half + 1 : qq;
-                                len = lt ? len - half - 1 : half;
-                            }
-                            for (uint32_t j = j0; j < j1 && qq < m; ++j) {
-                                const uint32_t v = __ldg(y + j);
-                                while (qq < m && sm[qq] < v) ++qq;
-                                hits += (qq < m && sm[qq] == v) ? 1u : 0u;
-                            }
-                        }
-                        hits = __reduce_add_sync(kFullMask, hits);
-                        if (lane == q) my_hits = hits;
-                    }
-                } else {
-                    // small pieces (< kLaneCol elements): one per lane, all at once
-                    if (valid && n < kLaneCol) {
-                        const uint32_t* y = p.el + y0;
-                        uint32_t j = 0;
-                        for (; j + 4 <= n; j += 4) {
-                            const uint32_t v0 = __ldg(y + j), v1 = __ldg(y + j + 1), v2 = __ldg(y + j + 2),
-                                           v3 = __ldg(y + j + 3);
+                // small pieces (< kLaneCol elements): one per lane, all at once
+                if (valid && n < kLaneCol) {
+                    const uint32_t* y = p.el + y0;
+                    uint32_t j = 0;
+                    for (; j + 4 <= n; j += 4) {
+                        const uint32_t v0 = __ldg(y + j), v1 = __ldg(y + j + 1), v2 = __ldg(y + j + 2),
+                                       v3 = __ldg(y + j + 3);
+                        if constexpr (kTech == SI_TECH_OBS) {
+                            const uint32_t v[4] = {v0, v1, v2, v3};
+                            find_sorted<4>(v, sm, base, span, m, my_hits);
+                        } else {
                             my_hits += probe_one<kTech>(v0, sm, base, span, m, has_max) +
                                        probe_one<kTech>(v1, sm, base, span, m, has_max) +
                                        probe_one<kTech>(v2, sm, base, span, m, has_max) +
                                        probe_one<kTech>(v3, sm, base, span, m, has_max);
                         }
-                        for (; j < n; ++j) my_hits += probe_one<kTech>(__ldg(y + j), sm, base, span, m, has_max);
                     }
-                    // large pieces: the whole warp, 16-byte loads
-                    uint32_t big = __ballot_sync(kFullMask, valid && n >= kLaneCol);
-                    while (big) {
-                        const int q = __ffs(big) - 1;
-                        big &= big - 1;
-                        const uint32_t ny = __shfl_sync(kFullMask, n, q);
-                        const uint32_t* y = p.el + __shfl_sync(kFullMask, y0, q);
-                        const uint32_t head =
-                            min(ny, static_cast<uint32_t>((16u - (reinterpret_cast<uintptr_t>(y) & 15u)) & 15u) >> 2);
-                        const uint32_t n4 = (ny - head) >> 2;
-                        const uint32_t tail0 = head + 4 * n4;
-                        uint32_t hits = 0;
-                        // head and tail: at most 3 elements each, plain loads
-                        if (lane < head) hits += probe_one<kTech>(__ldg(y + lane), sm, base, span, m, has_max);
-                        if (lane < ny - tail0)
-                            hits += probe_one<kTech>(__ldg(y + tail0 + lane), sm, base, span, m, has_max);
-                        const uint4* y4 = reinterpret_cast<const uint4*>(y + head);
-                        // kLd 16-byte loads in flight per lane (the bitmap probe is
-                        // the cheapest per element, so it keeps the most loads going)
-                        constexpr uint32_t kLd = kTech == SI_TECH_BITMAP ? 4 : 2;
-                        for (uint32_t i = lane; i < n4; i += 32 * kLd) {
-                            uint4 g[kLd];
+                    for (; j < n; ++j) my_hits += probe_one<kTech>(__ldg(y + j), sm, base, span, m, has_max);
+                }
+                // large pieces: the whole warp, 16-byte loads
+                uint32_t big = __ballot_sync(kFullMask, valid && n >= kLaneCol);
+                while (big) {
+                    const int q = __ffs(big) - 1;
+                    big &= big - 1;
+                    const uint32_t ny = __shfl_sync(kFullMask, n, q);
+                    const uint32_t* y = p.el + __shfl_sync(kFullMask, y0, q);
+                    const uint32_t head =
+                        min(ny, static_cast<uint32_t>((16u - (reinterpret_cast<uintptr_t>(y) & 15u)) & 15u) >> 2);
+                    const uint32_t n4 = (ny - head) >> 2;
+                    const uint32_t tail0 = head + 4 * n4;
+                    uint32_t hits = 0;
+                    // head and tail: at most 3 elements each, plain loads
+                    if (lane < head) hits += probe_one<kTech>(__ldg(y + lane), sm, base, span, m, has_max);
+                    if (lane < ny - tail0)
+                        hits += probe_one<kTech>(__ldg(y + tail0 + lane), sm, base, span, m, has_max);
+                    const uint4* y4 = reinterpret_cast<const uint4*>(y + head);
+                    // kLd 16-byte loads in flight per lane (the bitmap probe is
+                    // the cheapest per element, so it keeps the most loads going)
+                    constexpr uint32_t kLd = kTech == SI_TECH_BITMAP ? 4 : 2;
+                    for (uint32_t i = lane; i < n4; i += 32 * kLd) {
+                        uint4 g[kLd];
 #pragma unroll
-                            for (uint32_t u = 0; u < kLd; ++u)
-                                g[u] = i + 32 * u < n4 ? __ldg(y4 + i + 32 * u) : make_uint4(0, 0, 0, 0);
+                        for (uint32_t u = 0; u < kLd; ++u)
+                            g[u] = i + 32 * u < n4 ? __ldg(y4 + i + 32 * u) : make_uint4(0, 0, 0, 0);
+                        if constexpr (kTech == SI_TECH_OBS) {
+                            static_assert(kTech != SI_TECH_OBS || kLd == 2, "two groups at once");
+                            if (i + 32 < n4) {
+                                const uint32_t v[8] = {g[0].x, g[0].y, g[0].z, g[0].w,
+                                                       g[1].x, g[1].y, g[1].z, g[1].w};
+                                find_sorted<8>(v, sm, base, span, m, hits);
+                            } else {
+                                const uint32_t v[4] = {g[0].x, g[0].y, g[0].z, g[0].w};
+                                find_sorted<4>(v, sm, base, span, m, hits);
+                            }
+                        } else {
 #pragma unroll
                             for (uint32_t u = 0; u < kLd; ++u)
                                 if (i + 32 * u < n4)
@@ -649,9 +738,9 @@ __global__ void __launch_bounds__(kMisiThreads, misi_ctas_per_sm(kTech)) misi_pr
                                             probe_one<kTech>(g[u].z, sm, base, span, m, has_max) +
                                             probe_one<kTech>(g[u].w, sm, base, span, m, has_max);
                         }
-                        hits = __reduce_add_sync(kFullMask, hits);
-                        if (lane == q) my_hits = hits;
                     }
+                    hits = __reduce_add_sync(kFullMask, hits);
+                    if (lane == q) my_hits = hits;
                 }
                 if (valid) {
                     uint64_t idx;
@@ -701,6 +790,8 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     uint64_t* nseg = reinterpret_cast<uint64_t*>(w + L.off_nseg);
     uint64_t* items = reinterpret_cast<uint64_t*>(w + L.off_items);
     void* cub_tmp = w + L.off_cub;
+    if (t == SI_TECH_IP) t = SI_TECH_OBS;  // one kernel, see misi_probe_kernel
+    const ItemUnit rule = item_rule(t);
     if (L.rows <= kRankRows) {
         PhaseTimer timer("misi_plan", stream);
         unsigned long long* own = reinterpret_cast<unsigned long long*>(w + L.off_acc);
@@ -712,7 +803,7 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
         SI_LAUNCH_CHECK("misi_rank_kernel");
         const si_status st = launch_dependent(
             misi_order_kernel, dim3((L.rows + kOrderThreads - 1) / kOrderThreads), dim3(kOrderThreads), 0, stream,
-            d_offsets, A.start, L.nA, B.start, L.nB, L.self, static_cast<const unsigned long long*>(own),
+            d_offsets, A.start, L.nA, B.start, L.nB, L.self, rule, static_cast<const unsigned long long*>(own),
             static_cast<const unsigned long long*>(other), keys, P, cs, nseg, items, w);
         if (st != SI_OK) return st;
     } else {
@@ -739,7 +830,7 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
             SI_CUDA_TRY(cub::DeviceScan::InclusiveSum(cub_tmp, tmp, sizes + L.nA + 1, P + L.nA + 2,
                                                       static_cast<int>(L.nB), stream));
         }
-        misi_rows_kernel<<<g, 256, 0, stream>>>(keys, L.nA, L.nB, L.self, P, cs, nseg);
+        misi_rows_kernel<<<g, 256, 0, stream>>>(keys, L.nA, L.nB, L.self, rule, P, cs, nseg);
         SI_LAUNCH_CHECK("misi_rows_kernel");
         tmp = L.cub_bytes;
         SI_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, tmp, nseg, items, static_cast<int>(L.rows + 1), stream));
@@ -788,12 +879,11 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
         SI_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         const unsigned grid = static_cast<unsigned>(sm_count() * misi_ctas_per_sm(tech));
         PhaseTimer timer("misi_probe", stream);
-        kernel<<<grid, kMisiThreads, smem, stream>>>(prm);
+        kernel<<<grid, misi_threads(tech), smem, stream>>>(prm);
         SI_LAUNCH_CHECK("misi_probe_kernel");
         return SI_OK;
     };
     switch (t) {
-        case SI_TECH_IP: return launch(misi_probe_kernel<SI_TECH_IP>, SI_TECH_IP);
         case SI_TECH_OBS: return launch(misi_probe_kernel<SI_TECH_OBS>, SI_TECH_OBS);
         case SI_TECH_HI: return launch(misi_probe_kernel<SI_TECH_HI>, SI_TECH_HI);
         case SI_TECH_BITMAP: return launch(misi_probe_kernel<SI_TECH_BITMAP>, SI_TECH_BITMAP);

@@ -275,3 +275,22 @@ def test_hash_groups_that_fill_the_slots(cuda, big):
     ds, col = from_sets([s.astype(np.uint32) for s in sets])
     want = oracle.all_pairs(ds.elements, ds.offsets, ds.cardinality, ds.universe, "std")
     np.testing.assert_array_equal(run(col, "hi"), want)
+
+
+@pytest.mark.parametrize("tech", ["obs", "ip"])
+@pytest.mark.parametrize("span", [0, 1, 16383, 16384, 1 << 20, (1 << 32) - 1])
+def test_bucket_search_edges(cuda, tech, span):
+    """Buckets of the staged chunk: spans at the bucket limits, sets of one
+    bucket and of two far clusters, chunks of exactly 16384 elements and one
+    more, values below, between and above the chunk's."""
+    rng = np.random.default_rng(span % 1000 + 1)
+    base = min(5, (1 << 32) - 1 - span)
+    n = [1, 2, 100, 16384, 16385, 40000]
+    sets = [np.unique(rng.integers(base, base + span + 1, m, dtype=np.uint64)) for m in n]
+    full = np.arange(base, base + min(span + 1, 40000), dtype=np.uint64)
+    sets += [full, full[:16384], full[:16385], np.array([base, base + span], np.uint64)]
+    sets += [np.union1d(full[:9000], base + span - np.arange(min(span + 1, 9000), dtype=np.uint64)),
+             np.array([0], np.uint64), np.array([(1 << 32) - 1], np.uint64), np.zeros(0, np.uint64)]
+    ds, col = from_sets([s.astype(np.uint32) for s in sets])
+    want = oracle.all_pairs(ds.elements, ds.offsets, ds.cardinality, ds.universe, "std")
+    np.testing.assert_array_equal(run(col, tech), want)
