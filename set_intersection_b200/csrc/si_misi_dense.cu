@@ -27,76 +27,164 @@ namespace si {
 namespace {
 
 // --------------------------------------------------------- tile geometry --
-constexpr int kTileM = 128;        // rows of M (sets a) per tile  = TMEM lanes
-constexpr int kTileN = 256;        // rows of M (sets b) per tile  = TMEM columns
+// A pair of CTAs (one cluster, two SMs) computes a tile of 256 x 256 kN counts,
+// kN = 1 or 2: each CTA holds 128 rows of A and 128 kN rows of B,
+// tcgen05.mma.cta_group::2 multiplies the pair's A with the pair's B.  Shared
+// memory is what bounds it.  Per 32 bytes of K and 128 clocks of MMA an SM
+//   kN = 1: writes 8 KiB of operands and reads 12 (its A, and its half of B for
+//           itself and for the other SM): 160 clocks of its 128 bytes a clock;
+//   kN = 2: writes 6 and reads 10 (A is kept in the collector for the second
+//           MMA): 128 clocks.
+// One SM by itself with a 128 x 256 tile writes 12 and reads 12: 192 clocks.
+// Measured on 16384 sets over 65536 values, in the share of the tensor pipe's
+// peak: alone 68 % (5.47 ms), kN = 1 80 % (4.65 ms), kN = 2 90 % (4.16 ms).
+constexpr int kTile = 256;         // rows (sets a) and columns (sets b) of a pair's tile
+constexpr int kHalf = 128;         // rows of A, and of B, in each CTA = TMEM lanes
 constexpr int kTileK = 128;        // bytes of K per stage (one 128-byte swizzle span)
-constexpr int kStages = 4;
 constexpr int kMmaK = 32;          // K of one tcgen05.mma for 8-bit operands
 constexpr int kBand = 8;           // row panels per rasterisation band
-constexpr int kGemmThreads = 128;  // 4 warps: producer / MMA issuer / all four in the epilogue
-constexpr uint32_t kStageBytesA = kTileM * kTileK;  // 16 KiB
-constexpr uint32_t kStageBytesB = kTileN * kTileK;  // 32 KiB
-constexpr uint32_t kStageBytes = kStageBytesA + kStageBytesB;
-constexpr size_t kGemmSmem = size_t(kStages) * kStageBytes + 1024;  // + alignment slack
-constexpr uint32_t kTmemCols = kTileN;  // one s32/f32 column per output column
+constexpr int kEpiWarps = 8;       // warp w reads TMEM lanes 32 (w % 4) .., columns 128 kN (w / 4) ..
+constexpr int kTmaWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
+constexpr int kGemmThreads = (kEpiWarps + 2) * 32;
+constexpr uint32_t kOperandBytes = kHalf * kTileK;       // 16 KiB: a stage's A of one CTA, or B of one MMA
+constexpr uint32_t kRingBytes = 12 * kOperandBytes;      // the stages: 6 (kN = 1) or 4 (kN = 2)
+template <int kN>
+constexpr uint32_t kStageBytes = (1 + kN) * kOperandBytes;
+template <int kN>
+constexpr uint32_t kStages = kRingBytes / kStageBytes<kN>;
+constexpr uint32_t kBlockWords = 32 * 33;                // an epilogue warp's 32 x 32 counts, padded
+constexpr size_t kGemmSmem = size_t(kRingBytes) + kEpiWarps * kBlockWords * 4 + 1024;  // + alignment slack
+constexpr uint32_t kAccCols = kTile;  // one s32/f32 column per output column
+constexpr uint32_t kTmemCols = 2 * kAccCols;  // kN = 1: one is read out while the other fills; kN = 2: the tile's two
+constexpr uint32_t kSplitStages = 16;  // a part of a tile is at least this many stages of K
 
 __host__ __device__ inline uint64_t tri_index(uint64_t n, uint64_t i, uint64_t j) {
     return (n * (n - 1) / 2) - (n - i) * ((n - i) - 1) / 2 + j - i - 1;
 }
 
-// Upper-triangle tiles: tile (i, j) covers rows [128i, 128i+128) x
-// [256j, 256j+256) and is needed iff it holds a pair a < b, i.e. j >= i/2.
-// Order: bands of kBand row panels; in a band, column panel by column panel,
-// the band's row panels inside -- so the CTAs running at the same time share
-// a handful of A and B panels in L2.
-__host__ __device__ inline uint32_t band_tiles(uint32_t I, uint32_t J, uint32_t b) {
+// Upper-triangle tiles: tile (i, j) covers rows [256 i, 256 i + 256) x columns
+// [256 kN j, 256 kN (j + 1)) and is needed iff it holds a pair a < b, i.e.
+// j >= i / kN; T row panels, J column panels.  Order: bands of kBand row panels;
+// in a band, column panel by column panel, the band's row panels inside -- so
+// the pairs running at the same time share a handful of panels in L2.
+__host__ __device__ inline uint32_t band_tiles(uint32_t T, uint32_t J, uint32_t nN, uint32_t b) {
     uint32_t n = 0;
-    for (uint32_t i = b * kBand; i < min((b + 1) * kBand, I); ++i) n += J - i / 2;
+    for (uint32_t i = b * kBand; i < min((b + 1) * kBand, T); ++i) n += J - i / nN;
     return n;
 }
 
-__device__ inline void tile_of(uint32_t L, uint32_t I, uint32_t J, uint32_t& ti, uint32_t& tj) {
+__device__ inline void tile_of(uint32_t L, uint32_t T, uint32_t J, uint32_t nN, uint32_t& ti, uint32_t& tj) {
     uint32_t b = 0;
     for (;; ++b) {
-        const uint32_t n = band_tiles(I, J, b);
+        const uint32_t n = band_tiles(T, J, nN, b);
         if (L < n) break;
         L -= n;
     }
-    const uint32_t i0 = b * kBand, i1 = min(i0 + kBand, I);
-    ti = i0;
-    tj = J - 1;
-    for (uint32_t j = i0 / 2; j < J; ++j) {
-        // row panels i of this band with i/2 <= j
-        const uint32_t hi = min(i1, 2 * j + 2);
-        const uint32_t cnt = hi > i0 ? hi - i0 : 0;
-        if (L < cnt) {
-            ti = i0 + L;
-            tj = j;
-            return;
-        }
+    const uint32_t i0 = b * kBand, i1 = min(i0 + kBand, T);
+    // column panel j of the band holds the rows from i0 with i / nN <= j
+    uint32_t j = i0 / nN;
+    for (;; ++j) {
+        const uint32_t cnt = min(i1, nN * (j + 1)) - i0;
+        if (L < cnt) break;
         L -= cnt;
     }
+    ti = i0 + L;
+    tj = j;
+}
+
+// Who computes what.  Every pair takes whole tiles, as many as all pairs can;
+// each of the tiles left over is cut along K into `cuts` parts for as many
+// pairs, whose counts are added atomically into counts that the incidence
+// kernel has zeroed.  Pairs with the same part of K run side by side, so they
+// share panels in L2 (equal shares of the left-over tiles' stages, whatever tile
+// they fall in, read them from HBM instead: 5000 sets over 65536 values took
+// 669 us a call that way, 598 us this way).
+struct Schedule {
+    uint32_t T, J, nN;  // row panels, column panels, kN
+    uint32_t tiles;
+    uint32_t whole;     // tiles computed whole by all pairs (a multiple of the pairs)
+    uint32_t stages;    // K stages of a tile
+    uint32_t cuts;      // parts of each tile left over (1: it is whole too)
+};
+
+struct Work {
+    uint32_t tile, k0, k1;  // stages [k0, k1) of a tile
+};
+
+// Item n of pair w's work; false when there is none.
+__device__ __forceinline__ bool work_item(const Schedule& sc, uint32_t pairs, uint32_t w, uint32_t n, Work& out) {
+    const uint32_t rounds = sc.whole / pairs, left = sc.tiles - sc.whole;
+    if (n < rounds) {
+        out = {w + n * pairs, 0, sc.stages};
+        return true;
+    }
+    if (n > rounds || w >= left * sc.cuts) return false;
+    const uint32_t part = w / left;
+    out = {sc.whole + w % left, static_cast<uint32_t>(uint64_t(sc.stages) * part / sc.cuts),
+           static_cast<uint32_t>(uint64_t(sc.stages) * (part + 1) / sc.cuts)};
+    return true;
 }
 
 // ---------------------------------------------------------------- PTX ---
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+// The same shared-memory address in the cluster's CTA `rank`.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrives on an mbarrier of another CTA of the cluster.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Bounded wait on a phase that warps of both CTAs complete.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, uint32_t* err, uint32_t site,
+                                                  uint32_t info) {
+    WaitBudget budget;
+    do {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(done)
+            : "r"(smem_addr(bar)), "r"(parity)
+            : "memory");
+        if (done) return true;
+    } while (!budget.expired());
+    record_error(err, SI_ERR_TIMEOUT, site, info);
+    return false;
+}
+
+// A box of the matrix into this CTA's shared memory; bar (a cluster address)
+// is a barrier of either CTA of the pair.
+__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
     asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_addr(dst)),
-        "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
+        "%3}], [%4];" ::"r"(smem_addr(dst)),
+        "l"(map), "r"(x), "r"(y), "r"(bar)
         : "memory");
 }
 
+// TMEM of both CTAs of a pair: a warp of each makes the call.
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst_smem)),
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(dst_smem)),
                  "r"(ncols)
                  : "memory");
 }
 __device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -118,40 +206,50 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(const void* base) {
 template <bool kFp8>
 __host__ __device__ constexpr uint32_t instr_desc() {
     // kind::i8: D = s32 (2), A = B = unsigned 8-bit (0).  kind::f8f6f4: D = f32 (1), A = B = E4M3 (0).
-    return (kFp8 ? (1u << 4) : (2u << 4)) | (uint32_t(kTileN >> 3) << 17) | (uint32_t(kTileM >> 4) << 24);
+    return (kFp8 ? (1u << 4) : (2u << 4)) | (uint32_t(kTile >> 3) << 17) | (uint32_t(kTile >> 4) << 24);
 }
 
-template <bool kFp8>
+// kA: 0 = A is used once, 1 = keep A in the collector, 2 = take it from there
+// (the next MMA's A is the same / the last one's was).
+template <bool kFp8, int kA>
 __device__ __forceinline__ void mma_issue(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
     constexpr uint32_t idesc = instr_desc<kFp8>();
+#define SI_MMA(kind, collector)                                                                                   \
+    asm volatile("{\n\t.reg .pred p;\n\t"                                                                        \
+                 "setp.ne.b32 p, %4, 0;\n\t"                                                                     \
+                 "tcgen05.mma.cta_group::2.kind::" kind ".collector::a::" collector " [%0], %1, %2, %3, p;\n\t}" \
+                 ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)                                     \
+                 : "memory")
     if constexpr (kFp8) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-            : "memory");
+        if constexpr (kA == 0) SI_MMA("f8f6f4", "discard");
+        if constexpr (kA == 1) SI_MMA("f8f6f4", "fill");
+        if constexpr (kA == 2) SI_MMA("f8f6f4", "lastuse");
     } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),
-            "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-            : "memory");
+        if constexpr (kA == 0) SI_MMA("i8", "discard");
+        if constexpr (kA == 1) SI_MMA("i8", "fill");
+        if constexpr (kA == 2) SI_MMA("i8", "lastuse");
     }
+#undef SI_MMA
 }
 
-// Arrives on `bar` once every tcgen05.mma issued so far by this thread is done.
+// Arrives on `bar` in both CTAs of the pair once every tcgen05.mma issued so
+// far by this thread is done.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-                 : "memory");
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+            smem_addr(bar)),
+        "h"(static_cast<uint16_t>(3))
+        : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+          "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(taddr));
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -163,13 +261,32 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 // zero.  The set is read once, in order: each chunk's loop stops at the first
 // element past the chunk, which is where the next chunk starts.
 constexpr uint32_t kChunk = 32768;
+constexpr uint32_t kZeroBlocks = 32;  // blocks per cut tile, ahead of the rows' blocks
+static_assert(kTile == 256, "a thread zeroes a column of 256");
 __global__ void __launch_bounds__(256) build_incidence_kernel(const uint32_t* __restrict__ elements,
                                                               const uint64_t* __restrict__ offsets, uint32_t k,
                                                               uint8_t* __restrict__ M, uint64_t row_bytes,
-                                                              uint32_t universe, uint8_t one, uint32_t* err) {
+                                                              uint32_t universe, uint8_t one, uint32_t* err,
+                                                              Schedule sc,
+                                                              uint32_t* __restrict__ counts) {
     __shared__ __align__(16) uint8_t chunk[kChunk];
     __shared__ unsigned long long s_next;
-    const uint32_t row = blockIdx.x;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t zero_blocks = sc.cuts > 1 ? (sc.tiles - sc.whole) * kZeroBlocks : 0u;
+    if (blockIdx.x < zero_blocks) {  // zero a cut tile's counts, which its parts add into
+        constexpr uint32_t kRows = kTile / kZeroBlocks;
+        uint32_t ti, tj;
+        tile_of(sc.whole + blockIdx.x / kZeroBlocks, sc.T, sc.J, sc.nN, ti, tj);
+        const uint64_t a0 = uint64_t(ti) * kTile + blockIdx.x % kZeroBlocks * kRows;
+        for (uint32_t u = 0; u < sc.nN; ++u) {
+            const uint64_t b = (uint64_t(tj) * sc.nN + u) * kTile + threadIdx.x;
+#pragma unroll
+            for (uint32_t r = 0; r < kRows; ++r)
+                if (a0 + r < b && b < k) counts[tri_index(k, a0 + r, b)] = 0u;
+        }
+        return;
+    }
+    const uint32_t row = blockIdx.x - zero_blocks;
     uint4* c4 = reinterpret_cast<uint4*>(chunk);
     uint64_t lo = 0, e = 0;
     if (row < k) {
@@ -200,108 +317,170 @@ __global__ void __launch_bounds__(256) build_incidence_kernel(const uint32_t* __
 }
 
 // ----------------------------------------------------- tensor-core GEMM --
-template <bool kFp8>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-    tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, uint32_t k,
-                   uint32_t I, uint32_t J, uint32_t num_k_stages, uint32_t* __restrict__ counts, uint32_t* err) {
+// Persistent pairs.  Per CTA: warp 8 loads its halves of A and B, stage by
+// stage, onto the leader CTA's barrier; warp 9 of the leader (rank 0) issues
+// the MMAs of the pair; warps 0..7 read the finished accumulator out while the
+// next tile fills the other one.
+template <bool kFp8, int kN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+    tc_gemm_kernel(const __grid_constant__ CUtensorMap map, uint32_t k, const Schedule sc,
+                   uint32_t* __restrict__ counts, uint32_t* err) {
     extern __shared__ uint8_t dsmem[];
     // operand stages must start on 1024-byte boundaries (swizzle atoms)
     uint8_t* stages = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dsmem) + 1023) & ~uintptr_t(1023));
-    __shared__ __align__(8) uint64_t full[kStages], empty[kStages], accum_full;
+    uint32_t* blocks = reinterpret_cast<uint32_t*>(stages + kRingBytes);
+    constexpr uint32_t nStages = kStages<kN>, stageBytes = kStageBytes<kN>;
+    constexpr uint32_t nAcc = 2 / kN;  // accumulators
+    // full: the leader's, both CTAs' bytes of a stage; empty: each CTA's, the
+    // MMAs have read the stage; acc_full: each CTA's, an accumulator is done;
+    // acc_empty: the leader's, all epilogue warps of the pair have read it
+    __shared__ __align__(8) uint64_t full[nStages], empty[nStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t s_tmem;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint32_t ti, tj;
-    tile_of(blockIdx.x, I, J, ti, tj);
+    const uint32_t rank = cluster_rank(), pair = blockIdx.x / 2, pairs = gridDim.x / 2;
 
     if (tid == 0) {
-        for (int s = 0; s < kStages; ++s) {
+        for (uint32_t s = 0; s < nStages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        mbar_init(&accum_full, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&acc_full[s], 1);
+            mbar_init(&acc_empty[s], 2 * kEpiWarps);
+        }
         fence_mbar_init();
     }
-    if (warp == 0) {  // TMEM: 128 lanes x 256 columns of 32-bit accumulators
+    if (warp == kMmaWarp) {
         tmem_alloc(&s_tmem, kTmemCols);
         tmem_relinquish();
     }
     tc_fence_before();
     __syncthreads();
+    cluster_sync();  // both CTAs' barriers and TMEM are ready
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the matrix, and the zeroed counts
 
-    if (warp == 0 && lane == 0) {
-        // ---- TMA producer ----
-        for (uint32_t ks = 0; ks < num_k_stages; ++ks) {
-            const uint32_t s = ks % kStages, round = ks / kStages;
-            if (!mbar_wait_bounded(&empty[s], (round & 1) ^ 1, err, 21, ks)) break;
-            uint8_t* sa = stages + s * kStageBytes;
-            uint8_t* sb = sa + kStageBytesA;
-            mbar_arrive_expect_tx(&full[s], kStageBytes);
-            tma_load_2d(sa, &map_a, static_cast<int>(ks * kTileK), static_cast<int>(ti * kTileM), &full[s]);
-            tma_load_2d(sb, &map_b, static_cast<int>(ks * kTileK), static_cast<int>(tj * kTileN), &full[s]);
+    if (warp == kTmaWarp) {
+        if (lane == 0) {
+            uint32_t g = 0;  // stages loaded so far
+            bool ok = true;
+            Work wk;
+            for (uint32_t n = 0; ok && work_item(sc, pairs, pair, n, wk); ++n) {
+                uint32_t ti, tj;
+                tile_of(wk.tile, sc.T, sc.J, sc.nN, ti, tj);
+                const int ya = static_cast<int>(ti * kTile + rank * kHalf);
+                const int yb = static_cast<int>(tj * kTile * kN + rank * kHalf);
+                for (uint32_t ks = wk.k0; ks < wk.k1; ++ks, ++g) {
+                    const uint32_t s = g % nStages, round = g / nStages;
+                    ok = mbar_wait_bounded(&empty[s], (round & 1) ^ 1, err, 21, ks);
+                    if (!ok) break;
+                    uint8_t* sa = stages + s * stageBytes;
+                    const uint32_t bar = cluster_addr(&full[s], 0);
+                    if (rank == 0) mbar_arrive_expect_tx(&full[s], 2 * stageBytes);
+                    tma_load_2d(sa, &map, static_cast<int>(ks * kTileK), ya, bar);
+#pragma unroll
+                    for (int h = 0; h < kN; ++h)
+                        tma_load_2d(sa + (1 + h) * kOperandBytes, &map, static_cast<int>(ks * kTileK), yb + h * kTile, bar);
+                }
+            }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
-        bool ok = true;
-        for (uint32_t ks = 0; ks < num_k_stages && ok; ++ks) {
-            const uint32_t s = ks % kStages, round = ks / kStages;
-            ok = mbar_wait_bounded(&full[s], round & 1, err, 22, ks);
-            if (!ok) break;
+        __syncwarp();
+    } else if (warp == kMmaWarp) {
+        if (rank == 0 && lane == 0) {
+            uint32_t g = 0;
+            bool ok = true;
+            Work wk;
+            for (uint32_t n = 0; ok && work_item(sc, pairs, pair, n, wk); ++n) {
+                const uint32_t acc = n % nAcc;
+                ok = mbar_wait_cluster(&acc_empty[acc], ((n / nAcc) & 1) ^ 1, err, 25, n);
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t d = tmem + acc * kAccCols;
+                for (uint32_t ks = wk.k0; ks < wk.k1; ++ks, ++g) {
+                    const uint32_t s = g % nStages, round = g / nStages;
+                    ok = mbar_wait_bounded(&full[s], round & 1, err, 22, ks);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint8_t* sa = stages + s * stageBytes;
+                    const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sa + kOperandBytes);
+#pragma unroll
+                    for (int kk = 0; kk < kTileK / kMmaK; ++kk) {
+                        // advance 32 bytes along K inside the swizzle span: +2 in the 16-byte address field
+                        const uint32_t more = ks != wk.k0 || kk != 0;
+                        mma_issue<kFp8, kN == 1 ? 0 : 1>(d, da + 2 * kk, db + 2 * kk, more);
+                        if constexpr (kN == 2)
+                            mma_issue<kFp8, 2>(d + kAccCols, da + 2 * kk, db + kOperandBytes / 16 + 2 * kk, more);
+                    }
+                    mma_commit(&empty[s]);  // the stage is free once these MMAs have read it
+                }
+                if (ok) mma_commit(&acc_full[acc]);
+            }
+        }
+        __syncwarp();
+    } else {
+        uint32_t* blk = blocks + warp * kBlockWords;
+        Work wk;
+        for (uint32_t n = 0; work_item(sc, pairs, pair, n, wk); ++n) {
+            const uint32_t acc = n % nAcc;
+            // warp-uniform: the TMEM loads below are .sync.aligned
+            if (!__all_sync(kFullMask, mbar_wait_bounded(&acc_full[acc], (n / nAcc) & 1, err, 23, n))) break;
             tc_fence_after();
-            const uint8_t* sa = stages + s * kStageBytes;
-            const uint8_t* sb = sa + kStageBytesA;
-            const uint64_t da = smem_desc_sw128(sa), db = smem_desc_sw128(sb);
-#pragma unroll
-            for (int kk = 0; kk < kTileK / kMmaK; ++kk) {
-                // advance 32 bytes along K inside the swizzle span: +2 in the 16-byte address field
-                mma_issue<kFp8>(tmem, da + 2 * kk, db + 2 * kk, (ks | kk) != 0);
-            }
-            mma_commit(&empty[s]);  // the stage is free once these MMAs have read it
-        }
-        mma_commit(&accum_full);
-    }
-    __syncwarp();
-
-    // ---- epilogue: all four warps, warp w owns TMEM lanes (tile rows) 32w..32w+31 ----
-    // warp-uniform: the TMEM loads below are .sync.aligned
-    const bool done = __all_sync(kFullMask, mbar_wait_bounded(&accum_full, 0, err, 23, blockIdx.x));
-    tc_fence_after();
-    const uint64_t a = static_cast<uint64_t>(ti) * kTileM + warp * 32 + lane;
-    const uint64_t b0 = static_cast<uint64_t>(tj) * kTileN;
-    if (done) {
-        // Lane l holds row a = (warp's first row) + l.  Each 32 x 32 block of
-        // counts goes through a padded shared tile (the operand stages are free
-        // once every MMA has completed), so that each store writes 32
-        // consecutive counts of one row.
-        uint32_t* blk = reinterpret_cast<uint32_t*>(stages) + warp * (32 * 33);
-        const uint64_t rowbase = a < k ? tri_index(k, a, a + 1) - (a + 1) : 0;  // index of (a, b) = rowbase + b
-        const uint64_t a_first = static_cast<uint64_t>(ti) * kTileM + warp * 32;
+            uint32_t ti, tj;
+            tile_of(wk.tile, sc.T, sc.J, sc.nN, ti, tj);
+            const bool whole = sc.cuts == 1 || wk.tile < sc.whole;
+            const uint64_t a_first = uint64_t(ti) * kTile + rank * kHalf + (warp & 3) * 32;
+            const uint64_t b_first = uint64_t(tj) * kTile * kN + (warp >> 2) * kHalf * kN;
+            // TMEM lane l holds row a_first + l.  Each 32 x 32 block of counts
+            // goes through a padded shared tile, so that each store writes 32
+            // consecutive counts of one row; the index of (a, b) moves by
+            // k - a - 2 from one row to the next.
+            const uint32_t t0 =
+                tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + acc * kAccCols + (warp >> 2) * kHalf * kN;
+            const uint32_t rows = a_first < k ? static_cast<uint32_t>(min(uint64_t(32), k - a_first)) : 0u;
 #pragma unroll 1
-        for (int c = 0; c < kTileN; c += 32) {
-            uint32_t v[32];
-            tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c),
-                      *reinterpret_cast<uint32_t(*)[16]>(v));
-            tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c + 16),
-                      *reinterpret_cast<uint32_t(*)[16]>(v + 16));
+            for (int c = 0; c < kHalf * kN; c += 32) {
+                const uint64_t b0 = b_first + c, b = b0 + lane;
+                if (rows == 0 || b0 >= k || b0 + 31 <= a_first) continue;  // outside, or below the diagonal
+                uint32_t v[32];
+                tmem_ld32(t0 + static_cast<uint32_t>(c), v);
 #pragma unroll
-            for (int x = 0; x < 32; ++x)
-                blk[lane * 33 + x] = kFp8 ? static_cast<uint32_t>(__uint_as_float(v[x])) : v[x];
-            __syncwarp();
-            const uint64_t b = b0 + c + lane;
-#pragma unroll 4
-            for (int r = 0; r < 32; ++r) {
-                const uint64_t ar = a_first + r;
-                const uint64_t base_r = __shfl_sync(kFullMask, rowbase, r);
-                if (ar < k && b > ar && b < k) counts[base_r + b] = blk[r * 33 + lane];
+                for (int x = 0; x < 32; ++x)
+                    blk[lane * 33 + x] = kFp8 ? static_cast<uint32_t>(__uint_as_float(v[x])) : v[x];
+                __syncwarp();
+                uint32_t* out = counts + (tri_index(k, a_first, a_first + 1) + (b - a_first - 1));
+                uint64_t step = k - a_first - 2;
+                // lane's rows: those before b, none when b is past the sets
+                const uint32_t n = b >= k ? 0u : b <= a_first ? 0u : static_cast<uint32_t>(min(uint64_t(rows), b - a_first));
+                if (whole) {
+#pragma unroll 8
+                    for (uint32_t r = 0; r < 32; ++r) {
+                        if (r < n) *out = blk[r * 33 + lane];
+                        out += step--;
+                    }
+                } else {
+#pragma unroll 8
+                    for (uint32_t r = 0; r < 32; ++r) {
+                        const uint32_t x = blk[r * 33 + lane];
+                        if (r < n && x) atomicAdd(out, x);
+                        out += step--;
+                    }
+                }
+                __syncwarp();
             }
+            tc_fence_before();
             __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[acc], 0));
         }
+        __syncwarp();
     }
+    // A wait that gave up ends its role; the others' waits then give up in
+    // turn, seconds after the last copy was issued.
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, kTmemCols);
+    cluster_sync();  // neither CTA leaves while the other may still signal it or read its operands
+    if (warp == kMmaWarp) tmem_dealloc(tmem, kTmemCols);
 }
 
 // ------------------------------------------- plain AND-popcount (CUDA cores) --
@@ -412,6 +591,36 @@ struct DenseLayout {
 };
 constexpr size_t kDenseHeader = 256;  // error words
 
+Schedule make_schedule(uint32_t T, uint32_t stages, uint32_t nN, uint32_t pairs) {
+    Schedule sc;
+    sc.T = T;
+    sc.J = (T + nN - 1) / nN;
+    sc.nN = nN;
+    sc.stages = stages;
+    uint64_t tiles = 0;
+    for (uint32_t i = 0; i < T; ++i) tiles += sc.J - i / nN;
+    sc.tiles = tiles > 0x7fffffffull ? 0xffffffffu : static_cast<uint32_t>(tiles);
+    sc.whole = sc.tiles / pairs * pairs;
+    const uint32_t left = sc.tiles - sc.whole;
+    sc.cuts = left ? std::max(1u, std::min(pairs / left, stages / kSplitStages)) : 1u;
+    return sc;
+}
+
+// Time of a schedule in units of one stage's MMAs at the tensor pipe's peak
+// (512 clocks).  A stage of the narrow tile takes 1.25 units, of the wide one,
+// twice the work, 2.1; a round's read-out that the next tile does not hide (the
+// wide tile's accumulators fill TMEM, so all of it) 18 and 60, and half as much
+// again where the parts of a cut tile are added atomically.  Fitted to 1000 ..
+// 16384 sets over 2000 .. 65536 values; the wide tile is taken from 5000 sets
+// over 40009 values on (376 -> 367 us; 16384 over 65536 4.94 -> 4.45 ms), not for
+// 5000 over 10000 (113 us against 139) or 3001 over 40009 (166 against 227).
+double schedule_cost(const Schedule& sc, uint32_t pairs) {
+    const double stage = (sc.nN == 2 ? 2.1 : 1.25) * sc.stages, out = sc.nN == 2 ? 60 : 18;
+    double t = (sc.whole / pairs) * (stage + out);
+    if (sc.tiles > sc.whole) t += stage / sc.cuts + (sc.cuts > 1 ? 1.5 * out : out);
+    return t;
+}
+
 DenseLayout dense_layout(uint32_t k, uint32_t universe, si_technique t) {
     DenseLayout L;
     const uint64_t U = static_cast<uint64_t>(universe) + 1;  // values 0..universe
@@ -420,7 +629,7 @@ DenseLayout dense_layout(uint32_t k, uint32_t universe, si_technique t) {
         L.W = static_cast<uint32_t>((U + 31) / 32);
         L.total = L.off_matrix + static_cast<uint64_t>(k) * L.W * 4;
     } else {
-        L.k_pad = (k + kTileN - 1) / kTileN * kTileN;
+        L.k_pad = (k + kTile - 1) / kTile * kTile;
         L.row_bytes = (U + kTileK - 1) / kTileK * kTileK;
         L.total = L.off_matrix + static_cast<uint64_t>(L.k_pad) * L.row_bytes;
     }
@@ -464,38 +673,42 @@ si_status misi_dense(const uint32_t* d_elements, const uint64_t* d_offsets, uint
 
     // ---- mm on tensor cores ----
     uint8_t* M = reinterpret_cast<uint8_t*>(w + L.off_matrix);
+    const uint32_t pairs_max = std::max(1, sm_count() / 2);
+    const uint32_t nks = static_cast<uint32_t>(L.row_bytes / kTileK);
+    Schedule sc = make_schedule(L.k_pad / kTile, nks, 1, pairs_max);
+    const Schedule wide = make_schedule(L.k_pad / kTile, nks, 2, pairs_max);
+    if (schedule_cost(wide, pairs_max) < schedule_cost(sc, pairs_max)) sc = wide;
+    if (sc.tiles > 0x7fffffffu) return SI_ERR_UNSUPPORTED;
+    auto kern = sc.nN == 2 ? (fp8 ? tc_gemm_kernel<true, 2> : tc_gemm_kernel<false, 2>)
+                           : (fp8 ? tc_gemm_kernel<true, 1> : tc_gemm_kernel<false, 1>);
+    SI_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)));
+    const uint32_t left = sc.tiles - sc.whole;
+    const uint32_t pairs = sc.whole ? pairs_max : left * sc.cuts;
+    const uint32_t zero_blocks = sc.cuts > 1 ? left * kZeroBlocks : 0u;
     {
         PhaseTimer timer("mm_incidence", stream);
-        build_incidence_kernel<<<L.k_pad, 256, 0, stream>>>(d_elements, d_offsets, k, M, L.row_bytes, universe,
-                                                         fp8 ? uint8_t(0x38) : uint8_t(1), err);  // 1.0 in e4m3 = 0x38
+        build_incidence_kernel<<<L.k_pad + zero_blocks, 256, 0, stream>>>(
+            d_elements, d_offsets, k, M, L.row_bytes, universe, fp8 ? uint8_t(0x38) : uint8_t(1),  // 1.0 in e4m3 = 0x38
+            err, sc, d_counts);
     }
     SI_LAUNCH_CHECK("build_incidence_kernel");
 
     EncodeTiledFn enc = encode_tiled();
     if (!enc) return cuda_fail(cudaErrorNotSupported, "cuTensorMapEncodeTiled unavailable");
-    CUtensorMap map_a, map_b;
+    CUtensorMap map;
     const cuuint64_t gdim[2] = {L.row_bytes, L.k_pad};
     const cuuint64_t gstride[1] = {L.row_bytes};
     const cuuint32_t estride[2] = {1, 1};
-    const cuuint32_t box_a[2] = {kTileK, kTileM}, box_b[2] = {kTileK, kTileN};
-    const CUtensorMapDataType dt = CU_TENSOR_MAP_DATA_TYPE_UINT8;
-    if (enc(&map_a, dt, 2, M, gdim, gstride, box_a, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS ||
-        enc(&map_b, dt, 2, M, gdim, gstride, box_b, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint32_t box[2] = {kTileK, kHalf};
+    if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, M, gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cuda_fail(cudaErrorInvalidValue, "cuTensorMapEncodeTiled");
 
-    const uint32_t I = L.k_pad / kTileM, J = L.k_pad / kTileN;
-    uint64_t ntiles = 0;
-    for (uint32_t b = 0; b * kBand < I; ++b) ntiles += band_tiles(I, J, b);
-    const uint32_t nks = static_cast<uint32_t>(L.row_bytes / kTileK);
-    auto kern = fp8 ? tc_gemm_kernel<true> : tc_gemm_kernel<false>;
-    SI_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kGemmSmem)));
     PhaseTimer timer("mm_gemm", stream);
-    kern<<<static_cast<unsigned>(ntiles), kGemmThreads, kGemmSmem, stream>>>(map_a, map_b, k, I, J, nks, d_counts,
-                                                                           err);
+    const si_status st = launch_dependent(kern, dim3(2 * pairs), dim3(kGemmThreads), kGemmSmem, stream, map, k, sc,
+                                          d_counts, err);
+    if (st != SI_OK) return st;
     SI_LAUNCH_CHECK("tc_gemm_kernel");
     return SI_OK;
 }

@@ -110,3 +110,50 @@ def test_dense_config_16384_sets(cuda):
     want = oracle.all_pairs(el, off, k, 65535, "bitset", threads=os.cpu_count() or 1)
     assert want.size == k * (k - 1) // 2
     np.testing.assert_array_equal(c_int8, want)
+
+@pytest.mark.parametrize("dtype", ["int8", "fp8"])
+@pytest.mark.parametrize("k,values", [
+    (2, 1), (129, 127), (255, 128), (256, 4096), (257, 4097), (511, 300000), (513, 2049), (769, 5000), (1025, 2048),
+    (3000, 3000), (4300, 65536),
+])
+def test_paired_tiles_edges(cuda, k, values, dtype):
+    """Set counts at the edges of the 256-row panels, one to many K stages,
+    tiles cut along K and whole, the narrow tile and (4300 sets over 65536
+    values) the wide one; some sets empty, some full, against the popcount
+    kernel, and the oracle on sampled pairs."""
+    from set_intersection_b200 import generate
+    el, off = generate.bernoulli(k + values, k, values, min(0.3, 3e6 / (k * values)))
+    sets = [el[off[i]:off[i + 1]] for i in range(k)]
+    for i in (0, k // 2, k - 1):
+        sets[i] = np.arange(values, dtype=np.uint32)
+    if k > 2:
+        sets[1] = np.zeros(0, np.uint32)
+    ds = fmt.from_sets(sets, universe=values - 1)
+    col = collection(ds.elements, ds.offsets, values - 1)
+    got = counts(col, "mm", dtype)
+    np.testing.assert_array_equal(got, counts(col, "bitmap_naive", "int8"))
+    rng = np.random.default_rng(k)
+    a = rng.integers(0, k - 1, 200)
+    b = rng.integers(a + 1, k)
+    pairs = np.stack([a, b], 1).astype(np.uint32)
+    tri = k * (k - 1) // 2 - (k - a) * (k - a - 1) // 2 + b - a - 1
+    np.testing.assert_array_equal(got[tri], oracle.pairs(ds.elements, ds.offsets, k, pairs))
+
+
+@pytest.mark.parametrize("dtype", ["int8", "fp8"])
+def test_dense_call_in_a_graph(cuda, dtype):
+    import torch
+    from set_intersection_b200 import api, generate
+    k, n = 700, 6000
+    el, off = generate.bernoulli(7, k, n, 0.1)
+    want = oracle.all_pairs(el, off, k, n - 1, "std")
+    col, ws = collection(el, off, n - 1), api.Workspace()
+    out = torch.zeros(want.size, dtype=torch.int32, device="cuda")
+    api.misi_dense_into(col, out, "mm", dtype, ws)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        api.misi_dense_into(col, out, "mm", dtype, ws)
+    for _ in range(2):
+        out.fill_(3)
+        g.replay()
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
