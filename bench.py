@@ -101,6 +101,7 @@ def log(*a):
 
 
 SKEW_RATIO = 64  # SI_TECH_AUTO: obs when one set is more than this many times the other
+IP_TILE = 5184  # merged elements per tile of the intersect-path kernels
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from ncu
 # captures summarised in profiles/: the bitmap engine's bp_stream_kernel
@@ -110,8 +111,6 @@ SKEW_RATIO = 64  # SI_TECH_AUTO: obs when one set is more than this many times t
 TRAFFIC_PER_LAUNCH = {
     "bitmap/sisi_large/out": 2.246e9 + 121.53e6,   # one-pass dram__bytes capture of the 2^28 stream kernel
     "bitmap/sisi_mid/out": 321.59e6 + 5.21e6,      # from the 2^25 full capture
-    "ip/sisi_large/out": 8 * (268.727808e6 + 13.220096e6),
-    "ip/sisi_mid/out": 268.727808e6 + 13.220096e6,
 }
 
 
@@ -478,13 +477,16 @@ def run_ours(args, rank: int, world: int):
     peak = peaks.get("hbm_gbs", FALLBACK_HBM_GBS)
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
     alg_bytes = 4 * (n_a + n_b) + (4 * c if args.materialize else 0)
-    # the engine that ran: auto searches a much smaller set in the larger (obs)
-    # and streams pairs of similar size through the bitmap tiles
+    # the engine that ran: auto merges small pairs (ip), searches a much smaller
+    # set in the larger (obs) and streams the rest through window bitmaps
     engine = args.technique
     if engine == "auto":
-        engine = "obs" if min(n_a, n_b) * SKEW_RATIO < max(n_a, n_b) else "bitmap"
+        engine = ("ip" if n_a + n_b <= 1 << 21 else "obs" if min(n_a, n_b) * SKEW_RATIO < max(n_a, n_b)
+                  else "ip" if n_a + n_b <= 1 << 24 else "bitmap")
+    tiles = max(1, -(-(n_a + n_b) // IP_TILE))
+    ip_launches = (1 if tiles == 1 else 3 if tiles > 4096 or (tiles <= 2048 and args.materialize) else 2)
     kernel, launches = {
-        "ip": ("ip_tile_kernel<merge path>", 3),
+        "ip": ("ip_group_kernel" if tiles > 2048 and args.materialize else "ip_tile_kernel", ip_launches),
         "hi": ("bh_stream_kernel", 2 if args.materialize else 1),
         "bitmap": ("bp_stream_kernel", 2 if args.materialize else 1),
         "obs": ("obs_search_kernel", 3 if args.materialize else 2),

@@ -74,8 +74,8 @@ const char* si_last_error_string(void);
  * count; element output is this engine's addition, ordered as
  * std::set_intersection orders it.
  *
- * Techniques: IP merges the two sets tile by tile (value-pivot tiles of <= 6144
- * elements per set, both sets streamed once); HI streams them like BITMAP
+ * Techniques: IP merges the two sets along their merge path, tile by tile
+ * (5184 merged elements each); HI streams them like BITMAP
  * below, but each window of 512 elements of the smaller set goes into a
  * warp-private hash table that the larger set's elements probe; BITMAP streams
  * the larger set in equal ranges, one warp per range, with the matching part
@@ -83,8 +83,9 @@ const char* si_last_error_string(void);
  * AND and popcount), and orders the output by a scan of the range counts,
  * through a scratch array as long as the smaller set (so its workspace is
  * about 4 min(nA, nB) bytes larger); OBS searches every element of the smaller set in the larger one
- * (cached top levels in shared memory); AUTO takes OBS when one set is more
- * than 64 times larger than the other, else BITMAP.
+ * (cached top levels in shared memory); AUTO takes IP for pairs of up to 2^21
+ * elements in all, else OBS when one set is more than 64 times larger than the
+ * other, else IP up to 2^24 elements in all and BITMAP above.
  *
  * d_count: device uint64, receives |A ∩ B|.
  * d_out:   device uint32[out_cap] or NULL (count only).  When non-NULL,

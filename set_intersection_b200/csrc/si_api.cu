@@ -161,11 +161,11 @@ size_t si_sisi_workspace_size(uint64_t nA, uint64_t nB, si_technique t) {
         case SI_TECH_IP:
             return si::ip_workspace_size(nA, nB);
         case SI_TECH_HI:
-            return si::ip_workspace_size(nA, nB, 2);
+            return si::bm_workspace_size(nA, nB);
         case SI_TECH_BITMAP:
-            return si::ip_workspace_size(nA, nB, 1);
+            return si::bm_workspace_size(nA, nB);
         case SI_TECH_AUTO:
-            return std::max(si::ip_workspace_size(nA, nB, 1), si::obs_workspace_size(nA, nB));
+            return std::max({si::ip_workspace_size(nA, nB), si::bm_workspace_size(nA, nB), si::obs_workspace_size(nA, nB)});
         case SI_TECH_OBS:
             return si::obs_workspace_size(nA, nB);
         default:
@@ -184,17 +184,20 @@ si_status si_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t 
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     switch (t) {
         case SI_TECH_IP:
-            return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s, 0);
+            return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s);
         case SI_TECH_AUTO:
-            // skewed pairs: search the small set in the large one (reads a
-            // fraction of the large set); otherwise stream both through tiles
-            if (std::min(nA, nB) * si::kSkewRatio < std::max(nA, nB))
-                return si::obs_sisi(dA, nA, dB, nB, d_count, d_out, d_workspace, workspace_bytes, s);
-            return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s, 1);
+            switch (si::sisi_auto(nA, nB)) {
+                case SI_TECH_IP:
+                    return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s);
+                case SI_TECH_OBS:
+                    return si::obs_sisi(dA, nA, dB, nB, d_count, d_out, d_workspace, workspace_bytes, s);
+                default:
+                    return si::bm_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s);
+            }
         case SI_TECH_BITMAP:
-            return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s, 1);
+            return si::bm_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s);
         case SI_TECH_HI:
-            return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s, 2);
+            return si::bm_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s, true);
         case SI_TECH_OBS:
             return si::obs_sisi(dA, nA, dB, nB, d_count, d_out, d_workspace, workspace_bytes, s);
         default:

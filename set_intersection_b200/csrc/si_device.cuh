@@ -118,54 +118,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
     return false;
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 // Orders this thread's earlier generic-proxy shared-memory accesses before its
 // later async-proxy (bulk copy) ones.
 __device__ __forceinline__ void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
-// Named barrier over `count` threads (id 0 is __syncthreads).
-__device__ __forceinline__ void named_barrier(uint32_t id, uint32_t count) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
-
-// Named barrier that also ORs a predicate over the `count` threads: every
-// thread gets true if any passed true.
-__device__ __forceinline__ bool named_barrier_or(uint32_t id, uint32_t count, bool v) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 p, %1, 0;\n\t"
-        "barrier.red.or.pred q, %2, %3, p;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(r)
-        : "r"(v ? 1u : 0u), "r"(id), "r"(count)
-        : "memory");
-    return r != 0;
-}
-
-__device__ __forceinline__ uint64_t ld_acquire_shared_u64(const uint64_t* p) {
-    uint64_t v;
-    asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(smem_addr(p)) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_shared_u64(uint64_t* p, uint64_t v) {
-    asm volatile("st.release.cta.shared::cta.u64 [%0], %1;" ::"r"(smem_addr(p)), "l"(v) : "memory");
-}
-
-__device__ __forceinline__ uint32_t ld_acquire_shared_u32(const uint32_t* p) {
-    uint32_t v;
-    asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(smem_addr(p)) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_shared_u32(uint32_t* p, uint32_t v) {
-    asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(smem_addr(p)), "r"(v) : "memory");
 }
 
 // 1-D bulk copy global -> shared (TMA engine), completion counted on `bar`.
@@ -179,16 +135,6 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 
 // ------------------------------------------------------- flags (look-back) --
-__device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {
-    uint64_t v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_release_u64(uint64_t* p, uint64_t v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-
 // Relaxed (unordered) 64-bit accesses at GPU scope: for status words whose
 // flag and value travel together in one word, so no other access needs to be
 // ordered with them.
@@ -217,42 +163,6 @@ __device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFullMask, v, d);
     return v;
-}
-
-// ------------------------------------------------------ staging planning --
-// Plan for copying n uint32 from global g into a 16-byte aligned shared
-// buffer `buf` (capacity >= n + 8) so that element x lands at dst[x]:
-// the 16-byte aligned middle goes through the bulk-copy engine, the <= 3
-// leading and <= 3 trailing elements through ordinary loads.
-struct StagePlan {
-    uint32_t* dst;   // shared address of element 0
-    int head;        // elements [0, head) by plain loads
-    int body;        // elements [head, head + body) by bulk copy (body % 4 == 0)
-    int n;           // elements [head + body, n) by plain loads
-};
-
-__device__ __forceinline__ StagePlan plan_stage(const uint32_t* g, int n, uint32_t* buf) {
-    StagePlan p;
-    const int mis = static_cast<int>((reinterpret_cast<uintptr_t>(g) & 15u) >> 2);
-    int head = mis ? 4 - mis : 0;
-    if (head > n) head = n;
-    p.head = head;
-    p.body = ((n - head) >> 2) << 2;
-    p.dst = buf + ((4 - head) & 3);
-    p.n = n;
-    return p;
-}
-
-// Issued by one thread: the bulk part of a plan.
-__device__ __forceinline__ void issue_stage(const StagePlan& p, const uint32_t* g, uint64_t* bar) {
-    if (p.body > 0) bulk_g2s(p.dst + p.head, g + p.head, static_cast<uint32_t>(p.body) * 4u, bar);
-}
-
-// Done by threads [0, 6): the plain-load edges of a plan.
-__device__ __forceinline__ void edge_stage(const StagePlan& p, const uint32_t* g, int slot) {
-    int x = slot < 3 ? slot : p.head + p.body + (slot - 3);
-    bool want = slot < 3 ? (slot < p.head) : (x < p.n);
-    if (want) p.dst[x] = __ldg(g + x);
 }
 
 }  // namespace si

@@ -64,35 +64,30 @@ private:
     cudaStream_t stream_;
 };
 
-// ---- single-pair tile pipeline (si_sisi_ip.cu, si_sisi_bitmap.cu) ----
-// inner: 0 = merge path (technique ip), 1 = the bitmap engine (technique
-// bitmap: per-warp bitmap build + probe, si_sisi_bitmap.cu), 2 = hash probe
-// (technique hi).  The bitmap engine's workspace is larger (its scratch array).
-size_t ip_workspace_size(uint64_t nA, uint64_t nB, int inner = 0);
-// Value-pivot split of (A, B) at every S-th element of each set into
-// split_a/split_b[nA/S + nB/S + 2] (rounded up), through the sample arrays
-// samples_a/samples_b (pivot_samples_bytes in all, two 256-byte aligned
-// parts); also clears zero[0, nzero) and *d_count.  Lets the next kernel on
-// the stream start early (programmatic dependent launch); that kernel must
-// execute griddepcontrol.wait before it reads any of these.
-si_status pivot_split(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t S,
-                      uint64_t* split_a, uint64_t* split_b, uint32_t* samples_a, uint32_t* samples_b,
-                      uint64_t* zero, uint64_t nzero, uint64_t* d_count, cudaStream_t stream);
-size_t pivot_samples_bytes(uint64_t nA, uint64_t nB, uint64_t S);
+// ---- one pair ----
+// Intersect path (si_sisi_ip.cu).
+size_t ip_workspace_size(uint64_t nA, uint64_t nB);
+si_status ip_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
+                  uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream);
 // The stream engine of si_sisi_bitmap.cu: window bitmaps (technique bitmap)
 // or, with hash set, window hash tables (technique hi) on the same ranges.
 size_t bm_workspace_size(uint64_t nA, uint64_t nB);
 si_status bm_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
                   uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream,
                   bool hash = false);
-// SI_TECH_AUTO searches the smaller set in the larger (obs) when the sizes
-// differ by more than this factor.
-constexpr uint64_t kSkewRatio = 64;
+// What SI_TECH_AUTO runs for a pair.  Device time with elements out, ip /
+// bitmap / obs: 2^17 x 2^17 10 / 35 / 14 us, 2^20 x 2^20 17 / 36 / 34, 2^23 x 2^23
+// 43 / 45 / 186, 2^24 x 2^24 77 / 63; 1000 x 2^20 9 / 21 / 12 us, 10000 x 2^21
+// 12.4 / 21 / 12.1, 30000 x 2^23 21 / 25 / 15.
+inline si_technique sisi_auto(uint64_t nA, uint64_t nB) {
+    const uint64_t small = nA < nB ? nA : nB, large = nA < nB ? nB : nA, total = nA + nB;
+    if (total <= (1ull << 21)) return SI_TECH_IP;
+    if (small * 64 < large) return SI_TECH_OBS;
+    return total <= (1ull << 24) ? SI_TECH_IP : SI_TECH_BITMAP;
+}
 size_t obs_workspace_size(uint64_t nA, uint64_t nB);
 si_status obs_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
                    uint32_t* d_out, void* ws, size_t ws_bytes, cudaStream_t stream);
-si_status ip_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
-                  uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream, int inner = 0);
 
 // ---- all pairs of a dense collection (si_misi_dense.cu) ----
 // t: SI_TECH_MM (tensor cores; fp8 selects FP8-e4m3 operands instead of INT8)

@@ -1,6 +1,5 @@
 // si_sisi_bitmap.cu -- technique bitmap for one pair of large sorted sets
-// (and SI_TECH_AUTO for pairs of similar size), plus the value-pivot split
-// that the intersect-path tiles use.
+// (and SI_TECH_AUTO for pairs of similar size).
 //
 // Replaces the single-instance path of bitmap_dynamic (src/bitmap_dynamic.cu:
 // 168-176: constructBitmap over the whole universe, singleInstanceIntersect,
@@ -31,12 +30,6 @@
 //      the range's X elements up to the window's last value probe it; the
 //      same scratch, range scan and copy kernel as the bitmap stream.
 //
-//  pivot_sample_kernel + pivot_split_kernel  the intersect-path tiles' split
-//      (si_sisi_ip.cu): every S-th element of each set is a pivot; one warp
-//      per pivot finds its rank in the merged pivot order (a merge-path search
-//      over the compact samples) and its exact split in the other set (a
-//      128-element probe at the interpolated position, else a warp search).
-//
 // X is the larger set, Y the smaller (the scratch array is as long as Y).
 // Sets must be sorted and duplicate-free; this engine does not detect
 // unsorted input (si_validate_sorted does).
@@ -48,113 +41,6 @@
 
 namespace si {
 namespace {
-
-// ------------------------------------------------------------ pivot split --
-// Samples sa[k] = A[k S], sb[k] = B[k S]; clears zero[0, nzero) and the count.
-__global__ void __launch_bounds__(256) pivot_sample_kernel(const uint32_t* __restrict__ A, uint64_t nA,
-                                                           const uint32_t* __restrict__ B, uint64_t nB, uint64_t S,
-                                                           uint32_t* __restrict__ sa, uint32_t* __restrict__ sb,
-                                                           uint64_t* __restrict__ zero, uint64_t nzero,
-                                                           uint64_t* __restrict__ d_count) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    const uint64_t nSA = (nA + S - 1) / S, nSB = (nB + S - 1) / S;
-    const uint64_t t0 = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    if (t0 == 0) *d_count = 0;
-    for (uint64_t k = t0; k < nSA; k += stride) sa[k] = __ldg(A + k * S);
-    for (uint64_t k = t0; k < nSB; k += stride) sb[k] = __ldg(B + k * S);
-    for (uint64_t k = t0; k < nzero; k += stride) zero[k] = 0;
-}
-
-// #(O[lo, hi) < v) + lo, warp-cooperative, for a window whose elements before
-// lo are < v and from hi on are >= v.  vlo = O[lo]; vhi = O[hi] when
-// have_vhi.  First a 128-element probe around the position interpolated
-// between vlo and vhi (one round trip for evenly spread values), else a warp
-// search of the side of the probe the answer lies on.
-__device__ __forceinline__ uint64_t window_rank(const uint32_t* __restrict__ O, uint64_t lo, uint64_t hi, uint32_t v,
-                                                uint32_t vlo, uint32_t vhi, bool have_vhi) {
-    const uint32_t lane = threadIdx.x & 31;
-    constexpr uint64_t kW = 128;
-    uint64_t wb = lo;
-    if (hi - lo > kW) {
-        uint64_t est = lo + (hi - lo) / 2;
-        if (have_vhi && vhi > vlo && v >= vlo)
-            est = lo + static_cast<uint64_t>(v - vlo) * (hi - lo) / (static_cast<uint64_t>(vhi) - vlo);
-        wb = est > lo + kW / 2 ? est - kW / 2 : lo;
-        if (wb + kW > hi) wb = hi - kW;
-    }
-    uint32_t c = 0, first = 0, last = 0;
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const uint64_t x = wb + 32 * r + lane;
-        if (x < hi) {
-            const uint32_t e = __ldg(O + x);
-            c += e < v ? 1u : 0u;
-            if (r == 0 && lane == 0) first = e;
-            if (x == min(wb + kW, hi) - 1) last = e;
-        }
-    }
-    c = __reduce_add_sync(kFullMask, c);
-    first = __shfl_sync(kFullMask, first, 0);
-    const uint32_t last_lane = static_cast<uint32_t>((min(wb + kW, hi) - 1 - wb) & 31);
-    last = __shfl_sync(kFullMask, last, last_lane);
-    const uint64_t wend = min(wb + kW, hi);
-    if (wb > lo && first >= v)  // the answer lies before the probe
-        return warp_first_true(lo, wb, [&](uint64_t x) { return __ldg(O + x) >= v; });
-    if (wend < hi && last < v)  // ... or after it
-        return warp_first_true(wend, hi, [&](uint64_t x) { return __ldg(O + x) >= v; });
-    return wb + c;
-}
-
-// One warp per pivot rank u in [0, nSA + nSB) (thread 0 also closes the
-// table): split_a[u + 1] = #A elements below the pivot's value (exact for an
-// A pivot: its index), split_b[u + 1] likewise.  split[0] = (0, 0) and
-// split[nP + 1] = (nA, nB).  Ties between an A and a B pivot: A first.
-__global__ void __launch_bounds__(256) pivot_split_kernel(const uint32_t* __restrict__ A, uint64_t nA,
-                                                          const uint32_t* __restrict__ B, uint64_t nB, uint64_t S,
-                                                          const uint32_t* __restrict__ sa,
-                                                          const uint32_t* __restrict__ sb,
-                                                          uint64_t* __restrict__ split_a,
-                                                          uint64_t* __restrict__ split_b) {
-    // the dependent launch (the tile kernel) may start its set-up now; it
-    // waits for this grid's completion before it reads anything written here
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // the samples
-    const uint64_t nSA = (nA + S - 1) / S, nSB = (nB + S - 1) / S, nP = nSA + nSB;
-    const uint64_t tid = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const uint64_t nthreads = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    if (tid == 0) {
-        split_a[0] = 0;
-        split_b[0] = 0;
-        split_a[nP + 1] = nA;
-        split_b[nP + 1] = nB;
-    }
-    const uint32_t lane = threadIdx.x & 31;
-    for (uint64_t u = tid / 32; u < nP; u += nthreads / 32) {
-        // i = #A pivots among the first u of the merged order: the first i in
-        // [max(0, u - nSB), min(u, nSA)) whose A pivot comes after B pivot u-1-i
-        const uint64_t ilo = u > nSB ? u - nSB : 0, ihi = u < nSA ? u : nSA;
-        const uint64_t i = warp_first_true(ilo, ihi, [&](uint64_t x) { return sa[x] > sb[u - 1 - x]; });
-        const uint64_t j = u - i;
-        const uint32_t va = i < nSA ? sa[i] : 0u, vb = j < nSB ? sb[j] : 0u;
-        const bool isA = i < nSA && (j >= nSB || va <= vb);
-        // exact split in the other set O: #(O < v) lies in the window of O's
-        // preceding pivot, [(w - 1) S, min(w S, nO))
-        const uint32_t v = isA ? va : vb;
-        const uint32_t* O = isA ? B : A;
-        const uint32_t* SO = isA ? sb : sa;
-        const uint64_t nO = isA ? nB : nA, nSO = isA ? nSB : nSA, w = isA ? j : i;
-        uint64_t other = 0;
-        if (w > 0) {
-            const uint64_t lo = (w - 1) * S, hi = min(w * S, nO);
-            other = window_rank(O, lo, hi, v, SO[w - 1], w < nSO ? SO[w] : 0u, w < nSO);
-        }
-        if (lane == 0) {
-            split_a[u + 1] = isA ? i * S : other;
-            split_b[u + 1] = isA ? other : j * S;
-        }
-    }
-}
 
 // ------------------------------------------------------ bitmap stream --
 // values per window: 32768 (a 4 KiB bitmap per set; 16384 measured 2.4 %
@@ -491,27 +377,6 @@ BpLayout make_bp_layout(uint64_t nA, uint64_t nB) {
 }
 
 }  // namespace
-
-si_status pivot_split(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t S,
-                      uint64_t* split_a, uint64_t* split_b, uint32_t* samples_a, uint32_t* samples_b,
-                      uint64_t* zero, uint64_t nzero, uint64_t* d_count, cudaStream_t stream) {
-    const uint64_t nSA = (nA + S - 1) / S, nSB = (nB + S - 1) / S, nP = nSA + nSB;
-    PhaseTimer timer("sisi_split", stream);
-    const uint64_t work = std::max<uint64_t>(1, std::max(std::max(nSA, nSB), nzero));
-    const unsigned grid1 =
-        static_cast<unsigned>(std::min<uint64_t>((work + 255) / 256, static_cast<uint64_t>(sm_count()) * 8));
-    pivot_sample_kernel<<<grid1, 256, 0, stream>>>(dA, nA, dB, nB, S, samples_a, samples_b, zero, nzero, d_count);
-    SI_LAUNCH_CHECK("pivot_sample_kernel");
-    const unsigned grid2 = static_cast<unsigned>(
-        std::min<uint64_t>((std::max<uint64_t>(1, nP) + 7) / 8, static_cast<uint64_t>(sm_count()) * 16));
-    return launch_dependent(pivot_split_kernel, dim3(grid2), dim3(256), 0, stream, dA, nA, dB, nB, S,
-                            static_cast<const uint32_t*>(samples_a), static_cast<const uint32_t*>(samples_b),
-                            split_a, split_b);
-}
-
-size_t pivot_samples_bytes(uint64_t nA, uint64_t nB, uint64_t S) {
-    return align_up(((nA + S - 1) / S) * 4, 256) + align_up(((nB + S - 1) / S) * 4, 256);
-}
 
 size_t bm_workspace_size(uint64_t nA, uint64_t nB) { return make_bp_layout(nA, nB).total; }
 

@@ -1,4 +1,4 @@
-// si_sisi_ip.cu -- intersect-path (ip) for one pair of large sorted sets.
+// si_sisi_ip.cu -- intersect-path (ip) for one pair of sorted sets.
 //
 // Replaces findDiagonals (include/helpers.cuh:75-166) + intersectPath
 // (src/ip.cu:207-245) for the single-instance case.  Same two-level idea --
@@ -6,122 +6,143 @@
 // sub-diagonal of its tile and merges serially (include/helpers.cuh:24-61) --
 // re-designed for B200:
 //
-//  * Grid level: instead of one 32-thread warp probe per diagonal per pair,
-//    tiles are cut at VALUE pivots (pivot_split, si_sisi_bitmap.cu).  Every
-//    S-th element of A and of B is a pivot (S = 6144); a pivot's rank in the
-//    merged pivot order and its exact position in the other set are found by
-//    warp-cooperative searches.  Consecutive pivots bound a tile to <= S
-//    elements of each set, and because a tile boundary is a value, an equal
-//    pair is never split across tiles (no "augmentation" atomic, quirk of
+//  * Grid level (ip_split_kernel, ip_fine_kernel): tile t covers merged
+//    positions [t kTile, (t + 1) kTile).  One warp finds where a tile's diagonal
+//    crosses the path with a 32-ary search (four round trips for 2^20 elements);
+//    of very many tiles the warps take every 64th, and one thread each the rest,
+//    between its two neighbours.
+//  * Staging: a tile's A and B ranges go into shared memory by two bulk copies
+//    (TMA) of their 16-byte aligned supersets, each range with its successor
+//    element.  The successors stand for the next tile's first elements, so that
+//    an equal pair whose two halves fall into neighbouring tiles is found by the
+//    tile that holds the A element (no "augmentation" atomic, quirk of
 //    include/helpers.cuh:121-124).
-//  * Staging: each tile's A and B ranges are copied into shared memory by the
-//    bulk-copy (TMA) engine as their 16-byte aligned supersets (every block
-//    copied holds an element of the range); every input byte is read from HBM
-//    once.
-//  * Thread level: merge-path split per thread in shared memory with one
-//    tie rule (A first on ties), then a sentinel-terminated serial merge.
-//  * Output: matches are compacted per tile and placed with a decoupled
-//    look-back over tile aggregates (single pass); count-only mode instead
-//    accumulates tile counts into 256 spread partial sums.
+//  * Thread level: merge-path split per thread in shared memory with one tie
+//    rule (A first on ties), then kVT merge steps of eight instructions; a match
+//    is an A element taken while the head of B equals it.
+//  * Output (ip_tile_kernel, up to kPlaceTiles tiles): merged once for the
+//    tiles' counts and once more to write each tile's matches behind those of
+//    the tiles before it.  No CTA waits for another.  More tiles
+//    (ip_group_kernel): once, with a decoupled look-back per group of tiles.
 //
-// Techniques bitmap (and auto for pairs of similar size) and hi run the stream
-// engine of si_sisi_bitmap.cu, which also holds the pivot split.
+// A pair of one tile is a single launch of one CTA, which clears the header
+// itself.  Eight CTAs per SM hide each other's staging and searches, so a tile
+// has no warps of its own for them.  What bounds it: shared memory's banks (the
+// threads' reads are kVT / 2 words apart, 2.9 wavefronts a load; 79 % of the
+// LSU's data pipe) and issue slots (77 %) on large pairs, latency on small ones.
+//
+// Measured, device time with elements out / counts only (in brackets: a
+// persistent kernel with producer, consumer and output warps on tiles cut at
+// value pivots): 1000 x 1000 3.8 / 3.4 us (18 / 16), 2^20 x 2^20 17 / 8 us (42 /
+// 24), 2^24 x 2^24 77 / 49 us (96 / 68), 2^27 x 2^27 453 / 261 us (584 / 409).
+// 256 threads with 17 steps took 578 / 335 us at 2^27 x 2^27, with 23 steps 477 /
+// 284; a look-back per tile 1066 us (every tile's CTA polls the same words).
+//
+// Techniques bitmap (and auto for large pairs of similar size) and hi run the
+// stream engine of si_sisi_bitmap.cu.
 #include <algorithm>
 
 #include "si_device.cuh"
 #include "si_internal.h"
+#include "si_stream.cuh"
 
 namespace si {
 namespace {
 
-constexpr uint32_t kS = 6144;  // pivot (sample) stride: a tile holds at most this many elements of each set
-constexpr int kPartials = 256;
+constexpr int kIpThreads = 192;
+constexpr int kIpWarps = kIpThreads / 32;
+constexpr int kVT = 27;  // merge steps per thread: odd, so that consecutive threads' shared loads spread over the banks
+constexpr uint32_t kTile = kIpThreads * kVT;
+constexpr int kIpCtasPerSm = 8;
+// both ranges, their successors, the alignment of both, and the steps by which
+// a thread's reads can run over when the sets are not sorted
+constexpr uint32_t kStaged = kTile + 2 * 8 + 8 + 32;
+// Element output of up to this many tiles merges them twice; of more, once with
+// a look-back.
+constexpr uint64_t kPlaceTiles = 2048;  // 10.6 M merged elements
+constexpr uint64_t kFineTiles = 4096;        // more tiles than this are split in two steps
+constexpr uint32_t kCoarse = 64;             // tiles per coarse split
+static_assert(kVT <= 31, "a thread's matches are a 32-bit mask");
 
 constexpr uint64_t kFlagAgg = 1ull << 62;
 constexpr uint64_t kFlagInc = 2ull << 62;
 constexpr uint64_t kValMask = (1ull << 62) - 1;
 
-// Workspace layout.  Offsets in bytes from the workspace base.
+// Workspace: header ([0..16) error words), the groups' look-back status or the
+// tiles' counts, the tiles' splits (A elements before each tile).
+constexpr size_t kIpHeader = 256;
 struct Layout {
     uint64_t nTiles = 0;
-    size_t off_status = 0, off_split_a = 0, off_split_b = 0, off_samples = 0, total = 0;
+    size_t off_status = 0, off_split = 0, total = 0;
 };
-// Header: [0] u32 error word, [4] u32 error site, [8] u32 error detail,
-// [12] u32 sites that gave up, [16] u32 group ticket,
-// [64, 64 + 8*kPartials) u64 partial counts.
-constexpr size_t kOffTicket = 16, kOffPartials = 64;
 
-Layout make_layout(uint64_t nA, uint64_t nB, uint64_t S) {
+Layout make_layout(uint64_t nA, uint64_t nB) {
     Layout L;
-    L.nTiles = (nA + S - 1) / S + (nB + S - 1) / S + 1;
-    size_t o = align_up(kOffPartials + 8 * kPartials, 256);
+    L.nTiles = std::max<uint64_t>(1, (nA + nB + kTile - 1) / kTile);
+    size_t o = kIpHeader;
     L.off_status = o;
     o = align_up(o + L.nTiles * 8, 256);
-    L.off_split_a = o;
+    L.off_split = o;
     o = align_up(o + (L.nTiles + 1) * 8, 256);
-    L.off_split_b = o;
-    o = align_up(o + (L.nTiles + 1) * 8, 256);
-    L.off_samples = o;
-    o += pivot_samples_bytes(nA, nB, S);
     L.total = o;
     return L;
 }
 
-// K3: persistent, warp-specialised tile pipeline.
-//
-//   warps 0..8  consumers: intersect one tile at a time out of the input ring
-//   warp  9     producer:  takes its groups of tiles in order, reads their
-//                          splits, stages each tile's A and B ranges into the
-//                          input ring with the bulk-copy engine
-//   warp 10     output:    per tile, the tile's global output offset (a
-//                          decoupled look-back once per group, then a running
-//                          sum), then copies the tile's matches from the
-//                          output ring to global memory
-//
-// Input ring: a variable-size, in-order circular buffer (a tile takes about
-// |A_t| + |B_t| elements); descriptors pass through kSlots full/empty
-// mbarrier pairs.  Every consumer warp arrives on a tile's empty barrier when
-// done with it; the producer learns which ring space is free from those
-// barriers, in tile order.  With element output, consumers write a tile's
-// matches into an output ring (power-of-two, indexed modulo its size, so every
-// consumer thread tracks its head without a broadcast) and release the input
-// tile at once; the output warp places them once the tile's offset is known.
-// Offsets therefore never hold up merging.  Groups of
-// kGroup consecutive tiles are handed out by a ticket counter, so a
-// look-back only ever waits on tiles owned by CTAs that are already running
-// (the launch is also cooperative: every CTA is resident).
-constexpr int kConsumerWarps = 9;  // 288 threads: odd VT of the largest tile stays <= 31
-constexpr int kConsumers = kConsumerWarps * 32;
-constexpr int kProducerWarp = kConsumerWarps;
-constexpr int kOutputWarp = kConsumerWarps + 1;
-constexpr int kBlock = (kConsumerWarps + 2) * 32;
-constexpr int kCtasPerSm = 2;
-constexpr int kSlots = 8;
-constexpr int kOutQ = 16;                    // output descriptors in flight
-constexpr int kGroup = 4;                    // consecutive tiles per scheduling unit (one look-back each)
-constexpr uint32_t kInRing = 18432;          // u32: 72 KiB, about three average tiles
-constexpr uint32_t kOutRing = 8192;          // u32: 32 KiB, a power of two
-// Shared memory: input ring and output ring, 104 KiB: two CTAs per SM.
-constexpr size_t kTileSmem = size_t(kInRing + kOutRing) * sizeof(uint32_t);
-static_assert((kOutRing & (kOutRing - 1)) == 0, "output ring is indexed modulo its size");
-static_assert(kS <= kOutRing, "one tile's matches must fit the output ring");
-constexpr uint32_t kEndTile = 0xffffffffu;
-constexpr uint32_t kConsumerBar = 1;  // named barrier id of the consumer warps
+// A elements among the first d merged ones (A first on ties): the first i with
+// A[i] > B[d - 1 - i], by a warp.
+__device__ __forceinline__ uint64_t warp_diagonal(const uint32_t* __restrict__ A, const uint32_t* __restrict__ B,
+                                                  uint64_t d, uint64_t lo, uint64_t hi) {
+    return warp_first_true(lo, hi, [&](uint64_t i) { return __ldg(A + i) > __ldg(B + d - 1 - i); });
+}
 
-static_assert(2 * (kS + 8) + 16 <= kInRing, "a tile's aligned superset must fit the input ring");
-static_assert((((2 * kS + kConsumers - 1) / kConsumers) | 1) <= 63, "per-thread match mask is 64 bits");
-static_assert(kGroup + 1 <= 32, "a group's split entries are held one per lane");
+// Splits of tiles 0, step, 2 step, ... and nTiles; clears the header, the
+// look-back status and the count.
+__global__ void __launch_bounds__(256) ip_split_kernel(const uint32_t* __restrict__ A, uint64_t nA,
+                                                       const uint32_t* __restrict__ B, uint64_t nB, uint64_t nTiles,
+                                                       uint32_t step, uint64_t* __restrict__ split,
+                                                       uint64_t* __restrict__ zero, uint64_t nzero,
+                                                       uint64_t* __restrict__ d_count) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint64_t tid = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, threads = uint64_t(gridDim.x) * blockDim.x;
+    for (uint64_t i = tid; i < nzero; i += threads) zero[i] = 0;
+    if (tid == 0) {
+        *d_count = 0;
+        split[0] = 0;
+        split[nTiles] = nA;
+    }
+    for (uint64_t t = (tid / 32 + 1) * step; t < nTiles; t += threads / 32 * step) {
+        const uint64_t d = t * kTile;
+        const uint64_t s = warp_diagonal(A, B, d, d > nB ? d - nB : 0, d < nA ? d : nA);
+        if ((threadIdx.x & 31) == 0) split[t] = s;
+    }
+}
 
-struct InDesc {
-    uint32_t tile;
-    uint32_t offA, offB;  // ring offsets of element 0 of the staged A / B ranges
-    int na, nb;
-    uint32_t fast;        // both successor elements staged: sentinel-terminated merge
-};
+// The splits between those of every kCoarse-th tile, one thread each.
+__global__ void __launch_bounds__(256) ip_fine_kernel(const uint32_t* __restrict__ A, const uint32_t* __restrict__ B,
+                                                      uint64_t nTiles, uint64_t n, uint64_t* split) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the coarse splits
+    for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < nTiles; t += uint64_t(gridDim.x) * blockDim.x) {
+        if (t % kCoarse == 0) continue;
+        const uint64_t t0 = t / kCoarse * kCoarse, t1 = min(t0 + kCoarse, nTiles);
+        const uint64_t a0 = split[t0], a1 = split[t1], d = t * kTile;
+        const uint64_t b0 = t0 * kTile - a0, b1 = min(t1 * kTile, n) - a1;
+        uint64_t lo = d > b1 ? max(a0, d - b1) : a0;
+        const uint64_t hi = min(a1, d - b0);
+        uint64_t len = hi > lo ? hi - lo : 0;
+        while (len > 0) {
+            const uint64_t half = len >> 1, i = lo + half;
+            const bool before = __ldg(A + i) <= __ldg(B + d - 1 - i);
+            lo = before ? i + 1 : lo;
+            len = before ? len - half - 1 : half;
+        }
+        split[t] = lo;
+    }
+}
 
 constexpr int kLookBackPerLane = 4;  // status words per lane per round trip
 __device__ __forceinline__ uint64_t look_back(uint64_t* status, uint64_t t, uint32_t* err) {
-    // Warp-wide; returns the exclusive prefix of tile t (t > 0).  Flag and
+    // Warp-wide; returns the exclusive prefix of group t (t > 0).  Flag and
     // value share one 64-bit word, so relaxed accesses suffice.  Each round
     // trip reads the 128 nearest unvisited predecessors, lane l holding
     // tiles base - 4l - 1 ... base - 4l - 4.
@@ -183,412 +204,353 @@ __device__ __forceinline__ uint64_t look_back(uint64_t* status, uint64_t t, uint
     }
 }
 
-// ---------------------------------------------------------------------------
-// Per-tile inner algorithms.  Each consumer thread ends with the matches it
-// owns as a bit mask over a contiguous run of one staged set: the matched
-// values are src[start + x] for every set bit x, in ascending order, and the
-// runs of consecutive threads are consecutive.
-// (kBitmapProbe and kHashProbe select the stream engine of si_sisi_bitmap.cu,
-// with window bitmaps or window hash tables.)
-enum Inner { kMergePath = 0, kBitmapProbe = 1, kHashProbe = 2 };
-
-struct ThreadMatches {
-    const uint32_t* src;
-    int start;
-    uint64_t mask;
+// A tile's ranges and where they are staged.
+struct TileRange {
+    uint64_t a0, a1, b0, b1;
+    __device__ __forceinline__ uint32_t na() const { return static_cast<uint32_t>(a1 - a0); }
+    __device__ __forceinline__ uint32_t nb() const { return static_cast<uint32_t>(b1 - b0); }
 };
 
-// Merge path (the reference's intersect-path, include/helpers.cuh:24-61): the
-// thread takes diagonals [d0, d0 + VT) of the tile's merge of A and B, finds
-// its split with a branch-free binary search (A first on ties) and merges
-// serially; a match is recorded when an A element is consumed while the head
-// of B equals it.
-__device__ __forceinline__ ThreadMatches merge_inner(const uint32_t* sA, int na, const uint32_t* sB, int nb,
-                                                     bool fast, int tid) {
-    const int L = na + nb;
-    // Odd steps per thread: consecutive threads then start VT/2 (a non-integer)
-    // words apart in each set, which spreads their shared loads over the banks.
-    const int VT = ((L + kConsumers - 1) / kConsumers) | 1;
-    const int d0 = min(tid * VT, L), d1 = min(d0 + VT, L);
-    int lo = max(0, d0 - nb), len = min(d0, na) - lo;
+__device__ __forceinline__ TileRange tile_range(uint64_t t, uint64_t nA, uint64_t nB, const uint64_t* split,
+                                                uint64_t nTiles, uint32_t* err) {
+    TileRange r;
+    r.a0 = nTiles > 1 ? split[t] : 0;
+    r.a1 = nTiles > 1 ? split[t + 1] : nA;
+    r.b0 = t * kTile - r.a0;
+    r.b1 = min((t + 1) * kTile, nA + nB) - r.a1;
+    const bool sane = r.a0 <= r.a1 && r.a1 <= nA && r.a1 - r.a0 <= kTile && r.b0 <= r.b1 && r.b1 <= nB &&
+                      r.b1 - r.b0 <= kTile;
+    if (!sane) {  // only sets that are not sorted split like this
+        if (threadIdx.x == 0) record_error(err, SI_ERR_INVALID_INPUT, 12, static_cast<uint32_t>(t));
+        r.a0 = r.a1 = r.b0 = r.b1 = 0;
+    }
+    return r;
+}
+
+// Where a tile's ranges lie in its stage: each range and its successor, at
+// their 16-byte phase; every 16-byte block copied holds an element of its set.
+struct Staging {
+    const void *a_src, *b_src;
+    uint32_t bytes_a, bytes_b;
+    uint32_t a_at, b_at;  // words of the stage where the first elements are
+    __device__ __forceinline__ Staging(const uint32_t* A, uint64_t nA, const uint32_t* B, uint64_t nB,
+                                       const TileRange& r) {
+        const uint64_t a_end = r.a1 < nA ? r.a1 + 1 : r.a1, b_end = r.b1 < nB ? r.b1 + 1 : r.b1;
+        const uintptr_t a_lo = reinterpret_cast<uintptr_t>(A + r.a0) & ~uintptr_t(15);
+        const uintptr_t b_lo = reinterpret_cast<uintptr_t>(B + r.b0) & ~uintptr_t(15);
+        a_src = reinterpret_cast<const void*>(a_lo);
+        b_src = reinterpret_cast<const void*>(b_lo);
+        bytes_a = a_end > r.a0
+                      ? static_cast<uint32_t>(((reinterpret_cast<uintptr_t>(A + a_end) + 15) & ~uintptr_t(15)) - a_lo)
+                      : 0u;
+        bytes_b = b_end > r.b0
+                      ? static_cast<uint32_t>(((reinterpret_cast<uintptr_t>(B + b_end) + 15) & ~uintptr_t(15)) - b_lo)
+                      : 0u;
+        a_at = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(A + r.a0) & 15u) >> 2);
+        // (+ 4: room for A's end mark)
+        b_at = bytes_a / 4 + 4 + static_cast<uint32_t>((reinterpret_cast<uintptr_t>(B + r.b0) & 15u) >> 2);
+    }
+    // By one thread.
+    __device__ __forceinline__ void issue(uint32_t* stage, uint64_t* landed) const {
+        mbar_arrive_expect_tx(landed, bytes_a + bytes_b);
+        if (bytes_a) bulk_g2s(stage, a_src, bytes_a, landed);
+        if (bytes_b) bulk_g2s(stage + (b_at & ~3u), b_src, bytes_b, landed);
+    }
+};
+
+// Waits for the staged tile and merges it along its path: the thread's A
+// elements r.a0 + i0 + x with bit x of the mask set are in B.  False when the
+// wait gave up (in every thread).
+__device__ __forceinline__ bool merge_tile(uint64_t nA, uint64_t nB, const TileRange& r, const Staging& st, uint64_t t,
+                                           uint32_t* staged, uint64_t* landed, uint32_t phase, uint32_t* err,
+                                           uint32_t& mask, uint32_t& i0) {
+    const uint32_t tid = threadIdx.x;
+    const uint32_t na = r.na(), nb = r.nb(), total = na + nb;
+    uint32_t *sA = staged + st.a_at, *sB = staged + st.b_at;
+    const bool ok = mbar_wait_bounded(landed, phase, err, 5, static_cast<uint32_t>(t));
+    const bool ends = r.a1 == nA && r.b1 == nB;
+    if (r.a1 == nA && tid == 0) sA[na] = 0xffffffffu;
+    if (r.b1 == nB && tid == 1) sB[nb] = 0xffffffffu;
+    if (!__syncthreads_and(ok)) return false;
+    mask = 0;
+    i0 = 0;
+    if (na == 0) return true;
+    const uint32_t d0 = min(tid * kVT, total), d1 = min(d0 + kVT, total);
+    uint32_t lo = d0 > nb ? d0 - nb : 0u, len = min(d0, na) - lo;
     while (len > 0) {
-        const int half = len >> 1, mid = lo + half;
+        const uint32_t half = len >> 1, mid = lo + half;
         const bool c = sA[mid] <= sB[d0 - 1 - mid];
         lo = c ? mid + 1 : lo;
         len = c ? len - half - 1 : half;
     }
-    const int i0 = lo;
-    uint64_t mask = 0;  // bit x: A element i0 + x is in B
-    if (fast) {
-        // sA[na] / sB[nb] are the successor elements of the ranges, both at or
-        // above the next pivot and so above every value of the tile: they stop
-        // each side without bounds checks.  One shared load per step, through
-        // 32-bit shared-window byte addresses.
-        uint32_t pa = smem_addr(sA + i0), pb = smem_addr(sB + (d0 - i0));
-        uint32_t a = lds_u32(pa), b = lds_u32(pb), ka = 0;
-        const int steps = d1 - d0;
-#pragma unroll 4
-        for (int s = 0; s < steps; ++s) {
-            const bool takeA = a <= b;
-            mask |= static_cast<uint64_t>(a == b) << ka;
-            ka += takeA ? 1u : 0u;
-            pa += takeA ? 4u : 0u;
-            pb += takeA ? 0u : 4u;
-            const uint32_t v = lds_u32(takeA ? pa : pb);
-            a = takeA ? v : a;
-            b = takeA ? b : v;
+    i0 = lo;
+    // The heads after the ranges' ends are the successors, or 2^32 - 1 past the
+    // end of a set: right as long as the other set does not hold that value
+    // here, which only its last element can be.
+    const bool top = ends && (sA[na - 1] == 0xffffffffu || (nb && sB[nb - 1] == 0xffffffffu));
+    if (!top) {
+        uint32_t pa = smem_addr(sA + i0), pb = smem_addr(sB + (d0 - i0)), bit = 1;
+        uint32_t a = lds_u32(pa), b = lds_u32(pb);
+        auto merge_step = [&]() {
+            if (a == b) mask |= bit;
+            if (a <= b) {
+                bit <<= 1;
+                pa += 4;
+                a = lds_u32(pa);
+            } else {
+                pb += 4;
+                b = lds_u32(pb);
+            }
+        };
+        if (total == kTile) {
+#pragma unroll
+            for (int s = 0; s < kVT; ++s) merge_step();
+        } else {
+            for (uint32_t s = d0; s < d1; ++s) merge_step();
         }
     } else {
-        int i = i0, j = d0 - i0;
-        for (int s = d0; s < d1; ++s) {
-            const bool aOk = i < na, bOk = j < nb;
-            const uint32_t a = aOk ? sA[i] : 0u, b = bOk ? sB[j] : 0u;
-            const bool takeA = aOk && (!bOk || a <= b);
-            if (takeA && bOk && a == b) mask |= 1ull << (i - i0);
-            if (takeA) ++i; else ++j;
+        uint32_t i = i0, j = d0 - i0;
+        for (uint32_t s = d0; s < d1; ++s) {
+            const bool a_ok = i < na, b_ok = j < nb;
+            const uint32_t a = a_ok ? sA[i] : 0u, b = b_ok ? sB[j] : 0u;
+            const bool take_a = a_ok && (!b_ok || a <= b);
+            if (take_a && b_ok && a == b) mask |= 1u << (i - i0);
+            if (take_a) ++i; else ++j;
         }
     }
-    return {sA, i0, mask};
+    return true;
 }
 
-template <bool kOut>
-__global__ void __launch_bounds__(kBlock, kCtasPerSm) ip_tile_kernel(
-    const uint32_t* __restrict__ A, uint64_t nA, const uint32_t* __restrict__ B, uint64_t nB,
-    const uint64_t* __restrict__ split_a, const uint64_t* __restrict__ split_b, uint64_t nTiles,
-    unsigned char* __restrict__ ws, uint64_t* __restrict__ status, uint32_t* __restrict__ out, uint64_t out_cap,
-    uint64_t* __restrict__ d_count) {
-    extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* in_ring = smem;
-    constexpr uint32_t kRing = kInRing;
-    constexpr uint64_t kTileMax = kS;
-    uint32_t* out_ring = smem + kRing;
-    __shared__ __align__(8) uint64_t full[kSlots], empty[kSlots], ofull[kOutQ], oempty[kOutQ];
-    __shared__ __align__(8) uint64_t s_released_out;  // output ring: virtual offset written out so far
-    __shared__ uint32_t s_otile[kOutQ], s_ocount[kOutQ];
-    __shared__ uint64_t s_ostart[kOutQ];
-    __shared__ InDesc in_desc[kSlots];
-    __shared__ uint64_t s_in_end[kSlots];  // producer-private: ring end of the tile in each slot
-    __shared__ uint32_t s_warp[2][kConsumerWarps];  // by tile parity: a warp may run one tile ahead
+// Matches before this thread's in the tile, and the tile's (two barriers' worth
+// of s_warp: the caller synchronises before the next call).
+__device__ __forceinline__ uint32_t tile_scan(uint32_t cnt, uint32_t* s_warp, uint32_t& tile_count) {
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t incl = warp_inclusive_scan(cnt);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = incl - cnt;
+    tile_count = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < kIpWarps; ++w) {
+        before += w < warp ? s_warp[w] : 0u;
+        tile_count += s_warp[w];
+    }
+    return before;
+}
 
-    uint32_t* err = reinterpret_cast<uint32_t*>(ws);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// One tile per CTA.  kCount: its matches are added to the count.  kTileCounts:
+// they are stored, for a kPlace launch after it, which merges the tile again
+// and writes its matches behind those of the tiles before it.  A pair of one
+// tile needs kPlace alone.
+enum TileMode { kCount = 0, kTileCounts = 1, kPlace = 2 };
+template <int kMode>
+__global__ void __launch_bounds__(kIpThreads, kIpCtasPerSm) ip_tile_kernel(
+    const uint32_t* __restrict__ A, uint64_t nA, const uint32_t* __restrict__ B, uint64_t nB, const uint64_t* split,
+    uint64_t nTiles, uint32_t* header, uint32_t* tile_counts, uint32_t* __restrict__ out, uint64_t out_cap,
+    uint64_t* __restrict__ d_count) {
+    __shared__ __align__(16) uint32_t staged[kStaged];
+    __shared__ __align__(8) uint64_t landed;
+    __shared__ uint32_t s_warp[kIpWarps];
+    __shared__ uint64_t s_sum[kIpWarps];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t t = blockIdx.x;
     if (tid == 0) {
-        for (int i = 0; i < kSlots; ++i) {
-            mbar_init(&full[i], 1);
-            mbar_init(&empty[i], kConsumerWarps);
+        mbar_init(&landed, 1);
+        fence_mbar_init();
+    }
+    if (nTiles == 1) {
+        if (tid < kIpHeader / 4) header[tid] = 0;
+    } else {
+        if (kMode == kTileCounts) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the splits and the cleared header; the tiles' counts
+    }
+    __syncthreads();
+    const TileRange r = tile_range(t, nA, nB, split, nTiles, header);
+    uint64_t sum = 0;
+    if (kMode == kPlace && nTiles > 1) {  // the matches of the tiles before this one
+        for (uint64_t x = tid; x < t; x += kIpThreads) sum += __ldcg(tile_counts + x);
+        sum = warp_sum_u64(sum);
+        if (lane == 0) s_sum[warp] = sum;
+    }
+    const Staging st(A, nA, B, nB, r);
+    if (tid == 0) st.issue(staged, &landed);
+    uint32_t mask, i0;
+    if (!merge_tile(nA, nB, r, st, t, staged, &landed, 0, header, mask, i0)) return;
+    const uint32_t cnt = __popc(mask);
+    uint32_t tile_count;
+    const uint32_t before = tile_scan(cnt, s_warp, tile_count);
+    if constexpr (kMode == kCount) {
+        if (tid == 0) {
+            if (nTiles == 1) *d_count = tile_count;
+            else if (tile_count) atomicAdd(reinterpret_cast<unsigned long long*>(d_count), tile_count);
         }
-        for (int i = 0; i < kOutQ; ++i) {
-            mbar_init(&ofull[i], kConsumerWarps);  // every consumer warp has written its matches
-            mbar_init(&oempty[i], 1);
+    } else if constexpr (kMode == kTileCounts) {
+        if (tid == 0) tile_counts[t] = tile_count;
+    } else {
+        uint64_t prefix = 0;
+        if (nTiles > 1)
+#pragma unroll
+            for (uint32_t w = 0; w < kIpWarps; ++w) prefix += s_sum[w];
+        const uint32_t* mine = staged + st.a_at + i0;
+        uint64_t pos = prefix + before;
+        bool overflow = false;
+        for (uint32_t m = mask; m; m &= m - 1, ++pos) {
+            if (pos < out_cap) out[pos] = mine[__ffs(m) - 1];
+            else overflow = true;
         }
-        s_released_out = 0;
+        if (overflow) record_error(header, SI_ERR_OUTPUT_OVERFLOW, 9, static_cast<uint32_t>(t));
+        if (tid == 0 && t + 1 == nTiles) *d_count = prefix + tile_count;
+    }
+}
+
+// Element output of many tiles in one pass: persistent CTAs take groups of
+// kGroup consecutive tiles round robin, merge them, find the group's offset by
+// a decoupled look-back over the groups before it and write the matches from
+// the sets (a group's tiles are still in L2).  A group's look-back and writes
+// come after the next group's merge, when the groups before it have long
+// published their counts.  The launch is cooperative: all CTAs are resident and
+// a CTA's groups come in order, so a look-back only waits for groups that are
+// being merged.
+constexpr uint32_t kGroup = 4;
+struct GroupMatches {
+    uint32_t mask[kGroup][kIpThreads];  // each thread's own
+    uint16_t i0[kGroup][kIpThreads], before[kGroup][kIpThreads];
+    uint32_t count[kGroup];
+};
+__global__ void __launch_bounds__(kIpThreads, kIpCtasPerSm) ip_group_kernel(
+    const uint32_t* __restrict__ A, uint64_t nA, const uint32_t* __restrict__ B, uint64_t nB, const uint64_t* split,
+    uint64_t nTiles, uint32_t* header, uint64_t* status, uint32_t* __restrict__ out, uint64_t out_cap,
+    uint64_t* __restrict__ d_count) {
+    __shared__ __align__(16) uint32_t staged[kStaged];
+    __shared__ __align__(8) uint64_t landed;
+    __shared__ uint32_t s_warp[kIpWarps];
+    __shared__ GroupMatches s_group[2];
+    __shared__ uint64_t s_prefix;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) {
+        mbar_init(&landed, 1);
         fence_mbar_init();
     }
     __syncthreads();
-
-    if (warp == kProducerWarp) {
-        // ------------------------------------------------------ producer --
-        // Groups of kGroup consecutive tiles are handed out by a ticket
-        // counter, so groups complete roughly in global order and a
-        // look-back finds an inclusive prefix nearby.  Tickets are fetched
-        // two groups ahead and split entries one group ahead, so neither
-        // latency stalls the staging.  Lane x computes the staging parameters
-        // of the group's tile x.
-        uint32_t* ticket = reinterpret_cast<uint32_t*>(ws + kOffTicket);
-        uint64_t head = 0, released = 0;  // virtual ring offsets (lane 0)
-        uint32_t k = 0, k_rel = 0;        // tiles staged / tiles known released
-        bool done = false;
-        auto load_splits = [&](uint64_t grp, uint64_t& sa_, uint64_t& sb_) {
-            const uint64_t idx = grp * kGroup + lane;
-            sa_ = (lane <= kGroup && idx <= nTiles) ? split_a[idx] : 0;
-            sb_ = (lane <= kGroup && idx <= nTiles) ? split_b[idx] : 0;
-        };
-        // lane 0: wait for the oldest staged tile to be released by every consumer warp
-        auto wait_release = [&]() -> bool {
-            const uint32_t sl = k_rel % kSlots;
-            if (!mbar_wait_bounded(&empty[sl], (k_rel / kSlots) & 1, err, 2, k_rel)) return false;
-            released = s_in_end[sl];
-            ++k_rel;
-            return true;
-        };
-        uint32_t tk0 = 0, tk1 = 0;
-        if (lane == 0) {
-            tk0 = atomicAdd(ticket, 1u);
-            tk1 = atomicAdd(ticket, 1u);
-        }
-        uint64_t g = __shfl_sync(kFullMask, tk0, 0);
-        uint64_t g_next = __shfl_sync(kFullMask, tk1, 0);
-        uint64_t sp_a, sp_b;
-        load_splits(g, sp_a, sp_b);
-        while (!done) {
-            const uint64_t t_first = g * kGroup;
-            uint32_t tk2 = 0;
-            if (lane == 0 && t_first < nTiles) tk2 = atomicAdd(ticket, 1u);  // two groups ahead
-            uint64_t nsp_a, nsp_b;
-            load_splits(g_next, nsp_a, nsp_b);  // in flight while this group is staged
-            // ---- lane x: parameters of tile t_first + x ----
-            uint64_t a0 = __shfl_sync(kFullMask, sp_a, lane < kGroup ? lane : 0);
-            uint64_t a1 = __shfl_sync(kFullMask, sp_a, lane < kGroup ? lane + 1 : 1);
-            uint64_t b0 = __shfl_sync(kFullMask, sp_b, lane < kGroup ? lane : 0);
-            uint64_t b1 = __shfl_sync(kFullMask, sp_b, lane < kGroup ? lane + 1 : 1);
-            const bool ok = a0 <= a1 && a1 <= nA && a1 - a0 <= kTileMax && b0 <= b1 && b1 <= nB && b1 - b0 <= kTileMax;
-            const uint64_t t_mine = t_first + lane;
-            if (!ok && lane < kGroup && t_mine < nTiles) record_error(err, SI_ERR_INVALID_INPUT);
-            if (!ok) a0 = a1 = b0 = b1 = 0;
-            // 16-byte aligned superset of [x0, x1] (x1, the successor element
-            // when it exists, doubles as the merge sentinel).  Every 16-byte
-            // block copied holds at least one element of the range.
-            const uint64_t aEnd = a1 < nA ? a1 + 1 : a1, bEnd = b1 < nB ? b1 + 1 : b1;
-            const uintptr_t a_lo = reinterpret_cast<uintptr_t>(A + a0) & ~uintptr_t(15);
-            const uintptr_t b_lo = reinterpret_cast<uintptr_t>(B + b0) & ~uintptr_t(15);
-            const uint32_t bytesA =
-                aEnd > a0 ? static_cast<uint32_t>(((reinterpret_cast<uintptr_t>(A + aEnd) + 15) & ~uintptr_t(15)) - a_lo)
-                          : 0u;
-            const uint32_t bytesB =
-                bEnd > b0 ? static_cast<uint32_t>(((reinterpret_cast<uintptr_t>(B + bEnd) + 15) & ~uintptr_t(15)) - b_lo)
-                          : 0u;
-            const uint32_t needA = bytesA / 4 + 4, needB = bytesB / 4 + 4;  // (+4: room for misalignment)
-            const uint32_t misA = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(A + a0) & 15u) >> 2);
-            const uint32_t misB = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(B + b0) & 15u) >> 2);
-            const uint32_t fast = (t_mine + 1 < nTiles) && a1 < nA && b1 < nB;
-            for (int x = 0; x < kGroup; ++x) {
-                const uint64_t t = t_first + x;
-                const uint32_t slot = k % kSlots;
-                const uint64_t xa_lo = __shfl_sync(kFullMask, static_cast<uint64_t>(a_lo), x);
-                const uint64_t xb_lo = __shfl_sync(kFullMask, static_cast<uint64_t>(b_lo), x);
-                const uint32_t xbytesA = __shfl_sync(kFullMask, bytesA, x), xbytesB = __shfl_sync(kFullMask, bytesB, x);
-                const uint32_t xneedA = __shfl_sync(kFullMask, needA, x), xneedB = __shfl_sync(kFullMask, needB, x);
-                const uint32_t xmisA = __shfl_sync(kFullMask, misA, x), xmisB = __shfl_sync(kFullMask, misB, x);
-                const uint32_t xna = __shfl_sync(kFullMask, static_cast<uint32_t>(a1 - a0), x);
-                const uint32_t xnb = __shfl_sync(kFullMask, static_cast<uint32_t>(b1 - b0), x);
-                const uint32_t xfast = __shfl_sync(kFullMask, fast, x);
-                if (lane == 0) {
-                    // the slot's previous tile (k - kSlots) must be released by
-                    // every consumer warp before the slot is written, also for
-                    // the end marker
-                    bool alive = true;
-                    while (alive && k_rel + kSlots <= k) alive = wait_release();
-                    const bool slot_free = alive;
-                    alive = alive && t < nTiles;
-                    const uint32_t need = xneedA + xneedB;
-                    if (alive) {
-                        // A tile never wraps: if it does not fit before the ring's end it
-                        // starts the next lap.  It may be placed once it overlaps no live
-                        // tile: either every staged tile is released, or the live span
-                        // [released, head) ends at least kRing before the tile's end.
-                        const uint64_t phys = head % kRing;
-                        if (phys + need > kRing) head += kRing - phys;
-                        while (alive && k_rel < k && head + need - released > kRing) alive = wait_release();
-                    }
-                    if (!alive) {
-                        if (t < nTiles) record_error(err, SI_ERR_TIMEOUT, 3, static_cast<uint32_t>(t));
-                        if (slot_free) {  // else the consumers' own bounded waits end them
-                            in_desc[slot].tile = kEndTile;
-                            mbar_arrive(&full[slot]);
-                        }
-                    } else {
-                        const uint32_t base = static_cast<uint32_t>(head % kRing);
-                        head += need;
-                        s_in_end[slot] = head;
-                        InDesc& d = in_desc[slot];
-                        d.tile = static_cast<uint32_t>(t);
-                        d.offA = base + xmisA;
-                        d.offB = base + xneedA + xmisB;
-                        d.na = static_cast<int>(xna);
-                        d.nb = static_cast<int>(xnb);
-                        d.fast = xfast;
-                        mbar_arrive_expect_tx(&full[slot], xbytesA + xbytesB);
-                        if (xbytesA) bulk_g2s(in_ring + base, reinterpret_cast<const void*>(xa_lo), xbytesA, &full[slot]);
-                        if (xbytesB)
-                            bulk_g2s(in_ring + base + xneedA, reinterpret_cast<const void*>(xb_lo), xbytesB, &full[slot]);
-                    }
-                    done = !alive;
-                }
-                done = __shfl_sync(kFullMask, done ? 1u : 0u, 0) != 0;
-                if (done) break;
-                ++k;
+    uint32_t phase = 0, total = 0, last_total = 0;
+    const uint64_t nGroups = (nTiles + kGroup - 1) / kGroup;
+    uint32_t buf = 0;
+    for (uint64_t g = blockIdx.x; g < nGroups + gridDim.x; g += gridDim.x, buf ^= 1) {
+        const uint64_t t0 = g * kGroup;
+        if (g < nGroups) {
+            GroupMatches& gm = s_group[buf];
+            const uint32_t n = static_cast<uint32_t>(min(uint64_t(kGroup), nTiles - t0));
+            total = 0;
+            for (uint32_t q = 0; q < n; ++q) {
+                const TileRange r = tile_range(t0 + q, nA, nB, split, nTiles, header);
+                const Staging st(A, nA, B, nB, r);
+                if (tid == 0) st.issue(staged, &landed);
+                uint32_t mask, i0, count;
+                if (!merge_tile(nA, nB, r, st, t0 + q, staged, &landed, phase, header, mask, i0)) return;
+                phase ^= 1;
+                const uint32_t before = tile_scan(__popc(mask), s_warp, count);
+                gm.mask[q][tid] = mask;
+                gm.i0[q][tid] = static_cast<uint16_t>(i0);
+                gm.before[q][tid] = static_cast<uint16_t>(before);
+                if (tid == 0) gm.count[q] = count;
+                total += count;
+                // the tile is read before the next one is copied over it
+                fence_proxy_async_smem();
+                __syncthreads();
             }
-            g = g_next;
-            g_next = __shfl_sync(kFullMask, tk2, 0);
-            sp_a = nsp_a;
-            sp_b = nsp_b;
+            if (tid == 0) st_relaxed_u64(status + g, (g == 0 ? kFlagInc : kFlagAgg) | total);
         }
-        return;
-    }
-
-    if (warp == kOutputWarp) {
-        // -------------------------------------------------------- output --
-        // For each tile this CTA consumed, in order: its exclusive prefix (a
-        // look-back for the first tile of a group, else the running sum), its
-        // inclusive prefix published, its matches copied to global memory.
-        if constexpr (kOut) {
-            uint64_t prefix = 0;
-            for (uint32_t k = 0;; ++k) {
-                const uint32_t q = k % kOutQ;
-                if (!mbar_wait_bounded(&ofull[q], (k / kOutQ) & 1u, err, 4, k)) break;
-                const uint32_t t = s_otile[q], count = s_ocount[q];
-                const uint64_t start = s_ostart[q];
-                if (t == kEndTile) break;
-                if (t % kGroup == 0) prefix = t > 0 ? look_back(status, t, err) : 0;
-                if (t > 0 && lane == 0) st_relaxed_u64(status + t, kFlagInc | ((prefix + count) & kValMask));
-                bool overflow = false;
-                for (uint32_t x = lane; x < count; x += 32) {
-                    const uint64_t pos = prefix + x;
-                    if (pos < out_cap) out[pos] = out_ring[(start + x) & (kOutRing - 1)];
+        if (g >= gridDim.x) {  // the group before, gd
+            const uint64_t gd = g - gridDim.x, td = gd * kGroup;
+            if (gd >= nGroups) break;
+            if (warp == 0) {
+                const uint64_t p = gd > 0 ? look_back(status, gd, header) : 0;
+                if (lane == 0) {
+                    if (gd > 0) st_relaxed_u64(status + gd, kFlagInc | ((p + last_total) & kValMask));
+                    s_prefix = p;
+                }
+            }
+            __syncthreads();
+            uint64_t prefix = s_prefix;
+            const GroupMatches& gm = s_group[buf ^ 1];
+            const uint32_t n = static_cast<uint32_t>(min(uint64_t(kGroup), nTiles - td));
+            bool overflow = false;
+            for (uint32_t q = 0; q < n; ++q) {
+                const uint32_t* mine = A + split[td + q] + gm.i0[q][tid];
+                uint64_t pos = prefix + gm.before[q][tid];
+                for (uint32_t m = gm.mask[q][tid]; m; m &= m - 1, ++pos) {
+                    if (pos < out_cap) out[pos] = __ldg(mine + __ffs(m) - 1);
                     else overflow = true;
                 }
-                if (overflow) record_error(err, SI_ERR_OUTPUT_OVERFLOW, 9, t);
-                prefix += count;
-                if (lane == 0 && t + 1 == nTiles) *d_count = prefix;
-                __syncwarp();
-                if (lane == 0) {
-                    st_release_shared_u64(&s_released_out, start + count);
-                    mbar_arrive(&oempty[q]);
-                }
+                prefix += gm.count[q];
             }
+            if (overflow) record_error(header, SI_ERR_OUTPUT_OVERFLOW, 9, static_cast<uint32_t>(gd));
+            if (tid == 0 && td + n == nTiles) *d_count = prefix;
+            __syncthreads();  // the group's words are read before a later group writes them
         }
-        return;
-    }
-
-    // ---------------------------------------------------------- consumers --
-    uint64_t my_count = 0;     // count-only: this thread's matches over all its tiles
-    uint64_t ohead = 0;        // element output: virtual output-ring head (same in every thread)
-    uint32_t k = 0;            // tiles consumed so far
-    for (;; ++k) {
-        const uint32_t slot = k % kSlots;
-        bool gave_up = !mbar_wait_bounded(&full[slot], (k / kSlots) & 1, err, 5, k);
-        // Consumers that meet at named barriers (element output) give up
-        // together: a warp leaving alone would leave the others at a barrier
-        // it never reaches, which has no time limit.
-        if constexpr (kOut) gave_up = named_barrier_or(kConsumerBar, kConsumers, gave_up);
-        if (gave_up) break;
-        const InDesc d = in_desc[slot];
-        if (d.tile == kEndTile) break;
-        const uint32_t* sA = in_ring + d.offA;
-        const uint32_t* sB = in_ring + d.offB;
-        const ThreadMatches tm = merge_inner(sA, d.na, sB, d.nb, d.fast != 0, tid);
-        const uint32_t cnt = static_cast<uint32_t>(__popcll(tm.mask));
-
-        if constexpr (!kOut) {
-            my_count += cnt;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&empty[slot]);  // this warp is done with the tile
-        } else {
-            // block scan over the consumer warps
-            const uint32_t incl = warp_inclusive_scan(cnt);
-            if (lane == 31) s_warp[k & 1][warp] = incl;
-            named_barrier(kConsumerBar, kConsumers);
-            uint32_t wsum = 0, tile_count = 0;
-#pragma unroll
-            for (int w = 0; w < kConsumerWarps; ++w) {
-                const uint32_t v = s_warp[k & 1][w];
-                wsum += w < warp ? v : 0u;
-                tile_count += v;
-            }
-            const uint32_t q = k % kOutQ;
-            if (tid == 0) {
-                // the tile's aggregate goes out at once, for other tiles'
-                // look-backs (before the hand-off below, after which the
-                // output warp overwrites it with the inclusive value)
-                st_relaxed_u64(status + d.tile, (d.tile == 0 ? kFlagInc : kFlagAgg) | tile_count);
-            }
-            // queue entry q and ring space [ohead, ohead + tile_count) must be
-            // free: the output warp has written out what they last held
-            if (lane == 0) mbar_wait_bounded(&oempty[q], ((k / kOutQ) & 1u) ^ 1u, err, 7, k);
-            if (lane == 0 && tile_count) {
-                for (WaitBudget budget;;) {
-                    if (ohead + tile_count - ld_acquire_shared_u64(&s_released_out) <= kOutRing) break;
-                    if (budget.expired()) {
-                        record_error(err, SI_ERR_TIMEOUT, 6, d.tile);
-                        break;
-                    }
-                    __nanosleep(20);
-                }
-            }
-            __syncwarp();
-            uint64_t m = tm.mask;
-            uint64_t pos = ohead + incl - cnt + wsum;
-            while (m) {
-                const int x = __ffsll(m) - 1;
-                m &= m - 1;
-                out_ring[pos++ & (kOutRing - 1)] = tm.src[tm.start + x];
-            }
-            if (tid == 0) {
-                s_otile[q] = d.tile;
-                s_ocount[q] = tile_count;
-                s_ostart[q] = ohead;
-            }
-            ohead += tile_count;
-            __syncwarp();
-            if (lane == 0) {
-                mbar_arrive(&empty[slot]);  // this warp is done with the input tile
-                mbar_arrive(&ofull[q]);     // ... and has written its matches
-            }
-        }
-    }
-    if constexpr (kOut) {
-        if (tid == 0) {  // end marker for the output warp (its own phase of entry q)
-            const uint32_t q = k % kOutQ;
-            mbar_wait_bounded(&oempty[q], ((k / kOutQ) & 1u) ^ 1u, err, 8, k);
-            s_otile[q] = kEndTile;
-            s_ocount[q] = 0;
-            s_ostart[q] = ohead;
-            for (int w = 0; w < kConsumerWarps; ++w) mbar_arrive(&ofull[q]);
-        }
-    } else {
-        const uint64_t wsum = warp_sum_u64(my_count);
-        if (lane == 0 && wsum) atomicAdd(reinterpret_cast<unsigned long long*>(d_count), wsum);
+        last_total = total;
     }
 }
 
 }  // namespace
 
-size_t ip_workspace_size(uint64_t nA, uint64_t nB, int inner) {
-    return inner == kMergePath ? make_layout(nA, nB, kS).total : bm_workspace_size(nA, nB);
-}
+size_t ip_workspace_size(uint64_t nA, uint64_t nB) { return make_layout(nA, nB).total; }
 
 si_status ip_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
-                  uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream, int inner) {
-    if (inner != kMergePath)
-        return bm_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, ws, ws_bytes, stream, inner == kHashProbe);
-    const uint64_t S = kS;
-    const Layout L = make_layout(nA, nB, S);
+                  uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream) {
+    const Layout L = make_layout(nA, nB);
     if (ws_bytes < L.total) return SI_ERR_WORKSPACE_TOO_SMALL;
     if (L.nTiles > 0x7fffffffull) return SI_ERR_INVALID_ARGUMENT;
     unsigned char* w = static_cast<unsigned char*>(ws);
-    uint64_t* split_a = reinterpret_cast<uint64_t*>(w + L.off_split_a);
-    uint64_t* split_b = reinterpret_cast<uint64_t*>(w + L.off_split_b);
     uint64_t* status = reinterpret_cast<uint64_t*>(w + L.off_status);
-    // the split kernel also clears the header, the partial counts and the
-    // tiles' look-back status words
-    uint32_t* samples_a = reinterpret_cast<uint32_t*>(w + L.off_samples);
-    uint32_t* samples_b = samples_a + align_up(((nA + S - 1) / S) * 4, 256) / 4;
-    const si_status sst = pivot_split(dA, nA, dB, nB, S, split_a, split_b, samples_a, samples_b,
-                                      reinterpret_cast<uint64_t*>(w), L.off_split_a / 8, d_count, stream);
-    if (sst != SI_OK) return sst;
-
-    const uint64_t nGroups = (L.nTiles + kGroup - 1) / kGroup;
-    auto launch = [&](auto kernel, uint32_t* out) -> si_status {
-        const size_t smem = kTileSmem;
-        SI_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    uint64_t* split = reinterpret_cast<uint64_t*>(w + L.off_split);
+    uint32_t* header = reinterpret_cast<uint32_t*>(w);
+    const bool fine = L.nTiles > kFineTiles, grouped = d_out && L.nTiles > kPlaceTiles;
+    if (L.nTiles > 1) {
+        PhaseTimer timer("sisi_split", stream);
+        const uint32_t step = fine ? kCoarse : 1;
+        const uint64_t warps = (L.nTiles + step - 1) / step;
+        ip_split_kernel<<<static_cast<unsigned>((warps + 7) / 8), 256, 0, stream>>>(
+            dA, nA, dB, nB, L.nTiles, step, split, reinterpret_cast<uint64_t*>(w),
+            grouped ? L.off_split / 8 : kIpHeader / 8, d_count);
+        SI_LAUNCH_CHECK("ip_split_kernel");
+        if (fine) {
+            const si_status st = launch_dependent(
+                ip_fine_kernel, dim3(static_cast<unsigned>(std::min<uint64_t>((L.nTiles + 255) / 256, 65535))),
+                dim3(256), 0, stream, dA, dB, L.nTiles, nA + nB, split);
+            if (st != SI_OK) return st;
+        }
+    }
+    PhaseTimer timer("sisi_tile", stream);
+    const dim3 grid(static_cast<unsigned>(L.nTiles)), block(kIpThreads);
+    const uint64_t* csplit = split;
+    uint32_t* tile_counts = reinterpret_cast<uint32_t*>(status);
+    if (grouped) {
         int per_sm = 0;
-        SI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, smem));
+        SI_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ip_group_kernel, kIpThreads, 0));
         if (per_sm < 1) return SI_ERR_UNSUPPORTED;
-        const unsigned grid =
+        const uint64_t nGroups = (L.nTiles + kGroup - 1) / kGroup;
+        const unsigned ctas =
             static_cast<unsigned>(std::min<uint64_t>(nGroups, static_cast<uint64_t>(sm_count()) * per_sm));
-        uint64_t cap = out ? out_cap : 0;
         uint64_t nTiles = L.nTiles;
-        void* args[] = {(void*)&dA, (void*)&nA, (void*)&dB, (void*)&nB, (void*)&split_a, (void*)&split_b,
-                        (void*)&nTiles, (void*)&w, (void*)&status, (void*)&out, (void*)&cap, (void*)&d_count};
-        PhaseTimer timer("sisi_tile", stream);
-        SI_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid), dim3(kBlock), args,
-                                                smem, stream));
+        void* args[] = {&dA, &nA, &dB, &nB, &csplit, &nTiles, &header, &status, &d_out, &out_cap, &d_count};
+        SI_CUDA_TRY(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(ip_group_kernel), dim3(ctas), block, args,
+                                                0, stream));
         return SI_OK;
-    };
-    const si_status st = d_out ? launch(ip_tile_kernel<true>, d_out) : launch(ip_tile_kernel<false>, nullptr);
-    if (st != SI_OK) return st;
-    SI_LAUNCH_CHECK("sisi_tile_kernel");
-    return SI_OK;
+    }
+    if (L.nTiles == 1) {
+        const auto kernel = d_out ? ip_tile_kernel<kPlace> : ip_tile_kernel<kCount>;
+        kernel<<<grid, block, 0, stream>>>(dA, nA, dB, nB, csplit, L.nTiles, header, tile_counts, d_out, out_cap,
+                                           d_count);
+        SI_LAUNCH_CHECK("ip_tile_kernel");
+        return SI_OK;
+    }
+    const si_status st =
+        launch_dependent(d_out ? ip_tile_kernel<kTileCounts> : ip_tile_kernel<kCount>, grid, block, 0, stream, dA, nA,
+                         dB, nB, csplit, L.nTiles, header, tile_counts, d_out, out_cap, d_count);
+    if (st != SI_OK || !d_out) return st;
+    return launch_dependent(ip_tile_kernel<kPlace>, grid, block, 0, stream, dA, nA, dB, nB, csplit, L.nTiles, header,
+                            tile_counts, d_out, out_cap, d_count);
 }
 
 }  // namespace si

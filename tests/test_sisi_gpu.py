@@ -290,3 +290,61 @@ def test_obs_lane_groups_and_chunking(cuda, n_small):
         assert small.size == n_small
         check(small, big, "obs")
         check(big, small, "obs")
+
+
+IP_TILE = 192 * 27  # merged elements per tile of the intersect-path kernels
+
+
+@pytest.mark.parametrize("total", [1, IP_TILE - 1, IP_TILE, IP_TILE + 1, 2 * IP_TILE, 7 * IP_TILE + 26,
+                                   2048 * IP_TILE, 2048 * IP_TILE + 1, 4096 * IP_TILE, 4096 * IP_TILE + 1])
+@pytest.mark.parametrize("shape", ["dense", "equal", "uneven", "one_ends_early"])
+def test_ip_tile_edges(cuda, total, shape):
+    """Merged sizes at the edges of a tile, of the double merge (2048 tiles) and
+    of the one-step split (4096); equal pairs across tile boundaries; a set that
+    ends while the other goes on, up to 2^32 - 1; with elements and counting."""
+    rng = np.random.default_rng(total % 1000)
+    na = {"dense": total // 2, "equal": total // 2, "uneven": total // 9, "one_ends_early": total // 3}[shape]
+    nb = total - na if shape != "equal" else na
+    if shape == "equal":
+        a = b = np.arange(5, 5 + 3 * na, 3, dtype=np.uint64)
+    else:
+        step = 2 if shape == "one_ends_early" else max(2, (1 << 31) // max(nb, 1))
+        pick = lambda n: np.cumsum(rng.integers(1, step if step < 1 << 10 else 4, n, dtype=np.uint64))
+        a, b = pick(na), pick(nb)
+        if shape == "one_ends_early" and nb:
+            b[-1] = 0xffffffff
+            if na and total % 2:
+                a[-1] = 0xffffffff
+    a, b = np.unique(a).astype(np.uint32), np.unique(b).astype(np.uint32)
+    want = oracle.set_intersection(a, b)
+    for mat in (True, False):
+        c, got = run(a, b, "ip", materialize=mat)
+        assert c == want.size
+        if mat:
+            np.testing.assert_array_equal(got, want)
+    c, _ = run(b, a, "ip", materialize=False)
+    assert c == want.size
+
+
+@pytest.mark.parametrize("tech", ["ip", "auto"])
+@pytest.mark.parametrize("n", [1000, 300000, 9000000])
+def test_pair_call_in_a_graph(cuda, tech, n):
+    import torch
+    from set_intersection_b200 import api, generate
+    a, b = generate.uniform(61, n, 8 * n), generate.uniform(62, n // 2, 8 * n)
+    want = oracle.set_intersection(a, b)
+    da, db, ws = dev(a), dev(b), api.Workspace()
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    out = torch.zeros(n // 2, dtype=torch.int32, device="cuda")
+    api.sisi_into(da, db, count, out, ws, tech)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        api.sisi_into(da, db, count, out, ws, tech)
+    for _ in range(2):
+        count.fill_(-1)
+        out.zero_()
+        g.replay()
+        assert int(count.item()) == want.size
+        np.testing.assert_array_equal(out[:want.size].cpu().numpy().view(np.uint32), want)
+        assert not out[want.size:].any()
