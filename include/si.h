@@ -234,7 +234,10 @@ si_status si_misi(const uint32_t* d_elements, const uint64_t* d_offsets, si_set_
  * SI_TECH_BITMAP (AND of two bitmaps per window of 16384 values).
  * SI_TECH_AUTO: per bucket from `table` (host uint8[SI_BATCH_TABLE_SIZE] of
  * SI_BATCH_* codes; a code >= SI_BATCH_CODES counts as merge), or, with
- * table == NULL, search when l >= 16 s and hash otherwise.
+ * table == NULL, by a default rule: window bitmaps of 32768 values when the
+ * larger set is dense (d <= 1) and l < 16 s (but merge for s < 256 with l < 4 s,
+ * and search for s < 512 with l >= 4 s); else search when l >= 4 s (dense: 16 s)
+ * and merge when not.
  *   bucket = (d << 8) | (min(15, log2 s) << 4) | min(15, log2(l / s)),
  * s <= l the two sizes, d the larger set's density class: its mean gap
  * (last - first) / (l - 1) below 4, 32, 256 or larger (d = 0..3; 3 when

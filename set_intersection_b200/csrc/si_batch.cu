@@ -6,23 +6,25 @@
 // the 3-kernel SISI path).  Here a list of (a, b) pairs of a CSR collection is
 // counted by two persistent kernels over one work queue:
 //
-//  * Work queue: the pairs are ordered by estimated cost, largest first (a
-//    device radix sort of keys that carry each pair's technique), merge and
-//    search pairs first, hash and bitmap pairs after them; every warp takes
+//  * Work queue: the pairs are ordered by class of estimated cost, largest
+//    first (a counting sort of 12-bit keys: cost class, technique, kernel), merge
+//    and search pairs first, hash and bitmap pairs after them; every warp takes
 //    the next pair of its kernel's part from an atomic ticket, so the long
-//    pairs start first and the short ones fill the tail.  The merge / search
+//    pairs start first and the short ones fill the tail.  Pairs that are a
+//    good part of a warp's share of all the work are first taken by whole CTAs,
+//    each warp an eighth of the larger set's range.  The merge / search
 //    kernel runs 32 warps per SM (search is latency-bound), the hash / bitmap
-//    kernel 24 with 8 KiB of shared memory each.
+//    kernel 24 with 8 KiB of shared memory each; the second starts as the first
+//    one's CTAs end.
 //  * Six technique codes per pair, picked per bucket of (density class of the
 //    larger set, log2 of the smaller size, log2 of the size ratio) from a
 //    1024-entry table:
-//      MERGE (ip): the warp streams both sets through a shared-memory ring of
-//        two 256-element blocks per set; every round finalises the elements up
-//        to the smaller of the two window maxima and merges them along the
-//        merge path (each lane an equal share of the merged positions after a
-//        split search, as the reference's intersectPath splits a partition,
-//        src/ip.cu:207-245), then slides; the next block of each set is
-//        prefetched into registers a round ahead.
+//      MERGE (ip): the warp takes a window of 256 elements of each set into
+//        shared memory; every round finalises the elements up to the smaller of
+//        the two window maxima and merges them along the merge path (each lane
+//        an equal share of the merged positions after a split search, as the
+//        reference's intersectPath splits a partition, src/ip.cu:207-245), while
+//        the next windows are loaded into registers.
 //      SEARCH (obs): the warp takes the smaller set 256 elements at a time,
 //        bounds the window of the larger set that can hold them, caches 256
 //        samples of a long window in shared memory, and every lane runs 8
@@ -42,7 +44,6 @@
 //    sample of every populated bucket, or the default rule.
 #include <algorithm>
 #include <cstring>
-#include <cub/device/device_radix_sort.cuh>
 #include <mutex>
 #include <vector>
 
@@ -65,35 +66,43 @@ constexpr uint32_t kWarpSmem = 8192;     // stream kernel: shared bytes per warp
 constexpr uint32_t kBSmem = kBWarps * kWarpSmem + 4096;  // + the skew to a 4 KiB boundary
 constexpr uint32_t kW = 256;             // window (block) per set per round
 constexpr int kVT = kW / 32;             // elements per lane per block
-// header: [0..16) error words, [16] u32 ticket of the merge / search kernel,
-// [20] u32 ticket of the stream kernel, [24] u32 pairs in the merge / search
-// part of the queue (its first part)
+// header: [0..16) error words, then per kernel (merge / search, stream) u32
+// tickets of the warps [16, 24) and of the CTAs [24, 32), u32 pairs in the
+// queue's first part (merge / search) [32], u64 cost of each part [40, 56)
 constexpr size_t kBatchHeader = 256;
+constexpr size_t kWarpTicket = 16, kCtaTicket = 24, kNFirst = 32, kPartCost = 40;
 // technique codes: the table's bytes (si.h SI_BATCH_*)
 constexpr uint8_t kMerge = 0, kSearch = 1, kHash1024 = 2, kHash512 = 3, kBitmap16K = 4, kBitmap32K = 5;
 constexpr uint8_t kTechCodes = 6;
 constexpr uint32_t kTableSize = 1024;    // 4 density classes x 16 size classes x 16 ratio classes
 
+// The queue's bins: part (1 bit), falling cost class (8 bits), technique (3 bits).
+constexpr uint32_t kBins = 4096;
+constexpr int kKeyThreads = 256;
+constexpr uint32_t kKeyPairs = 4;  // pairs per thread of the key and queue kernels
+
 struct BatchLayout {
-    size_t off_keys_in = 0, off_keys = 0, off_cub = 0, cub_bytes = 0, total = 0;
+    size_t off_hist = 0, off_cursor = 0, off_bins = 0, off_queue = 0, total = 0;
 };
 
 BatchLayout batch_layout(uint64_t npairs) {
     BatchLayout L;
     size_t o = kBatchHeader;
-    L.off_keys_in = o;  o = align_up(o + npairs * 8, 256);
-    L.off_keys = o;     o = align_up(o + npairs * 8, 256);
-    size_t sort_bytes = 0;
-    if (cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, static_cast<const uint64_t*>(nullptr),
-                                       static_cast<uint64_t*>(nullptr), static_cast<int>(std::max<uint64_t>(npairs, 1))) !=
-        cudaSuccess)
-        sort_bytes = npairs * 8 + (1u << 20);  // without a device to ask: a bound
-    cudaGetLastError();
-    L.cub_bytes = align_up(sort_bytes, 256);
-    L.off_cub = o;
-    o += L.cub_bytes;
+    L.off_hist = o;    o += kBins * 4;  // the header, the histogram and the cursors start at zero
+    L.off_cursor = o;  o += kBins * 4;
+    L.off_bins = o;    o = align_up(o + npairs * 2, 256);
+    L.off_queue = o;   o = align_up(o + npairs * 8, 256);
     L.total = o;
     return L;
+}
+
+// Class of a cost: its exponent and three more bits (a class spans an eighth of
+// its cost).
+__device__ __forceinline__ uint32_t cost_class(uint64_t cost) {
+    const uint32_t c = static_cast<uint32_t>(min(cost, uint64_t(0xffffffffu)));
+    if (c < 8) return c;
+    const uint32_t e = 31 - __clz(c);
+    return (e - 2) * 8 + ((c >> (e - 3)) & 7u);
 }
 
 __host__ __device__ inline uint32_t log2_floor(uint64_t x) {  // x >= 1
@@ -154,39 +163,104 @@ __device__ __forceinline__ uint32_t device_bucket(const uint32_t* el, const Pair
 
 __host__ __device__ constexpr bool is_stream_tech(uint8_t t) { return t >= kHash1024 && t < kTechCodes; }
 
-// Queue key per pair: stream class (1 bit: hash or bitmap), descending cost
-// (28 bits, saturated), technique (3 bits), pair index (32 bits).  Sorted
-// ascending, the merge / search pairs come first, each part largest first;
-// n_first counts the first part.  A stream technique falls back to merge for
-// a pair whose larger set has 2^32 - 1024 elements or more (stream positions
-// are 32-bit).
-__global__ void batch_keys_kernel(const uint32_t* __restrict__ el, const uint64_t* __restrict__ off,
-                                  const uint32_t* __restrict__ pairs, uint64_t npairs, uint32_t k, TechTable table,
-                                  int forced, uint64_t* __restrict__ keys, uint32_t* err, uint32_t* n_first) {
-    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x;
-    const uint64_t end = (npairs + 31) / 32 * 32;  // whole warps, for the aggregated count
-    for (uint64_t p = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; p < end; p += stride) {
-        bool first_part = false;
-        if (p < npairs) {
-            const uint32_t a = pairs[2 * p], b = pairs[2 * p + 1];
-            uint64_t cost = 0;
-            uint8_t t = kMerge;
-            if (a >= k || b >= k) {
-                record_error(err, SI_ERR_INVALID_INPUT, 50, static_cast<uint32_t>(p));
-            } else {
-                const PairSets ps = pair_sets(off, a, b);
-                t = forced >= 0 ? static_cast<uint8_t>(forced) : table.t[device_bucket(el, ps)];
-                if (t >= kTechCodes || (is_stream_tech(t) && max(ps.na, ps.nb) >= kMaxStream)) t = kMerge;
-                cost = t == kSearch ? search_cost(min(ps.na, ps.nb), max(ps.na, ps.nb)) : ps.na + ps.nb;
-            }
-            const uint64_t c = min(cost, uint64_t(0x0fffffffu));
-            const uint64_t cls = is_stream_tech(t) ? 1u : 0u;
-            keys[p] = (((cls << 28 | (0x0fffffffu - c)) << 3 | t) << 32) | static_cast<uint32_t>(p);
-            first_part = cls == 0;
+// Each pair's bin, the bins' histogram and the parts' total cost.  A stream
+// technique falls back to merge for a pair whose larger set has 2^32 - 1024
+// elements or more (stream positions are 32-bit).
+__global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
+    const uint32_t* __restrict__ el, const uint64_t* __restrict__ off, const uint32_t* __restrict__ pairs,
+    uint64_t npairs, uint32_t k, const __grid_constant__ TechTable table, int forced, uint16_t* __restrict__ bins,
+    uint32_t* __restrict__ hist, unsigned char* header) {
+    __shared__ uint32_t s_hist[kBins];
+    __shared__ unsigned long long s_cost[2];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads) s_hist[i] = 0;
+    if (threadIdx.x < 2) s_cost[threadIdx.x] = 0;
+    __syncthreads();
+    const uint64_t p0 = uint64_t(blockIdx.x) * kKeyThreads * kKeyPairs + threadIdx.x;
+    uint64_t part_cost[2] = {0, 0};
+#pragma unroll
+    for (uint32_t u = 0; u < kKeyPairs; ++u) {
+        const uint64_t p = p0 + u * kKeyThreads;
+        if (p >= npairs) continue;
+        const uint32_t a = pairs[2 * p], b = pairs[2 * p + 1];
+        uint64_t cost = 0;
+        uint8_t t = kMerge;
+        if (a >= k || b >= k) {
+            record_error(reinterpret_cast<uint32_t*>(header), SI_ERR_INVALID_INPUT, 50, static_cast<uint32_t>(p));
+        } else {
+            const PairSets ps = pair_sets(off, a, b);
+            t = forced >= 0 ? static_cast<uint8_t>(forced) : table.t[device_bucket(el, ps)];
+            if (t >= kTechCodes || (is_stream_tech(t) && max(ps.na, ps.nb) >= kMaxStream)) t = kMerge;
+            cost = t == kSearch ? search_cost(min(ps.na, ps.nb), max(ps.na, ps.nb)) : ps.na + ps.nb;
         }
-        const uint32_t m = __ballot_sync(kFullMask, first_part);
-        if ((threadIdx.x & 31) == 0 && m) atomicAdd(n_first, static_cast<uint32_t>(__popc(m)));
+        const uint32_t part = is_stream_tech(t) ? 1u : 0u;
+        const uint32_t bin = part << 11 | (255u - cost_class(cost)) << 3 | t;
+        bins[p] = static_cast<uint16_t>(bin);
+        atomicAdd(&s_hist[bin], 1u);
+        part_cost[part] += cost;
     }
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+        const uint64_t c = warp_sum_u64(part_cost[part]);
+        if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_cost[part], static_cast<unsigned long long>(c));
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads)
+        if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
+    if (threadIdx.x < 2 && s_cost[threadIdx.x])
+        atomicAdd(reinterpret_cast<unsigned long long*>(header + kPartCost) + threadIdx.x, s_cost[threadIdx.x]);
+}
+
+// The queue: every pair (its bin in bits 32.., its index below) at its bin's
+// offset.  A CTA scans the histogram itself and reserves room in each bin once;
+// the order within a bin does not matter.
+__global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t* __restrict__ bins, uint64_t npairs,
+                                                                  const uint32_t* __restrict__ hist,
+                                                                  uint32_t* __restrict__ cursor,
+                                                                  uint64_t* __restrict__ queue,
+                                                                  unsigned char* header) {
+    __shared__ uint32_t s_off[kBins];    // the bin's offset, then where this CTA's next pair of it goes
+    __shared__ uint32_t s_count[kBins];  // this CTA's pairs of the bin
+    __shared__ uint32_t s_warp[kKeyThreads / 32];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads) s_count[i] = 0;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the bins and their histogram
+    constexpr uint32_t kPer = kBins / kKeyThreads;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t v[kPer], sum = 0;
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) {
+        v[q] = __ldcg(hist + threadIdx.x * kPer + q);
+        sum += v[q];
+    }
+    const uint32_t incl = warp_inclusive_scan(sum);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t o = incl - sum;
+    for (uint32_t w = 0; w < warp; ++w) o += s_warp[w];
+#pragma unroll
+    for (uint32_t q = 0; q < kPer; ++q) {
+        s_off[threadIdx.x * kPer + q] = o;
+        o += v[q];
+    }
+    uint32_t bin[kKeyPairs];
+    const uint64_t p0 = uint64_t(blockIdx.x) * kKeyThreads * kKeyPairs + threadIdx.x;
+#pragma unroll
+    for (uint32_t u = 0; u < kKeyPairs; ++u) {
+        const uint64_t p = p0 + u * kKeyThreads;
+        bin[u] = p < npairs ? bins[p] : kBins;
+        if (bin[u] < kBins) atomicAdd(&s_count[bin[u]], 1u);
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint32_t*>(header + kNFirst) = s_off[kBins / 2];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads)
+        if (s_count[i]) s_off[i] += atomicAdd(cursor + i, s_count[i]);
+    __syncthreads();
+#pragma unroll
+    for (uint32_t u = 0; u < kKeyPairs; ++u)
+        if (bin[u] < kBins)
+            queue[atomicAdd(&s_off[bin[u]], 1u)] = uint64_t(bin[u]) << 32 | (p0 + u * kKeyThreads);
 }
 
 // ------------------------------------------------------ per-warp techniques --
@@ -226,7 +300,7 @@ __device__ __forceinline__ uint32_t window_count_le(const uint32_t* w, uint32_t 
 //
 // A merge step is eight instructions, a round of some 500 elements about 330:
 // 0.65 warp instructions per element, where rings of blocks with masked indexes
-// and clamped ends took 2.7 (all pairs of 20000 sets merged: 16.4 ms against 21.7).
+// and clamped ends took 2.7 (all pairs of 20000 sets merged: 15.1 ms against 21.7).
 constexpr uint32_t kMergeWords = 2 * (kW + 32);  // per set: the window, then end marks that a lane's steps may run into
 __device__ uint32_t merge_pair(const uint32_t* A, uint64_t na, const uint32_t* B, uint64_t nb, uint32_t* win,
                                uint32_t lane) {
@@ -335,14 +409,32 @@ __device__ uint32_t search_pair(const uint32_t* S, uint64_t ns, const uint32_t* 
             }
             __syncwarp();
         }
-        uint32_t v[kVT];
-        uint64_t pos[kVT], len[kVT];
+        if (W >= (uint64_t(1) << 32)) {  // a window past 32-bit offsets: one plain search after another
+            for (uint32_t t = 0; t < kVT; ++t) {
+                const uint64_t i = base + lane + 32u * t;
+                if (i > last_i) break;
+                const uint32_t v = __ldg(S + i);
+                uint64_t p = lo, len = W;
+                while (len > 1) {
+                    const uint64_t half = len >> 1;
+                    const bool c = __ldg(L + p + half) <= v;
+                    p = c ? p + half : p;
+                    len = c ? len - half : half;
+                }
+                hits += __ldg(L + p) == v ? 1u : 0u;
+            }
+            __syncwarp();  // the samples are not read, and written again by the next block
+            continue;
+        }
+        const uint32_t* Lw = L + lo;
+        const uint32_t W32 = static_cast<uint32_t>(W);
+        uint32_t v[kVT], o32[kVT], n32[kVT];
 #pragma unroll
         for (int t = 0; t < kVT; ++t) {
             const uint64_t i = base + lane + 32u * t;
             v[t] = i <= last_i ? __ldg(S + i) : 0u;
-            pos[t] = lo;
-            len[t] = i <= last_i ? W : 0;
+            o32[t] = 0;
+            n32[t] = i <= last_i ? W32 : 0u;
         }
         if (sampled) {
 #pragma unroll
@@ -353,72 +445,45 @@ __device__ uint32_t search_pair(const uint32_t* S, uint64_t ns, const uint32_t* 
                 for (uint32_t step = kSample / 2; step > 0; step >>= 1)
                     c = samp[c + step - 1] <= v[t] ? c + step : c;
                 c = (c == kSample - 1 && samp[kSample - 1] <= v[t]) ? kSample : c;
-                const uint64_t p0 = lo + W * (c ? c - 1 : 0) / kSample;
-                const uint64_t p1 = c == kSample ? hi : lo + W * c / kSample;
-                pos[t] = p0;
-                len[t] = c == 0 ? 0 : (len[t] ? p1 - p0 : 0);  // c == 0: v is below L[lo]
+                const uint32_t p0 = static_cast<uint32_t>(uint64_t(W32) * (c ? c - 1 : 0) / kSample);
+                const uint32_t p1 = static_cast<uint32_t>(uint64_t(W32) * c / kSample);  // W32 for c == kSample
+                o32[t] = p0;
+                n32[t] = c == 0 || n32[t] == 0 ? 0u : p1 - p0;  // c == 0: v is below L[lo]
             }
             __syncwarp();  // the samples are read before the next block writes them
         }
         // interleaved searches for the last element <= v: kVT independent load
-        // chains per lane, in 32-bit offsets from lo when the window allows
-        if (W < (uint64_t(1) << 32)) {
-            const uint32_t* Lw = L + lo;
-            uint32_t o32[kVT], n32[kVT];
+        // chains per lane; 4-ary steps (three independent loads, a quarter of the
+        // gap left) while the gap allows, then binary: half the dependent load
+        // rounds of a binary search
+        bool more = true;
+        while (more) {
+            more = false;
 #pragma unroll
             for (int t = 0; t < kVT; ++t) {
-                o32[t] = static_cast<uint32_t>(pos[t] - lo);
-                n32[t] = static_cast<uint32_t>(len[t]);
-            }
-            // 4-ary steps (three independent loads, a quarter of the gap
-            // left) while the gap allows, then binary: half the dependent
-            // load rounds of a binary search
-            bool more = true;
-            while (more) {
-                more = false;
-#pragma unroll
-                for (int t = 0; t < kVT; ++t) {
-                    const uint32_t n = n32[t];
-                    if (n >= 4) {
-                        const uint32_t q1 = n >> 2, q2 = n >> 1, q3 = q1 + q2;
-                        const uint32_t o = o32[t];
-                        const bool c1 = __ldg(Lw + o + q1) <= v[t];
-                        const bool c2 = __ldg(Lw + o + q2) <= v[t];
-                        const bool c3 = __ldg(Lw + o + q3) <= v[t];
-                        const uint32_t lo_q = c3 ? q3 : c2 ? q2 : c1 ? q1 : 0u;
-                        const uint32_t hi_q = c3 ? n : c2 ? q3 : c1 ? q2 : q1;
-                        o32[t] = o + lo_q;
-                        n32[t] = hi_q - lo_q;
-                        more |= n32[t] > 1;
-                    } else if (n > 1) {
-                        const uint32_t half = n >> 1;
-                        const bool c = __ldg(Lw + o32[t] + half) <= v[t];
-                        o32[t] = c ? o32[t] + half : o32[t];
-                        n32[t] = c ? n - half : half;
-                        more |= n32[t] > 1;
-                    }
+                const uint32_t n = n32[t];
+                if (n >= 4) {
+                    const uint32_t q1 = n >> 2, q2 = n >> 1, q3 = q1 + q2;
+                    const uint32_t o = o32[t];
+                    const bool c1 = __ldg(Lw + o + q1) <= v[t];
+                    const bool c2 = __ldg(Lw + o + q2) <= v[t];
+                    const bool c3 = __ldg(Lw + o + q3) <= v[t];
+                    const uint32_t lo_q = c3 ? q3 : c2 ? q2 : c1 ? q1 : 0u;
+                    const uint32_t hi_q = c3 ? n : c2 ? q3 : c1 ? q2 : q1;
+                    o32[t] = o + lo_q;
+                    n32[t] = hi_q - lo_q;
+                    more |= n32[t] > 1;
+                } else if (n > 1) {
+                    const uint32_t half = n >> 1;
+                    const bool c = __ldg(Lw + o32[t] + half) <= v[t];
+                    o32[t] = c ? o32[t] + half : o32[t];
+                    n32[t] = c ? n - half : half;
+                    more |= n32[t] > 1;
                 }
             }
-#pragma unroll
-            for (int t = 0; t < kVT; ++t) hits += (n32[t] == 1 && __ldg(Lw + o32[t]) == v[t]) ? 1u : 0u;
-        } else {
-            bool more = true;
-            while (more) {
-                more = false;
-#pragma unroll
-                for (int t = 0; t < kVT; ++t) {
-                    if (len[t] > 1) {
-                        const uint64_t half = len[t] >> 1;
-                        const bool c = __ldg(L + pos[t] + half) <= v[t];
-                        pos[t] = c ? pos[t] + half : pos[t];
-                        len[t] = c ? len[t] - half : half;
-                        more |= len[t] > 1;
-                    }
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < kVT; ++t) hits += (len[t] == 1 && __ldg(L + pos[t]) == v[t]) ? 1u : 0u;
         }
+#pragma unroll
+        for (int t = 0; t < kVT; ++t) hits += (n32[t] == 1 && __ldg(Lw + o32[t]) == v[t]) ? 1u : 0u;
     }
     return __reduce_add_sync(kFullMask, hits);
 }
@@ -529,23 +594,56 @@ struct BatchParams {
     const uint64_t* off;
     const uint32_t* pairs;
     uint32_t k;
-    const uint64_t* keys;    // sorted queue keys: technique in bits 32..34, pair index in the low 32
+    const uint64_t* queue;   // bin in bits 32.., pair index below
     const uint32_t* subset;  // when non-null: the queue is these pair indices, in order, all by `forced`
     uint64_t nqueue;         // queue length (all pairs, or the subset)
-    const uint32_t* n_first; // pairs in the queue's first part (merge / search), from the key kernel
     uint32_t* counts;
-    uint32_t* ticket;        // this kernel's ticket
+    unsigned char* header;
     int forced;
+    bool first;              // the first kernel after the queue's
 };
 
+// |S ∩ L| by one warp.
+template <bool kStream>
+__device__ __forceinline__ uint32_t count_pair(uint8_t tech, const uint32_t* S, uint64_t ns, const uint32_t* L,
+                                               uint64_t nl, uint32_t* region, uint32_t lane) {
+    if constexpr (kStream) {
+        if (nl >= kMaxStream) tech = kMerge;  // only reachable with a tuner subset
+        switch (tech) {
+            case kMerge: return merge_pair(S, ns, L, nl, region, lane);
+            case kHash512: return hash_pair<2>(S, ns, L, nl, region, lane);
+            case kBitmap16K: return bitmap_pair<512>(L, nl, S, ns, region, lane);
+            case kBitmap32K: return bitmap_pair<1024>(L, nl, S, ns, region, lane);
+            default: return hash_pair<4>(S, ns, L, nl, region, lane);
+        }
+    } else {
+        return tech == kSearch ? search_pair(S, ns, L, nl, region, lane) : merge_pair(S, ns, L, nl, region, lane);
+    }
+}
+
+// Pairs of more than a kCoopShare-th of a warp's share of the part's cost are
+// taken by whole CTAs when they are worth the searches that divide them.  Their
+// warps would otherwise hold up the end.  Merge and search, shares of 1/2, 2 and
+// 8 warps' work: 20000 pairs of 5000 sets of up to 2^18 elements 1.88, 1.25 and
+// 1.04 ms by the default rule (12.1 without), 2000 pairs 0.29, 0.30 and 0.28 ms
+// (10.1); 200000 pairs by search 16.3, 15.4 and 15.2 ms (15.3).  Hash and bitmap:
+// 11.5, 6.2 and 5.1 ms, and 8.3, 8.2 and 9.2 ms for the 20000.
+constexpr uint64_t kCoopCost = 8192;
+template <bool kStream>
+constexpr uint64_t kCoopShareOf = kStream ? 2 : 8;
+
 // One kernel per part of the queue.  kStream = false: merge and search pairs
-// (the first part), rings in static shared memory; kStream = true: hash and
+// (the first part), windows in static shared memory; kStream = true: hash and
 // bitmap pairs (the rest), 8 KiB of dynamic shared memory per warp.  With a
 // subset (the tuner) the kernel of the forced technique takes it all.
 template <bool kStream>
 __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearchCtasPerSm)
     batch_kernel(BatchParams p) {
     extern __shared__ __align__(16) uint32_t smem[];
+    __shared__ uint32_t s_q, s_hits[kBWarps];
+    // the part of the queue left, in shared memory: the counting below wants the registers
+    __shared__ uint64_t s_q0, s_q1;
+    __shared__ uint32_t s_class;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // stream kernel: the warp's 8 KiB, 4 KiB aligned (the bitmaps' word
     // addresses are one LOP3); merge / search kernel: the warp's two windows
@@ -557,62 +655,124 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
         __shared__ __align__(16) uint32_t windows[kBWarps][kMergeWords];
         region = windows[warp];
     }
-    uint64_t q0 = 0, q1 = p.nqueue;
-    if (!p.subset) {
-        const uint32_t nf = *p.n_first;
-        q0 = kStream ? nf : 0;
-        q1 = kStream ? p.nqueue : nf;
+    // the queue is ready when its kernel's first successor runs; the second one
+    // may then start while the first one's last CTAs run
+    if (p.first) asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (threadIdx.x == 0) {
+        uint64_t q0 = 0, q1 = p.nqueue;
+        uint32_t cls = 0;
+        if (!p.subset) {
+            const uint32_t nf = *reinterpret_cast<const volatile uint32_t*>(p.header + kNFirst);
+            q0 = kStream ? nf : 0;
+            q1 = kStream ? p.nqueue : nf;
+            const uint64_t cost = reinterpret_cast<const volatile uint64_t*>(p.header + kPartCost)[kStream];
+            cls = cost_class(max(kCoopCost, cost / kCoopShareOf<kStream> / (uint64_t(gridDim.x) * kBWarps)));
+        }
+        s_q0 = q0;
+        s_q1 = q1;
+        s_class = cls;
     }
+    __syncthreads();
+    auto is_small = [&](uint64_t q) { return 255u - (static_cast<uint32_t>(p.queue[q] >> 35) & 255u) < s_class; };
+    bool coop = !p.subset && s_q0 < s_q1 && !is_small(s_q0);  // CTA-uniform; the queue falls in cost
     for (;;) {
-        uint32_t t = 0;
-        if (lane == 0) t = atomicAdd(p.ticket, 1u);
-        const uint64_t q = q0 + __shfl_sync(kFullMask, t, 0);
-        if (q >= q1) break;
+        uint64_t q;
+        if (coop) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_q = atomicAdd(reinterpret_cast<uint32_t*>(p.header + kCtaTicket) + kStream, 1u);
+            __syncthreads();
+            q = s_q0 + s_q;
+            if (q >= s_q1 || is_small(q)) {  // the rest goes to the warps
+                coop = false;
+                const uint64_t q0 = warp_first_true(s_q0, s_q1, is_small);
+                __syncthreads();
+                if (threadIdx.x == 0) s_q0 = q0;
+                __syncthreads();
+                continue;
+            }
+        } else {
+            uint32_t t = 0;
+            if (lane == 0) t = atomicAdd(reinterpret_cast<uint32_t*>(p.header + kWarpTicket) + kStream, 1u);
+            q = s_q0 + __shfl_sync(kFullMask, t, 0);
+            if (q >= s_q1) break;
+        }
         uint32_t pi;
         uint8_t tech;
         if (p.subset) {
             pi = p.subset[q];
             tech = static_cast<uint8_t>(p.forced);
         } else {
-            const uint64_t key = p.keys[q];
+            const uint64_t key = p.queue[q];
             pi = static_cast<uint32_t>(key);
             tech = static_cast<uint8_t>((key >> 32) & 7u);
         }
         const uint32_t a = p.pairs[2 * uint64_t(pi)], b = p.pairs[2 * uint64_t(pi) + 1];
-        if (a >= p.k || b >= p.k) continue;  // recorded by the key kernel
+        if (a >= p.k || b >= p.k) continue;  // recorded by the key kernel (cost 0: never taken by a CTA)
         const PairSets ps = pair_sets(p.off, a, b);
         const bool as = ps.na <= ps.nb;  // A is the smaller set
         const uint32_t* S = p.el + (as ? ps.a0 : ps.b0);
         const uint32_t* L = p.el + (as ? ps.b0 : ps.a0);
-        const uint64_t ns = as ? ps.na : ps.nb, nl = as ? ps.nb : ps.na;
-        uint32_t c;
-        if constexpr (kStream) {
-            if (nl >= kMaxStream) tech = kMerge;  // only reachable with a tuner subset
-            switch (tech) {
-                case kMerge:
-                    c = merge_pair(p.el + ps.a0, ps.na, p.el + ps.b0, ps.nb, region, lane);
-                    break;
-                case kHash512: c = hash_pair<2>(S, ns, L, nl, region, lane); break;
-                case kBitmap16K: c = bitmap_pair<512>(L, nl, S, ns, region, lane); break;
-                case kBitmap32K: c = bitmap_pair<1024>(L, nl, S, ns, region, lane); break;
-                default: c = hash_pair<4>(S, ns, L, nl, region, lane); break;
+        uint64_t ns = as ? ps.na : ps.nb, nl = as ? ps.nb : ps.na;
+        if (coop) {  // an eighth of L, and the elements of S from its first to the next one's
+            const uint64_t l0 = nl * warp / kBWarps, l1 = nl * (warp + 1) / kBWarps;
+            uint64_t s0 = 0, s1 = ns;
+            if (warp > 0) {
+                const uint32_t v = __ldg(L + l0);
+                s0 = warp_first_true(0, ns, [&](uint64_t i) { return __ldg(S + i) >= v; });
+            }
+            if (warp + 1 < kBWarps) {
+                const uint32_t v = __ldg(L + l1);
+                s1 = warp_first_true(s0, ns, [&](uint64_t i) { return __ldg(S + i) >= v; });
+            }
+            S += s0;
+            L += l0;
+            ns = s1 - s0;
+            nl = l1 - l0;
+            if (ns > nl) {
+                const uint32_t* x = S;
+                S = L;
+                L = x;
+                const uint64_t n = ns;
+                ns = nl;
+                nl = n;
+            }
+        }
+        const uint32_t c = count_pair<kStream>(tech, S, ns, L, nl, region, lane);
+        if (coop) {
+            if (lane == 0) s_hits[warp] = c;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                uint32_t sum = 0;
+#pragma unroll
+                for (int w = 0; w < kBWarps; ++w) sum += s_hits[w];
+                p.counts[pi] = sum;
             }
         } else {
-            if (tech == kSearch)
-                c = search_pair(S, ns, L, nl, region, lane);
-            else
-                c = merge_pair(p.el + ps.a0, ps.na, p.el + ps.b0, ps.nb, region, lane);
+            if (lane == 0) p.counts[pi] = c;
+            __syncwarp();
         }
-        if (lane == 0) p.counts[pi] = c;
-        __syncwarp();
     }
+    // this kernel does not end before the one it started beside
+    if (!p.first) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-// Default rule: search when the larger set is at least 16 times the smaller,
-// else hash.
+// Default rule, from every technique's time on pairs of each bucket over pools
+// of 2^14 .. 2^26 values.  Dense larger sets (mean gap below 32): window bitmaps
+// of 32768 values, but search when the smaller set is short or 16 times smaller
+// (gap 8..32, 1024 against 8192 elements: bitmap 18 ns a pair, search 20, merge
+// 25, hash 81; 512 against 32768: 37, 23, 73, 186).  Sparse ones: search from a
+// ratio of 4 on, else merge (gap 64..256, 8192 against 12000: merge 71 ns, search
+// 152, bitmap 116, hash 285).  Hash is never the fastest.
 TechTable default_table() {
     TechTable T;
-    for (uint32_t b = 0; b < kTableSize; ++b) T.t[b] = (b & 15u) >= 4 ? kSearch : kHash1024;
+    for (uint32_t b = 0; b < kTableSize; ++b) {
+        const uint32_t d = b >> 8, ls = (b >> 4) & 15u, lr = b & 15u;
+        if (d <= 1)
+            T.t[b] = lr >= 4 || (ls < 9 && lr >= 2) ? kSearch : ls < 8 ? kMerge : kBitmap32K;
+        else
+            T.t[b] = lr >= 2 ? kSearch : kMerge;
+    }
     return T;
 }
 
@@ -648,52 +808,55 @@ si_status batch_launch(const uint32_t* d_elements, const uint64_t* d_offsets, ui
     const BatchLayout L = batch_layout(npairs);
     if (ws_bytes < L.total) return SI_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* w = static_cast<unsigned char*>(ws);
-    uint32_t* err = reinterpret_cast<uint32_t*>(w);
-    SI_CUDA_TRY(cudaMemsetAsync(w, 0, kBatchHeader, stream));
+    SI_CUDA_TRY(cudaMemsetAsync(w, 0, d_subset || npairs == 0 ? kBatchHeader : L.off_bins, stream));
     if (npairs == 0) return SI_OK;
-    uint64_t* keys_in = reinterpret_cast<uint64_t*>(w + L.off_keys_in);
-    uint64_t* keys = reinterpret_cast<uint64_t*>(w + L.off_keys);
-    uint32_t* n_first = reinterpret_cast<uint32_t*>(w + 24);
+    uint64_t* queue = reinterpret_cast<uint64_t*>(w + L.off_queue);
     BatchParams prm;
     prm.el = d_elements;
     prm.off = d_offsets;
     prm.pairs = d_pairs;
     prm.k = k;
-    prm.keys = keys;
+    prm.queue = queue;
     prm.subset = d_subset;
     prm.nqueue = d_subset ? nsubset : npairs;
-    prm.n_first = n_first;
     prm.counts = d_counts;
+    prm.header = w;
     prm.forced = forced;
     if (!d_subset) {
         PhaseTimer timer("batch_plan", stream);
-        const unsigned g = static_cast<unsigned>(std::min<uint64_t>((npairs + 255) / 256, uint64_t(sm_count()) * 8));
-        batch_keys_kernel<<<g, 256, 0, stream>>>(d_elements, d_offsets, d_pairs, npairs, k, table, forced, keys_in,
-                                                 err, n_first);
+        uint32_t* hist = reinterpret_cast<uint32_t*>(w + L.off_hist);
+        uint32_t* cursor = reinterpret_cast<uint32_t*>(w + L.off_cursor);
+        uint16_t* bins = reinterpret_cast<uint16_t*>(w + L.off_bins);
+        const unsigned g = static_cast<unsigned>((npairs + kKeyThreads * kKeyPairs - 1) / (kKeyThreads * kKeyPairs));
+        batch_keys_kernel<<<g, kKeyThreads, 0, stream>>>(d_elements, d_offsets, d_pairs, npairs, k, table, forced,
+                                                         bins, hist, w);
         SI_LAUNCH_CHECK("batch_keys_kernel");
-        size_t tmp = L.cub_bytes;
-        SI_CUDA_TRY(cub::DeviceRadixSort::SortKeys(w + L.off_cub, tmp, keys_in, keys, static_cast<int>(npairs), 0, 64,
-                                                   stream));
+        const si_status st = launch_dependent(batch_queue_kernel, dim3(g), dim3(kKeyThreads), 0, stream,
+                                              static_cast<const uint16_t*>(bins), npairs,
+                                              static_cast<const uint32_t*>(hist), cursor, queue, w);
+        if (st != SI_OK) return st;
     }
     const BatchOccupancy occ = batch_occupancy();
     const int search_per_sm = occ.search, stream_per_sm = occ.stream;
     if (search_per_sm == 0 || stream_per_sm == 0) return cuda_fail(cudaGetLastError(), "batch_kernel attributes");
     // the subset of the tuner runs in its technique's kernel; the whole queue
-    // in both, one part each (no stream part when every pair merges or searches)
+    // in both, one part each (no stream part when every pair merges or searches,
+    // nor the other when every pair is forced to the stream kernel: those too
+    // large for it, which merge there, are in the first part)
     const bool forced_stream = forced >= 0 && is_stream_tech(static_cast<uint8_t>(forced));
     const bool run_search = d_subset ? !forced_stream : true;
     const bool run_stream = d_subset ? forced_stream : forced < 0 || forced_stream;
     PhaseTimer timer("batch_count", stream);
+    prm.first = true;
     if (run_search) {
-        prm.ticket = reinterpret_cast<uint32_t*>(w + 16);
-        batch_kernel<false><<<static_cast<unsigned>(sm_count() * search_per_sm), kBThreads, 0, stream>>>(prm);
-        SI_LAUNCH_CHECK("batch_kernel<merge/search>");
+        const si_status st = launch_dependent(batch_kernel<false>, dim3(static_cast<unsigned>(sm_count() * search_per_sm)),
+                                              dim3(kBThreads), 0, stream, prm);
+        if (st != SI_OK) return st;
+        prm.first = false;
     }
-    if (run_stream) {
-        prm.ticket = reinterpret_cast<uint32_t*>(w + 20);
-        batch_kernel<true><<<static_cast<unsigned>(sm_count() * stream_per_sm), kBThreads, kBSmem, stream>>>(prm);
-        SI_LAUNCH_CHECK("batch_kernel<hash/bitmap>");
-    }
+    if (run_stream)
+        return launch_dependent(batch_kernel<true>, dim3(static_cast<unsigned>(sm_count() * stream_per_sm)),
+                                dim3(kBThreads), kBSmem, stream, prm);
     return SI_OK;
 }
 
@@ -734,7 +897,7 @@ si_status batch_tune(const uint32_t* d_elements, const uint64_t* d_offsets, uint
     if (npairs == 0) return SI_OK;
     // bucket of every pair, on the device, read back
     unsigned char* w = static_cast<unsigned char*>(ws);
-    uint16_t* d_bucket = reinterpret_cast<uint16_t*>(w + L.off_keys_in);  // scratch: 2 npairs bytes
+    uint16_t* d_bucket = reinterpret_cast<uint16_t*>(w + L.off_bins);
     const unsigned g = static_cast<unsigned>(std::min<uint64_t>((npairs + 255) / 256, uint64_t(sm_count()) * 8));
     bucket_kernel<<<g, 256, 0, stream>>>(d_elements, d_offsets, d_pairs, npairs, k, d_bucket);
     SI_LAUNCH_CHECK("bucket_kernel");
@@ -744,8 +907,8 @@ si_status batch_tune(const uint32_t* d_elements, const uint64_t* d_offsets, uint
     std::vector<std::vector<uint32_t>> members(kTableSize);
     for (uint64_t p = 0; p < npairs; ++p)
         if (members[bucket[p]].size() < sample) members[bucket[p]].push_back(static_cast<uint32_t>(p));
-    // sample lists on the device, in the queue keys' room
-    uint32_t* d_subset = reinterpret_cast<uint32_t*>(w + L.off_keys);  // npairs * 8 bytes of room
+    // sample lists on the device, in the queue's room
+    uint32_t* d_subset = reinterpret_cast<uint32_t*>(w + L.off_queue);  // npairs * 8 bytes of room
     cudaEvent_t e0, e1;
     SI_CUDA_TRY(cudaEventCreate(&e0));
     SI_CUDA_TRY(cudaEventCreate(&e1));
