@@ -7,7 +7,8 @@
 // counted by two persistent kernels over one work queue:
 //
 //  * Work queue: the pairs are ordered by class of estimated cost, largest
-//    first (a counting sort of 12-bit keys: cost class, technique, kernel), merge
+//    first (a counting sort of 12-bit keys: kernel, cost class, a hash of the
+//    larger set, whose pairs then find it in L2), merge
 //    and search pairs first, hash and bitmap pairs after them; every warp takes
 //    the next pair of its kernel's part from an atomic ticket, so the long
 //    pairs start first and the short ones fill the tail.  Pairs that are a
@@ -25,10 +26,12 @@
 //        an equal share of the merged positions after a split search, as the
 //        reference's intersectPath splits a partition, src/ip.cu:207-245), while
 //        the next windows are loaded into registers.
-//      SEARCH (obs): the warp takes the smaller set 256 elements at a time,
-//        bounds the window of the larger set that can hold them, caches 256
-//        samples of a long window in shared memory, and every lane runs 8
-//        interleaved binary searches in the gaps between samples.
+//      SEARCH (obs): sets of similar size stream the larger one through shared
+//        memory, the smaller one's elements searching its windows.  Otherwise
+//        the warp takes the smaller set 256 elements at a time, bounds the
+//        window of the larger set that can hold them, caches 256 samples of a
+//        long window in shared memory, and every lane runs 8 interleaved binary
+//        searches in the gaps between samples.
 //      HASH (hi, windows of 1024 or 512 elements): the smaller set S is cut
 //        into windows of consecutive elements; each window goes into the
 //        warp's 2048-slot open-addressing table (load <= 1/2 or 1/4) and the
@@ -76,8 +79,13 @@ constexpr uint8_t kMerge = 0, kSearch = 1, kHash1024 = 2, kHash512 = 3, kBitmap1
 constexpr uint8_t kTechCodes = 6;
 constexpr uint32_t kTableSize = 1024;    // 4 density classes x 16 size classes x 16 ratio classes
 
-// The queue's bins: part (1 bit), falling cost class (8 bits), technique (3 bits).
+// The queue's bins: part (1 bit), falling cost class (7 bits), a hash of the
+// larger set (4 bits), so that the pairs of a set run close together in time and
+// find it in L2.  A pair's 16-bit key has its technique above the bin.
 constexpr uint32_t kBins = 4096;
+__host__ __device__ constexpr uint32_t key_bin(uint32_t key) { return key & (kBins - 1); }
+__host__ __device__ constexpr uint32_t key_class(uint32_t key) { return 127u - ((key >> 4) & 127u); }
+__host__ __device__ constexpr uint8_t key_tech(uint32_t key) { return static_cast<uint8_t>((key >> 12) & 7u); }
 constexpr int kKeyThreads = 256;
 constexpr uint32_t kKeyPairs = 4;  // pairs per thread of the key and queue kernels
 
@@ -96,13 +104,13 @@ BatchLayout batch_layout(uint64_t npairs) {
     return L;
 }
 
-// Class of a cost: its exponent and three more bits (a class spans an eighth of
+// Class of a cost: its exponent and two more bits (a class spans a quarter of
 // its cost).
 __device__ __forceinline__ uint32_t cost_class(uint64_t cost) {
     const uint32_t c = static_cast<uint32_t>(min(cost, uint64_t(0xffffffffu)));
-    if (c < 8) return c;
+    if (c < 4) return c;
     const uint32_t e = 31 - __clz(c);
-    return (e - 2) * 8 + ((c >> (e - 3)) & 7u);
+    return (e - 1) * 4 + ((c >> (e - 2)) & 3u);
 }
 
 __host__ __device__ inline uint32_t log2_floor(uint64_t x) {  // x >= 1
@@ -136,8 +144,12 @@ struct TechTable {
     uint8_t t[kTableSize];
 };
 
+// Costs are in warp instructions, about: a merge takes one per element; the
+// streamed search two per element of the smaller set and a quarter per element
+// of the larger; the sampled search eight per element.
+constexpr uint64_t kStreamRatio = 32;  // below this ratio a search streams the larger set
 __device__ __forceinline__ uint64_t search_cost(uint64_t s, uint64_t l) {
-    return s * (log2_floor(l + 1) + 4);
+    return l < kStreamRatio * s ? 2 * s + l / 4 : 8 * s;
 }
 
 struct PairSets {
@@ -184,6 +196,7 @@ __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
         if (p >= npairs) continue;
         const uint32_t a = pairs[2 * p], b = pairs[2 * p + 1];
         uint64_t cost = 0;
+        uint32_t larger = 0;
         uint8_t t = kMerge;
         if (a >= k || b >= k) {
             record_error(reinterpret_cast<uint32_t*>(header), SI_ERR_INVALID_INPUT, 50, static_cast<uint32_t>(p));
@@ -192,10 +205,11 @@ __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
             t = forced >= 0 ? static_cast<uint8_t>(forced) : table.t[device_bucket(el, ps)];
             if (t >= kTechCodes || (is_stream_tech(t) && max(ps.na, ps.nb) >= kMaxStream)) t = kMerge;
             cost = t == kSearch ? search_cost(min(ps.na, ps.nb), max(ps.na, ps.nb)) : ps.na + ps.nb;
+            larger = ps.na > ps.nb ? a : b;
         }
         const uint32_t part = is_stream_tech(t) ? 1u : 0u;
-        const uint32_t bin = part << 11 | (255u - cost_class(cost)) << 3 | t;
-        bins[p] = static_cast<uint16_t>(bin);
+        const uint32_t bin = part << 11 | (127u - cost_class(cost)) << 4 | (larger * 0x9e3779b1u) >> 28;
+        bins[p] = static_cast<uint16_t>(bin | uint32_t(t) << 12);
         atomicAdd(&s_hist[bin], 1u);
         part_cost[part] += cost;
     }
@@ -211,7 +225,7 @@ __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
         atomicAdd(reinterpret_cast<unsigned long long*>(header + kPartCost) + threadIdx.x, s_cost[threadIdx.x]);
 }
 
-// The queue: every pair (its bin in bits 32.., its index below) at its bin's
+// The queue: every pair (its key in bits 32.., its index below) at its bin's
 // offset.  A CTA scans the histogram itself and reserves room in each bin once;
 // the order within a bin does not matter.
 __global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t* __restrict__ bins, uint64_t npairs,
@@ -243,13 +257,13 @@ __global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t
         s_off[threadIdx.x * kPer + q] = o;
         o += v[q];
     }
-    uint32_t bin[kKeyPairs];
+    uint32_t key[kKeyPairs];
     const uint64_t p0 = uint64_t(blockIdx.x) * kKeyThreads * kKeyPairs + threadIdx.x;
 #pragma unroll
     for (uint32_t u = 0; u < kKeyPairs; ++u) {
         const uint64_t p = p0 + u * kKeyThreads;
-        bin[u] = p < npairs ? bins[p] : kBins;
-        if (bin[u] < kBins) atomicAdd(&s_count[bin[u]], 1u);
+        key[u] = p < npairs ? bins[p] : ~0u;
+        if (key[u] != ~0u) atomicAdd(&s_count[key_bin(key[u])], 1u);
     }
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint32_t*>(header + kNFirst) = s_off[kBins / 2];
@@ -259,8 +273,8 @@ __global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t
     __syncthreads();
 #pragma unroll
     for (uint32_t u = 0; u < kKeyPairs; ++u)
-        if (bin[u] < kBins)
-            queue[atomicAdd(&s_off[bin[u]], 1u)] = uint64_t(bin[u]) << 32 | (p0 + u * kKeyThreads);
+        if (key[u] != ~0u)
+            queue[atomicAdd(&s_off[key_bin(key[u])], 1u)] = uint64_t(key[u]) << 32 | (p0 + u * kKeyThreads);
 }
 
 // ------------------------------------------------------ per-warp techniques --
@@ -298,9 +312,11 @@ __device__ __forceinline__ uint32_t window_count_le(const uint32_t* w, uint32_t 
 // registers.  Neither set holds 2^32 - 1 here (matched apart), which marks the
 // positions past a set's or a window's end.
 //
-// A merge step is eight instructions, a round of some 500 elements about 330:
-// 0.65 warp instructions per element, where rings of blocks with masked indexes
-// and clamped ends took 2.7 (all pairs of 20000 sets merged: 15.1 ms against 21.7).
+// A merge step is eight instructions, a round of some 500 elements of sets of
+// similar size about 330.  200000 pairs of 20000 sets of 32 .. 2^18 elements, all
+// merged (most of very different sizes): 1.35 warp instructions per element,
+// bound by issue (83 %) and the shared-memory pipe (88 %), 15.1 ms; rings of
+// blocks with masked indexes and clamped ends took 2.7 and 21.6 ms.
 constexpr uint32_t kMergeWords = 2 * (kW + 32);  // per set: the window, then end marks that a lane's steps may run into
 __device__ uint32_t merge_pair(const uint32_t* A, uint64_t na, const uint32_t* B, uint64_t nb, uint32_t* win,
                                uint32_t lane) {
@@ -366,6 +382,76 @@ __device__ uint32_t merge_pair(const uint32_t* A, uint64_t na, const uint32_t* B
     return __reduce_add_sync(kFullMask, hits);
 }
 
+// SEARCH of sets of similar size (the larger below kStreamRatio times the
+// smaller): L streams through shared memory in windows of kSWin elements, the
+// next one landing (cp.async, 16 bytes a lane, coalesced) while the elements of
+// S up to the window's last value are binary-searched in this one, 32 at a time.
+// Reads every element of L once, 4 nl / ns bytes per element of S, where the
+// sampled search below takes some six random sectors; per element of S 2.4 warp
+// instructions at a ratio of 4 and 6 at 32, against 6.4.  The same pairs, all
+// searched: 9.6 ms with both, 15.2 ms with the sampled search alone.
+constexpr uint32_t kSWin = 512;
+constexpr uint32_t kSearchWords = 2 * kSWin;  // per warp
+static_assert(kSearchWords >= kMergeWords, "one region serves both");
+__device__ uint32_t stream_search_pair(const uint32_t* S, uint64_t ns, const uint32_t* L, uint64_t nl, uint32_t* win,
+                                       uint32_t lane) {
+    const uint32_t lo_v = max(__ldg(S), __ldg(L));
+    if (__ldg(S + ns - 1) < lo_v || __ldg(L + nl - 1) < lo_v) return 0;  // value ranges apart
+    const uint64_t s0 = warp_first_true(0, ns, [&](uint64_t i) { return __ldg(S + i) >= lo_v; });
+    const uint64_t l0 = warp_first_true(0, nl, [&](uint64_t i) { return __ldg(L + i) >= lo_v; });
+    // positions count from the 16-byte boundary below L[l0]; elements are [v0, v1)
+    const uint32_t v0 = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(L + l0) & 15u) >> 2);
+    const uint32_t* base = L + l0 - v0;
+    const uint32_t v1 = v0 + static_cast<uint32_t>(nl - l0), last_group = (v1 - 1) & ~3u;
+    const uint32_t at = smem_addr(win) + 16 * lane;
+    auto issue = [&](uint32_t w) {  // window w into its half; groups past the last read it again
+#pragma unroll
+        for (uint32_t q = 0; q < kSWin / 128; ++q)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + (w & 1) * kSWin * 4 + q * 512),
+                         "l"(base + min(w * kSWin + q * 128 + 4 * lane, last_group))
+                         : "memory");
+    };
+    uint64_t is = s0;
+    uint32_t hits = 0;
+    uint32_t v = is + lane < ns ? __ldg(S + is + lane) : 0xffffffffu;
+    const uint32_t windows = (v1 + kSWin - 1) / kSWin;
+    issue(0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (uint32_t w = 0; w < windows && is < ns; ++w) {
+        if (w + 1 < windows) issue(w + 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        uint32_t* sm = win + (w & 1) * kSWin;
+        // positions that are no elements get copies of the nearest one
+        if (w == 0 && lane < v0) sm[lane] = sm[v0];
+        if (w + 1 == windows) {
+            const uint32_t n = v1 - w * kSWin, last = sm[n - 1];
+            __syncwarp();
+            for (uint32_t x = n + lane; x < kSWin; x += 32) sm[x] = last;
+        }
+        __syncwarp();
+        const uint32_t top = sm[kSWin - 1];
+        for (;;) {
+            const bool valid = is + lane < ns && v <= top;
+            const uint32_t n = __popc(__ballot_sync(kFullMask, valid));  // valid lanes are a prefix
+            if (n) {
+                uint32_t pos = 0;
+#pragma unroll
+                for (uint32_t step = kSWin / 2; step > 0; step >>= 1) pos = sm[pos + step] <= v ? pos + step : pos;
+                hits += valid && sm[pos] == v ? 1u : 0u;
+                is += n;
+                v = is + lane < ns ? __ldg(S + is + lane) : 0xffffffffu;
+            }
+            if (n < 32) break;
+        }
+        __syncwarp();  // the half is read before the window after next lands in it
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    return __reduce_add_sync(kFullMask, hits);
+}
+
 // SEARCH: every element of the smaller set S, binary-searched in the larger
 // L, 256 elements of S at a time.  The window of L that can hold the block
 // comes from two 32-ary warp searches; a window longer than 512 elements is
@@ -378,6 +464,7 @@ constexpr uint32_t kSample = 256;
 __device__ uint32_t search_pair(const uint32_t* S, uint64_t ns, const uint32_t* L, uint64_t nl, uint32_t* samp,
                                int lane) {
     if (ns == 0 || nl == 0) return 0;
+    if (ns >= 32 && nl < kStreamRatio * ns && nl < kMaxStream) return stream_search_pair(S, ns, L, nl, samp, lane);
     uint32_t hits = 0;
     uint64_t from = 0;  // the windows advance monotonically
     for (uint64_t base = 0; base < ns; base += kW) {
@@ -594,7 +681,7 @@ struct BatchParams {
     const uint64_t* off;
     const uint32_t* pairs;
     uint32_t k;
-    const uint64_t* queue;   // bin in bits 32.., pair index below
+    const uint64_t* queue;   // key in bits 32.., pair index below
     const uint32_t* subset;  // when non-null: the queue is these pair indices, in order, all by `forced`
     uint64_t nqueue;         // queue length (all pairs, or the subset)
     uint32_t* counts;
@@ -652,7 +739,7 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
         const uint32_t skew = ((smem_addr(smem) + 4095u) & ~4095u) - smem_addr(smem);
         region = smem + skew / 4 + warp * (kWarpSmem / 4);
     } else {
-        __shared__ __align__(16) uint32_t windows[kBWarps][kMergeWords];
+        __shared__ __align__(16) uint32_t windows[kBWarps][kSearchWords];
         region = windows[warp];
     }
     // the queue is ready when its kernel's first successor runs; the second one
@@ -674,7 +761,7 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
         s_class = cls;
     }
     __syncthreads();
-    auto is_small = [&](uint64_t q) { return 255u - (static_cast<uint32_t>(p.queue[q] >> 35) & 255u) < s_class; };
+    auto is_small = [&](uint64_t q) { return key_class(static_cast<uint32_t>(p.queue[q] >> 32)) < s_class; };
     bool coop = !p.subset && s_q0 < s_q1 && !is_small(s_q0);  // CTA-uniform; the queue falls in cost
     for (;;) {
         uint64_t q;
@@ -705,7 +792,7 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
         } else {
             const uint64_t key = p.queue[q];
             pi = static_cast<uint32_t>(key);
-            tech = static_cast<uint8_t>((key >> 32) & 7u);
+            tech = key_tech(static_cast<uint32_t>(key >> 32));
         }
         const uint32_t a = p.pairs[2 * uint64_t(pi)], b = p.pairs[2 * uint64_t(pi) + 1];
         if (a >= p.k || b >= p.k) continue;  // recorded by the key kernel (cost 0: never taken by a CTA)

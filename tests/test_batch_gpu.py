@@ -194,3 +194,50 @@ def test_batched_config_full_pool(cuda):
         graph.close()
     want = oracle.pairs(el, off, off.size - 1, pairs, threads=os.cpu_count() or 1)
     np.testing.assert_array_equal(got, want)
+
+
+def crafted_pool(seed):
+    """Sets at the edges of the batch kernels' windows and routes: sizes around
+    256 and 512 elements, ratios around 4 and 32, starts at every 4-byte
+    phase, sets that end in 2^32 - 1, equal and nested sets, two far clusters."""
+    rng = np.random.default_rng(seed)
+    u = lambda n, hi: np.unique(rng.integers(0, hi, 2 * n + 8, dtype=np.uint64))[:n]
+    sets = [u(n, hi) for n in (1, 31, 32, 33, 255, 256, 257, 511, 512, 513, 1024, 1025, 8191, 8193, 16385, 40000)
+            for hi in (1 << 17, 1 << 32)]
+    big = u(70000, 1 << 24)
+    sets += [big, big[::2], big[::31], big[::33], big[1::64], big[:300], big[-300:], big[35000:35512]]
+    sets += [np.union1d(s, [0xffffffff]) for s in (big[::7], sets[9], sets[3])]
+    sets += [np.union1d(np.arange(5000), (1 << 32) - 5001 + np.arange(5000)), np.arange(3, 700), np.array([0xffffffff])]
+    return fmt.from_sets([s.astype(np.uint32) for s in sets])
+
+
+@pytest.mark.parametrize("tech", ["ip", "obs", "hi", "bitmap", "auto"])
+def test_windows_and_routes(cuda, tech):
+    """Every pair of the crafted pool, as one batch (whole CTAs take the large
+    pairs) and as batches of a few pairs, of one, and of 1025 (two blocks of the
+    queue kernels)."""
+    ds = crafted_pool(1)
+    k = ds.cardinality
+    col = collection(ds.elements, ds.offsets, ds.universe)
+    pairs = np.array([(a, b) for a in range(k) for b in range(k)], np.uint32)
+    want = oracle.pairs(ds.elements, ds.offsets, k, pairs)
+    np.testing.assert_array_equal(count(col, pairs, tech), want)
+    for n in (1, 7, 1024, 1025):
+        sel = np.random.default_rng(n).integers(0, len(pairs), n)
+        np.testing.assert_array_equal(count(col, pairs[sel], tech), want[sel])
+
+
+@pytest.mark.parametrize("tech", ["ip", "obs", "hi", "bitmap", "auto"])
+def test_few_large_pairs(cuda, tech):
+    """Pairs far above a warp's share: dense, sparse, nested, disjoint halves."""
+    rng = np.random.default_rng(3)
+    a = np.unique(rng.integers(0, 1 << 21, 400000)).astype(np.uint32)
+    b = np.unique(rng.integers(0, 1 << 31, 500000, dtype=np.uint64)).astype(np.uint32)
+    c = np.unique(np.concatenate([a[::3], b[::5]])).astype(np.uint32)
+    ds = fmt.from_sets([a, b, c, a[:200000], a[200000:], b[::40].copy(), np.array([7], np.uint32)])
+    k = ds.cardinality
+    pairs = np.array([(x, y) for x in range(k) for y in range(k)], np.uint32)
+    want = oracle.pairs(ds.elements, ds.offsets, k, pairs)
+    col = collection(ds.elements, ds.offsets, ds.universe)
+    np.testing.assert_array_equal(count(col, pairs, tech), want)
+    np.testing.assert_array_equal(count(col, pairs[:2], tech), want[:2])
