@@ -100,14 +100,23 @@ def log(*a):
     print(*a, file=sys.stderr, flush=True)
 
 
-SKEW_RATIO = 64  # SI_TECH_AUTO: obs when one set is more than this many times the other
+def auto_engine(small, large, elements):
+    """What SI_TECH_AUTO runs for one pair: a much smaller set is searched for
+    in the larger (obs), small pairs are merged (ip), and the rest streams
+    through window bitmaps."""
+    total = small + large
+    ratio = 16 if elements and total <= 1 << 25 else 32 if total <= 1 << 27 else 64
+    if total > (IP_TILE if elements else 1 << 18) and small <= large // ratio:
+        return "obs"
+    return "ip" if total <= 1 << 24 else "bitmap"
+
+
 IP_TILE = 5184  # merged elements per tile of the intersect-path kernels
 
 # DRAM bytes (read + write) per launch of the dominant kernel, from ncu
 # captures summarised in profiles/: the bitmap engine's bp_stream_kernel
 # measured at full size (a one-pass dram__bytes capture of the 2^28 x 2^28
-# launch); the ip tile kernel from its 2^25 x 2^25 capture scaled by 8 (tiles,
-# inputs and matches grow in proportion).
+# launch).
 TRAFFIC_PER_LAUNCH = {
     "bitmap/sisi_large/out": 2.246e9 + 121.53e6,   # one-pass dram__bytes capture of the 2^28 stream kernel
     "bitmap/sisi_mid/out": 321.59e6 + 5.21e6,      # from the 2^25 full capture
@@ -383,8 +392,7 @@ def run_ours(args, rank: int, world: int):
     tile_ms, tile_n = ctypes.c_double(0), ctypes.c_uint64(0)
     lib.si_timer_read(b"sisi_tile", ctypes.byref(tile_ms), ctypes.byref(tile_n))
     phases = {}
-    for ph in ("sisi_split", "sisi_tile", "sisi_scan", "sisi_copy", "obs_sample", "obs_search",
-               "obs_compact"):
+    for ph in ("sisi_split", "sisi_tile", "sisi_scan", "sisi_copy", "obs_search", "obs_compact"):
         p_ms, p_n = ctypes.c_double(0), ctypes.c_uint64(0)
         lib.si_timer_read(ph.encode(), ctypes.byref(p_ms), ctypes.byref(p_n))
         if p_n.value:
@@ -477,19 +485,16 @@ def run_ours(args, rank: int, world: int):
     peak = peaks.get("hbm_gbs", FALLBACK_HBM_GBS)
     peak_src = "measured" if "hbm_gbs" in peaks else "fallback"
     alg_bytes = 4 * (n_a + n_b) + (4 * c if args.materialize else 0)
-    # the engine that ran: auto merges small pairs (ip), searches a much smaller
-    # set in the larger (obs) and streams the rest through window bitmaps
     engine = args.technique
     if engine == "auto":
-        engine = ("ip" if n_a + n_b <= 1 << 21 else "obs" if min(n_a, n_b) * SKEW_RATIO < max(n_a, n_b)
-                  else "ip" if n_a + n_b <= 1 << 24 else "bitmap")
+        engine = auto_engine(min(n_a, n_b), max(n_a, n_b), args.materialize)
     tiles = max(1, -(-(n_a + n_b) // IP_TILE))
     ip_launches = (1 if tiles == 1 else 3 if tiles > 4096 or (tiles <= 2048 and args.materialize) else 2)
     kernel, launches = {
         "ip": ("ip_group_kernel" if tiles > 2048 and args.materialize else "ip_tile_kernel", ip_launches),
         "hi": ("bh_stream_kernel", 2 if args.materialize else 1),
         "bitmap": ("bp_stream_kernel", 2 if args.materialize else 1),
-        "obs": ("obs_search_kernel", 3 if args.materialize else 2),
+        "obs": ("obs_search_kernel", 2),
     }[engine]
     if engine == "obs":
         tile_avg_ms = phases.get("obs_search")

@@ -82,10 +82,12 @@ const char* si_last_error_string(void);
  * of the smaller set, through windows of 32768 values (two bitmaps per warp,
  * AND and popcount), and orders the output by a scan of the range counts,
  * through a scratch array as long as the smaller set (so its workspace is
- * about 4 min(nA, nB) bytes larger); OBS searches every element of the smaller set in the larger one
- * (cached top levels in shared memory); AUTO takes IP for pairs of up to 2^21
- * elements in all, else OBS when one set is more than 64 times larger than the
- * other, else IP up to 2^24 elements in all and BITMAP above.
+ * about 4 min(nA, nB) bytes larger); OBS searches every element of the smaller
+ * set in the larger one (samples of it in shared memory, then interpolation);
+ * AUTO takes OBS when one set is 32 times larger than the other (16 times with
+ * elements written and up to 2^25 elements in all, 64 times above 2^27; not for
+ * pairs of up to 5184 elements, or 2^18 when only counted), else IP up to 2^24
+ * elements in all and BITMAP above.
  *
  * d_count: device uint64, receives |A ∩ B|.
  * d_out:   device uint32[out_cap] or NULL (count only).  When non-NULL,
@@ -327,9 +329,8 @@ si_status si_misi_dense(const uint32_t* d_elements, const uint64_t* d_offsets, u
  * "sisi_split", "sisi_tile", and for BITMAP with elements "sisi_scan",
  * "sisi_copy"; dense all pairs "mm_incidence", "mm_gemm",
  * "naive_bitmaps", "naive_popcount"; all pairs of a tile "misi_plan",
- * "misi_slab" (bitmap), "misi_probe"; single pair by search "obs_sample", "obs_search" (with the
- * offsets scan when elements are written), "obs_compact"; batched pairs
- * "batch_plan", "batch_count".  The events come from a pool that
+ * "misi_slab" (bitmap), "misi_probe"; single pair by search "obs_search" and
+ * "obs_compact" (adds up the counts, writes the elements); batched pairs "batch_plan", "batch_count".  The events come from a pool that
  * si_timer_reset refills, so a timed launch costs two event records.
  * si_timer_read synchronises on the recorded events and returns the summed
  * milliseconds and the number of launches of one phase.

@@ -186,7 +186,7 @@ si_status si_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t 
         case SI_TECH_IP:
             return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s);
         case SI_TECH_AUTO:
-            switch (si::sisi_auto(nA, nB)) {
+            switch (si::sisi_auto(nA, nB, d_out != nullptr)) {
                 case SI_TECH_IP:
                     return si::ip_sisi(dA, nA, dB, nB, d_count, d_out, out_cap, d_workspace, workspace_bytes, s);
                 case SI_TECH_OBS:

@@ -66,6 +66,7 @@ private:
 
 // ---- one pair ----
 // Intersect path (si_sisi_ip.cu).
+constexpr uint64_t kIpOneTile = 192 * 27;  // a tile of ip: elements of both sets that one CTA merges
 size_t ip_workspace_size(uint64_t nA, uint64_t nB);
 si_status ip_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
                   uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream);
@@ -75,14 +76,28 @@ size_t bm_workspace_size(uint64_t nA, uint64_t nB);
 si_status bm_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
                   uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream,
                   bool hash = false);
-// What SI_TECH_AUTO runs for a pair.  Device time with elements out, ip /
-// bitmap / obs: 2^17 x 2^17 10 / 35 / 14 us, 2^20 x 2^20 17 / 36 / 34, 2^23 x 2^23
-// 43 / 45 / 186, 2^24 x 2^24 77 / 63; 1000 x 2^20 9 / 21 / 12 us, 10000 x 2^21
-// 12.4 / 21 / 12.1, 30000 x 2^23 21 / 25 / 15.
-inline si_technique sisi_auto(uint64_t nA, uint64_t nB) {
+// What SI_TECH_AUTO runs for a pair.  Device time with elements out (counted
+// only), us:
+//                       ip           bitmap       obs
+//   2^20 x 2^20           17 (8)       36 (25)      25 (21)
+//   2^23 x 2^23           43 (23)      45 (31)      159 (138)
+//   2^24 x 2^24           77           63
+//   2^17, 1/16 of it      8.7 (5.0)                 6.6 (5.2)
+//   2^17, 1/32            8.7 (5.0)                 6.7 (5.6)
+//   2^20, 1/16            11.0 (6.0)                7.3 (6.1)
+//   2^22, 1/8             17.7 (9.5)   25.7 (16.7)  17.1 (14.2)
+//   2^22, 1/16            17.1 (9.1)   24.6 (16.5)  12.0 (10.0)
+//   2^22, 1/32            16.4 (8.9)   23.2 (16.4)  9.1 (7.7)
+//   2^24, 1/16            36 (20)      37 (27)      28 (24)
+//   2^24, 1/32            36 (19)      37 (27)      19 (16)
+//   2^27, 1/16            204 (130)    155 (115)    210 (185)
+//   2^27, 1/32            192 (122)    147 (111)    139 (125)
+//   2^27, 1/64            187 (117)    141 (108)    110 (101)
+// A pair of one merge tile is one launch of ip: 3.8 us against 4.2 and more.
+inline si_technique sisi_auto(uint64_t nA, uint64_t nB, bool elements) {
     const uint64_t small = nA < nB ? nA : nB, large = nA < nB ? nB : nA, total = nA + nB;
-    if (total <= (1ull << 21)) return SI_TECH_IP;
-    if (small * 64 < large) return SI_TECH_OBS;
+    const uint64_t ratio = elements && total <= (1ull << 25) ? 16 : total <= (1ull << 27) ? 32 : 64;
+    if (total > (elements ? kIpOneTile : 1ull << 18) && small <= large / ratio) return SI_TECH_OBS;
     return total <= (1ull << 24) ? SI_TECH_IP : SI_TECH_BITMAP;
 }
 size_t obs_workspace_size(uint64_t nA, uint64_t nB);

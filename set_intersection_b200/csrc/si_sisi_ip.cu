@@ -53,6 +53,7 @@ constexpr int kIpThreads = 192;
 constexpr int kIpWarps = kIpThreads / 32;
 constexpr int kVT = 27;  // merge steps per thread: odd, so that consecutive threads' shared loads spread over the banks
 constexpr uint32_t kTile = kIpThreads * kVT;
+static_assert(kTile == kIpOneTile, "the engine's choice counts tiles");
 constexpr int kIpCtasPerSm = 8;
 // both ranges, their successors, the alignment of both, and the steps by which
 // a thread's reads can run over when the sets are not sorted

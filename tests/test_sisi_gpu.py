@@ -292,6 +292,35 @@ def test_obs_lane_groups_and_chunking(cuda, n_small):
         check(big, small, "obs")
 
 
+@pytest.mark.parametrize("spread", ["even", "dense", "steps", "clusters"])
+@pytest.mark.parametrize("n_large", [1, 2, 255, 256, 257, 1023, 1024, 1025, 65537, 300001])
+def test_obs_windows(cuda, n_large, spread):
+    """obs with samples 1, 2 and many elements apart and the last window short,
+    values that interpolation finds at once or hardly ever, and searches below
+    the first, above the last and between all elements; few chunks (many
+    samples each) and more than 148 of them."""
+    rng = np.random.default_rng(n_large)
+    if spread == "even":
+        big = _u(rng, n_large, 1 << 32)
+    elif spread == "dense":
+        big = (np.arange(n_large, dtype=np.uint64) + 77).astype(np.uint32)
+    elif spread == "steps":  # runs of consecutive values, gaps doubling
+        i = np.arange(n_large, dtype=np.uint64)
+        big = np.unique(i + (np.uint64(1) << np.minimum(i * 31 // max(1, n_large), 30)))
+        big = big.astype(np.uint32)
+    else:
+        c = rng.integers(0, 1 << 32, size=max(1, n_large // 1000), dtype=np.uint64)
+        big = np.unique((rng.choice(c, n_large) + rng.geometric(1e-3, n_large).astype(np.uint64)) & 0xFFFFFFFF)
+        big = big.astype(np.uint32)
+    near = np.concatenate([big, big + np.uint32(1), big - np.uint32(1)])
+    for n_small in (min(64, big.size), min(148 * 256, big.size), min(148 * 256 + 1, big.size)):
+        small = np.unique(rng.choice(near, size=max(1, n_small)))
+        if rng.integers(2):
+            small = np.unique(np.concatenate([small, np.array([0, 0xFFFFFFFF], dtype=np.uint32)]))[:big.size]
+        check(small, big, "obs")
+        check(small, big, "auto")
+
+
 IP_TILE = 192 * 27  # merged elements per tile of the intersect-path kernels
 
 
