@@ -319,6 +319,9 @@ __device__ __forceinline__ bool merge_tile(uint64_t nA, uint64_t nB, const TileR
             if (take_a) ++i; else ++j;
         }
     }
+    // a thread of sets that are not sorted can step past the tile's A elements:
+    // no match is read from there
+    if (na - i0 < 32) mask &= (1u << (na - i0)) - 1;
     return true;
 }
 
