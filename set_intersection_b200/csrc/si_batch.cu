@@ -981,6 +981,8 @@ si_status batch_tune(const uint32_t* d_elements, const uint64_t* d_offsets, uint
     std::memcpy(table_out, T.t, kTableSize);
     const BatchLayout L = batch_layout(npairs);
     if (ws_bytes < L.total) return SI_ERR_WORKSPACE_TOO_SMALL;
+    // the error words: a batch without a bucket of 32 pairs launches nothing else that clears them
+    SI_CUDA_TRY(cudaMemsetAsync(ws, 0, kBatchHeader, stream));
     if (npairs == 0) return SI_OK;
     // bucket of every pair, on the device, read back
     unsigned char* w = static_cast<unsigned char*>(ws);

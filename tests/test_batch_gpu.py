@@ -241,3 +241,17 @@ def test_few_large_pairs(cuda, tech):
     col = collection(ds.elements, ds.offsets, ds.universe)
     np.testing.assert_array_equal(count(col, pairs, tech), want)
     np.testing.assert_array_equal(count(col, pairs[:2], tech), want[:2])
+
+
+@pytest.mark.parametrize("npairs", [1, 40])
+def test_tune_few_pairs_on_a_used_workspace(cuda, npairs):
+    """A batch without a bucket of 32 pairs: the tuner times nothing, and what
+    the workspace held before is not taken for an error."""
+    from set_intersection_b200 import _lib, api, generate
+    el, off = generate.loguniform(21, 50, 1, 1 << 14, 1 << 20)
+    pairs = generate.random_pairs(22, 50, npairs)
+    col = collection(el, off, (1 << 20) - 1)
+    ws = api.Workspace()
+    ws.get(_lib.lib.si_batch_workspace_size(npairs)).fill_(0xF5)
+    table = api.batch_tune(col, dev(pairs.view(np.int32)), workspace=ws)
+    np.testing.assert_array_equal(count(col, pairs, "auto", table, ws), oracle.pairs(el, off, 50, pairs))
