@@ -1,5 +1,5 @@
 // si_sisi_bitmap.cu -- technique bitmap for one pair of large sorted sets
-// (and SI_TECH_AUTO for pairs of similar size).
+// (and SI_TECH_AUTO for pairs of similar size above 2^24 elements in all).
 //
 // Replaces the single-instance path of bitmap_dynamic (src/bitmap_dynamic.cu:
 // 168-176: constructBitmap over the whole universe, singleInstanceIntersect,
