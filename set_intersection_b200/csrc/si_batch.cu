@@ -348,7 +348,9 @@ __device__ uint32_t merge_pair(const uint32_t* A, uint64_t na, const uint32_t* B
         const uint32_t cB = max_b <= m && !last_round ? kW : window_count_le(wb, m - (last_round ? 1u : 0u), lane);
         ia += cA;
         ib += cB;
-        const bool more = ia < na && ib < nb;
+        // both sets end in a last round's windows; in sets padded with 2^32 - 1
+        // it may take nothing, so it also ends the loop
+        const bool more = !last_round && ia < na && ib < nb;
         if (more) {  // the next windows, in flight during the merge
             fetch_window(A, ia, na, lane, ra);
             fetch_window(B, ib, nb, lane, rb);

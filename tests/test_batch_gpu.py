@@ -255,3 +255,21 @@ def test_tune_few_pairs_on_a_used_workspace(cuda, npairs):
     ws.get(_lib.lib.si_batch_workspace_size(npairs)).fill_(0xF5)
     table = api.batch_tune(col, dev(pairs.view(np.int32)), workspace=ws)
     np.testing.assert_array_equal(count(col, pairs, "auto", table, ws), oracle.pairs(el, off, 50, pairs))
+
+
+@pytest.mark.parametrize("pad", [2, 255, 300, 700])
+def test_merge_ends_on_padded_sets(cuda, pad):
+    """Sets padded with 2^32 - 1 break the rule that a set has no duplicates,
+    but the merge ends on them, in a warp's pairs and in whole CTAs' (the pairs
+    of 200000 elements), counts each value once, and leaves the others alone."""
+    rng = np.random.default_rng(pad)
+    top = 0xffffffff
+    plain = [np.unique(rng.integers(0, hi, n)) for n, hi in ((40, 1 << 8), (900, 1 << 12), (3000, 1 << 13))]
+    plain += [np.unique(rng.integers(0, 1 << 19, 200000)) for _ in range(2)]
+    sets = plain + [np.concatenate([s, np.full(n, top)]) for s in plain for n in (1, pad)]
+    ds = fmt.from_sets([s.astype(np.uint32) for s in sets])
+    pairs = np.array([(a, b) for a in range(len(sets)) for b in range(len(sets))], np.uint32)
+    want = np.array([len(np.intersect1d(sets[a], sets[b])) for a, b in pairs], np.uint32)
+    col = collection(ds.elements, ds.offsets, top)
+    np.testing.assert_array_equal(count(col, pairs, "ip"), want)
+    np.testing.assert_array_equal(count(col, pairs[-1:], "ip"), want[-1:])
