@@ -150,9 +150,8 @@ MisiLayout misi_layout(si_set_range A, si_set_range B, si_technique t) {
 }
 
 // ------------------------------------------------------------------ plan --
-// Sum over the warp's active lanes (a prefix of the warp), in lane 0.
-__device__ __forceinline__ uint64_t warp_sum_active(uint32_t v) {
-    const uint32_t m = __activemask();
+// Sum over the warp's lanes of mask m, all of which make the call.
+__device__ __forceinline__ uint64_t warp_sum_masked(uint32_t m, uint32_t v) {
     const uint64_t lo = __reduce_add_sync(m, v & 0xffffu), hi = __reduce_add_sync(m, v >> 16);
     return lo + (hi << 16);
 }
@@ -264,6 +263,9 @@ __global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint32_t* __
     s_size[tid] = tid < tile ? size_of(j0 + tid) : 0u;
     __syncthreads();
     const uint32_t i = blockIdx.x * kRankTile + tid;
+    // the warp's lanes that hold a set (the first ones); what comes next may
+    // split the warp, so the reductions below name them
+    const uint32_t lanes = __ballot_sync(kFullMask, i < n);
     if (i >= n) return;
     const uint32_t size = size_of(i);
     const bool iA = i < nA;
@@ -311,15 +313,15 @@ __global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint32_t* __
     if (before) atomicAdd(own + i, (before_sum << kRankBits) | before);
     if (larger) atomicAdd(other + i, (larger_sum << kRankBits) | larger);
     if (blockIdx.y == 0) {
-        const uint64_t sumA = warp_sum_active(iA ? size : 0u), sumB = warp_sum_active(iA ? 0u : size);
+        const uint64_t sumA = warp_sum_masked(lanes, iA ? size : 0u);
+        const uint64_t sumB = warp_sum_masked(lanes, iA ? 0u : size);
         uint32_t vmin = 0, vmax = 0;
         if (size) {
             vmin = ~__ldg(el + off[set_id(i)]);
             vmax = __ldg(el + off[set_id(i) + 1] - 1);
         }
-        const uint32_t m = __activemask();
-        vmin = __reduce_max_sync(m, vmin);
-        vmax = __reduce_max_sync(m, vmax);
+        vmin = __reduce_max_sync(lanes, vmin);
+        vmax = __reduce_max_sync(lanes, vmax);
         if ((tid & 31) == 0) {
             unsigned long long* totals = reinterpret_cast<unsigned long long*>(header + kMisiTotals);
             if (sumA) atomicAdd(totals, sumA);

@@ -294,3 +294,22 @@ def test_bucket_search_edges(cuda, tech, span):
     ds, col = from_sets([s.astype(np.uint32) for s in sets])
     want = oracle.all_pairs(ds.elements, ds.offsets, ds.cardinality, ds.universe, "std")
     np.testing.assert_array_equal(run(col, tech), want)
+
+
+@pytest.mark.parametrize("n_a,n_b", [(1, 30), (17, 16), (33, 62), (95, 130), (300, 213)])
+def test_plan_totals_of_split_warps(cuda, n_a, n_b):
+    """A warp of the plan holds sets of both sides, empty ones, and lanes past
+    the last set: the totals and the range of the values still cover every set
+    (bitmap and hi leave out values outside the range, obs has work items for the
+    totals alone)."""
+    rng = np.random.default_rng(n_a)
+    k = n_a + n_b
+    sets = [np.unique(rng.integers(1 << 19, (1 << 19) + 4000, rng.integers(0, 200))) for _ in range(k)]
+    for i in range(0, k, 5):
+        sets[i] = sets[i][:0]
+    sets[n_a - 1] = np.union1d(sets[n_a - 1], [3, 9, 1 << 20])       # the smallest and the largest value
+    sets[k - 1] = np.union1d(sets[k - 1], [5, 9, (1 << 20) + 31])    # lie in single lanes
+    ds, col = from_sets([s.astype(np.uint32) for s in sets])
+    want = np.array([[len(np.intersect1d(sets[a], sets[n_a + b])) for b in range(n_b)] for a in range(n_a)])
+    for tech in ("bitmap", "hi", "obs"):
+        np.testing.assert_array_equal(run(col, tech, (0, n_a), (n_a, k)).reshape(n_a, n_b), want)
