@@ -228,9 +228,8 @@ __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
 // The queue: every pair (its key in bits 32.., its index below) at its bin's
 // offset.  A CTA scans the histogram itself and reserves room in each bin once;
 // the order within a bin does not matter.
-__global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t* __restrict__ bins, uint64_t npairs,
-                                                                  const uint32_t* __restrict__ hist,
-                                                                  uint32_t* __restrict__ cursor,
+__global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t* bins, uint64_t npairs,
+                                                                  const uint32_t* hist, uint32_t* __restrict__ cursor,
                                                                   uint64_t* __restrict__ queue,
                                                                   unsigned char* header) {
     __shared__ uint32_t s_off[kBins];    // the bin's offset, then where this CTA's next pair of it goes
@@ -244,7 +243,7 @@ __global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t
     uint32_t v[kPer], sum = 0;
 #pragma unroll
     for (uint32_t q = 0; q < kPer; ++q) {
-        v[q] = __ldcg(hist + threadIdx.x * kPer + q);
+        v[q] = hist[threadIdx.x * kPer + q];
         sum += v[q];
     }
     const uint32_t incl = warp_inclusive_scan(sum);

@@ -33,7 +33,9 @@ int sm_count();
 // Launches `kernel` with programmatic stream serialization: it may start while
 // the previous kernel on the stream finishes, and must execute
 // griddepcontrol.wait before it reads that kernel's results (or writes what
-// that kernel still reads).
+// that kernel still reads).  It reads them by plain or L2 loads: __ldg, or
+// const __restrict__ on the parameter, would promise that nobody writes them
+// while it runs, and let the compiler move the loads above the wait.
 template <class Kernel, class... Args>
 si_status launch_dependent(Kernel kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};

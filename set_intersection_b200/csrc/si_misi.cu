@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kRankTile) misi_rank_kernel(const uint32_t* __
 constexpr int kOrderThreads = 256;
 __global__ void __launch_bounds__(kOrderThreads) misi_order_kernel(
     const uint64_t* __restrict__ off, uint32_t a_start, uint32_t nA, uint32_t b_start, uint32_t nB, bool self,
-    ItemUnit rule, const unsigned long long* __restrict__ own, const unsigned long long* __restrict__ other,
+    ItemUnit rule, const unsigned long long* own, const unsigned long long* other,
     uint64_t* __restrict__ keys, uint64_t* __restrict__ P, uint32_t* __restrict__ cs, uint64_t* __restrict__ nseg,
     uint64_t* __restrict__ items, unsigned char* header) {
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the ranks

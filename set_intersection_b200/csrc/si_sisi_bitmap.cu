@@ -298,10 +298,9 @@ __global__ void __launch_bounds__(kStBlock, kStCtasPerSm) bh_stream_kernel(
 // and each lane keeps 16 loads in flight.  The warp of the last range writes
 // the total count.
 constexpr int kCopyUnroll = 16;
-__global__ void __launch_bounds__(256) bp_copy_kernel(const uint32_t* __restrict__ tile_count,
-                                                      const uint64_t* __restrict__ tile_off,
-                                                      const uint64_t* __restrict__ split_y, uint64_t nTiles,
-                                                      const uint32_t* __restrict__ scratch, uint32_t* __restrict__ out,
+__global__ void __launch_bounds__(256) bp_copy_kernel(const uint32_t* tile_count, const uint64_t* tile_off,
+                                                      const uint64_t* split_y, uint64_t nTiles,
+                                                      const uint32_t* scratch, uint32_t* __restrict__ out,
                                                       uint64_t out_cap, uint64_t* __restrict__ d_count, uint32_t* err) {
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the counts, offsets and hits of the tile kernel
     const uint32_t lane = threadIdx.x & 31;
@@ -330,7 +329,7 @@ __global__ void __launch_bounds__(256) bp_copy_kernel(const uint32_t* __restrict
 #pragma unroll
             for (int u = 0; u < kCopyUnroll; ++u) {
                 const uint32_t i = i0 + 32 * u + lane;
-                v[u] = i < n ? __ldg(scratch + src + i) : 0u;
+                v[u] = i < n ? scratch[src + i] : 0u;
             }
 #pragma unroll
             for (int u = 0; u < kCopyUnroll; ++u) {

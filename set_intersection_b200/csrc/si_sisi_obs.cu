@@ -196,8 +196,7 @@ __global__ void __launch_bounds__(kObsThreads, kObsSearchCtasPerSm)
 // element output it is the only one and has no words.
 template <bool kOut>
 __global__ void __launch_bounds__(kObsThreads) obs_compact_kernel(const uint32_t* __restrict__ S,
-                                                                  const uint32_t* __restrict__ mask,
-                                                                  const uint32_t* __restrict__ ccount,
+                                                                  const uint32_t* mask, const uint32_t* ccount,
                                                                   uint32_t* __restrict__ out,
                                                                   uint64_t* __restrict__ d_count, uint64_t nChunks,
                                                                   uint64_t per, uint32_t W, uint32_t seg) {
@@ -208,7 +207,7 @@ __global__ void __launch_bounds__(kObsThreads) obs_compact_kernel(const uint32_t
     const uint64_t c0 = kOut ? blockIdx.x * per : nChunks;
     uint64_t sum = 0;
 #pragma unroll 8
-    for (uint64_t i = threadIdx.x; i < c0; i += kObsThreads) sum += __ldg(ccount + i);
+    for (uint64_t i = threadIdx.x; i < c0; i += kObsThreads) sum += ccount[i];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(kFullMask, sum, d);
     if (lane == 0) s_sum[warp] = sum;
@@ -220,7 +219,7 @@ __global__ void __launch_bounds__(kObsThreads) obs_compact_kernel(const uint32_t
         const uint64_t end = (c0 + per < nChunks ? c0 + per : nChunks) * W;
         for (uint64_t b = c0 * W; b < end; b += uint64_t(kObsWarps) * seg) {
             const uint64_t w0 = b + uint64_t(warp) * seg;
-            const uint32_t word = lane < seg && w0 + lane < end ? __ldg(mask + w0 + lane) : 0u;
+            const uint32_t word = lane < seg && w0 + lane < end ? mask[w0 + lane] : 0u;
             const uint32_t n = __popc(word);
             const uint32_t incl = warp_inclusive_scan(n);
             if (lane == 31) s_warp[warp] = incl;
