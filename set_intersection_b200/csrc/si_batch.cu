@@ -744,7 +744,9 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
         region = windows[warp];
     }
     // the queue is ready when its kernel's first successor runs; the second one
-    // may then start while the first one's last CTAs run
+    // may then start while the first one's last CTAs run.  It has not waited for
+    // the queue's kernel itself, so it (the stream kernel) reads the queue from
+    // L2, where it lies whole
     if (p.first) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
@@ -762,7 +764,8 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
         s_class = cls;
     }
     __syncthreads();
-    auto is_small = [&](uint64_t q) { return key_class(static_cast<uint32_t>(p.queue[q] >> 32)) < s_class; };
+    auto key_of = [&](uint64_t q) { return kStream ? ld_relaxed_u64(p.queue + q) : p.queue[q]; };
+    auto is_small = [&](uint64_t q) { return key_class(static_cast<uint32_t>(key_of(q) >> 32)) < s_class; };
     bool coop = !p.subset && s_q0 < s_q1 && !is_small(s_q0);  // CTA-uniform; the queue falls in cost
     for (;;) {
         uint64_t q;
@@ -791,7 +794,7 @@ __global__ void __launch_bounds__(kBThreads, kStream ? kStreamCtasPerSm : kSearc
             pi = p.subset[q];
             tech = static_cast<uint8_t>(p.forced);
         } else {
-            const uint64_t key = p.queue[q];
+            const uint64_t key = key_of(q);
             pi = static_cast<uint32_t>(key);
             tech = key_tech(static_cast<uint32_t>(key >> 32));
         }
