@@ -103,7 +103,7 @@ struct MisiLayout {
     uint32_t nA = 0, nB = 0, rows = 0;
     bool self = true;
     size_t off_keys_in = 0, off_keys = 0, off_sizes = 0, off_P = 0, off_cs = 0, off_nseg = 0, off_items = 0,
-           off_cub = 0, cub_bytes = 0, off_acc = 0, off_slab = 0, total = 0;
+           off_cub = 0, cub_bytes = 0, off_slab = 0, total = 0;
 };
 
 // Sort key of a set: size descending, then local index ascending.
@@ -119,9 +119,12 @@ MisiLayout misi_layout(si_set_range A, si_set_range B, si_technique t) {
     L.rows = L.nA + L.nB;
     const uint64_t n = L.rows;
     size_t o = kMisiHeader;
+    // Up to kRankRows sets neither keys_in nor sizes is used, and they hold the
+    // ranks' accumulators (own, other): a smaller tile never needs more room
+    // than a larger one.
     L.off_keys_in = o;  o = align_up(o + n * 8, 256);
-    L.off_keys = o;     o = align_up(o + n * 8, 256);
     L.off_sizes = o;    o = align_up(o + (n + 2) * 8, 256);  // sorted sizes (u64), per side
+    L.off_keys = o;     o = align_up(o + n * 8, 256);
     L.off_P = o;        o = align_up(o + (n + 2) * 8, 256);  // prefix sums per side: nA + 1, nB + 1
     L.off_cs = o;       o = align_up(o + n * 4, 256);
     L.off_nseg = o;     o = align_up(o + (n + 1) * 8, 256);
@@ -140,8 +143,6 @@ MisiLayout misi_layout(si_set_range A, si_set_range B, si_technique t) {
     L.cub_bytes = align_up(std::max(sort_bytes, scan_bytes), 256);
     L.off_cub = o;
     o += L.cub_bytes;
-    L.off_acc = o;  // the ranks' accumulators
-    o = align_up(o + (n <= kRankRows ? n * 16 : 0), 256);
     L.off_slab = o;  // the value-major matrix of techniques bitmap and hi
     if ((t == SI_TECH_BITMAP || t == SI_TECH_HI) && L.rows >= kSlabMinRows) o += kSlabBytes;
     if (t == SI_TECH_HI && L.rows >= kSlabMinRows) o += kSlabKeyBytes;
@@ -796,9 +797,9 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
     const ItemUnit rule = item_rule(t);
     if (L.rows <= kRankRows) {
         PhaseTimer timer("misi_plan", stream);
-        unsigned long long* own = reinterpret_cast<unsigned long long*>(w + L.off_acc);
-        unsigned long long* other = own + L.rows;
-        SI_CUDA_TRY(cudaMemsetAsync(own, 0, size_t(L.rows) * 16, stream));
+        unsigned long long* own = reinterpret_cast<unsigned long long*>(w + L.off_keys_in);
+        unsigned long long* other = reinterpret_cast<unsigned long long*>(w + L.off_sizes);
+        SI_CUDA_TRY(cudaMemsetAsync(own, 0, L.off_sizes - L.off_keys_in + size_t(L.rows) * 8, stream));
         const unsigned tiles = (L.rows + kRankTile - 1) / kRankTile;
         misi_rank_kernel<<<dim3(tiles, tiles), kRankTile, 0, stream>>>(d_elements, d_offsets, A.start, L.nA, B.start,
                                                                        L.nB, own, other, w);

@@ -272,3 +272,16 @@ def test_bounded_wait_gives_up_and_reports(cuda):
     b = torch.arange(0, 1000, 3, dtype=torch.int32, device=cuda)
     c, _ = api.intersect(a, b, "auto")
     assert c == 167
+
+
+def test_misi_workspace_grows_with_the_tile():
+    """One buffer of the largest tile's size serves the smaller tiles of a run:
+    no tile needs less room than one of fewer sets, whichever way the plan orders
+    them (16384 sets is the most it ranks by counting)."""
+    L = si.lib
+    R = _lib.SetRange
+    for t in (Technique.IP, Technique.OBS, Technique.HI, Technique.BITMAP, Technique.AUTO):
+        for cross in (False, True):
+            sizes = [L.si_misi_workspace_size(R(0, k // 2 if cross else k), R(k // 2, k) if cross else R(0, k), int(t))
+                     for k in (2, 31, 32, 33, 1000, 8192, 16000, 16383, 16384, 16385, 16400, 17000, 40000)]
+            assert sizes == sorted(sizes)
