@@ -81,23 +81,37 @@ constexpr uint32_t kTableSize = 1024;    // 4 density classes x 16 size classes 
 
 // The queue's bins: part (1 bit), falling cost class (7 bits), a hash of the
 // larger set (4 bits), so that the pairs of a set run close together in time and
-// find it in L2.  A pair's 16-bit key has its technique above the bin.
+// find it in L2.  A pair's 16-bit key has its technique above the bin.  shift = 1
+// leaves out the hash's last bit.
 constexpr uint32_t kBins = 4096;
-__host__ __device__ constexpr uint32_t key_bin(uint32_t key) { return key & (kBins - 1); }
+__host__ __device__ constexpr uint32_t key_bin(uint32_t key, uint32_t shift) { return (key & (kBins - 1)) >> shift; }
 __host__ __device__ constexpr uint32_t key_class(uint32_t key) { return 127u - ((key >> 4) & 127u); }
 __host__ __device__ constexpr uint8_t key_tech(uint32_t key) { return static_cast<uint8_t>((key >> 12) & 7u); }
 constexpr int kKeyThreads = 256;
 constexpr uint32_t kKeyPairs = 4;  // pairs per thread of the key and queue kernels
+// Up to kPlanMost pairs are ordered by one CTA, whose histogram needs no room
+// outside it, and up to kHalfBins the others' has half of the bins: two 64-bit
+// words a pair of workspace are enough for a batch of any size.  A whole call,
+// one CTA against two kernels: 1 short pair 16.5 us against 17.2, 1000 pairs 20.7
+// and 24.6, 3000 26.4 and 26.2, 4500 29.5 and 27.3.  200000 pairs with half of the
+// bins: 8.48 ms against 8.39.
+constexpr int kPlanThreads = 1024;
+constexpr uint32_t kPlanPairs = 3;  // per thread
+constexpr uint64_t kPlanMost = uint64_t(kPlanThreads) * kPlanPairs;
+constexpr uint64_t kHalfBins = 8192;
 
 struct BatchLayout {
+    uint32_t shift = 0;
     size_t off_hist = 0, off_cursor = 0, off_bins = 0, off_queue = 0, total = 0;
 };
 
 BatchLayout batch_layout(uint64_t npairs) {
     BatchLayout L;
+    L.shift = npairs <= kHalfBins ? 1 : 0;
+    const size_t bins = npairs > kPlanMost ? kBins >> L.shift : 0;
     size_t o = kBatchHeader;
-    L.off_hist = o;    o += kBins * 4;  // the header, the histogram and the cursors start at zero
-    L.off_cursor = o;  o += kBins * 4;
+    L.off_hist = o;    o += bins * 4;  // the header, the histogram and the cursors start at zero
+    L.off_cursor = o;  o += bins * 4;
     L.off_bins = o;    o = align_up(o + npairs * 2, 256);
     L.off_queue = o;   o = align_up(o + npairs * 8, 256);
     L.total = o;
@@ -175,17 +189,39 @@ __device__ __forceinline__ uint32_t device_bucket(const uint32_t* el, const Pair
 
 __host__ __device__ constexpr bool is_stream_tech(uint8_t t) { return t >= kHash1024 && t < kTechCodes; }
 
-// Each pair's bin, the bins' histogram and the parts' total cost.  A stream
-// technique falls back to merge for a pair whose larger set has 2^32 - 1024
-// elements or more (stream positions are 32-bit).
+// A pair's key and cost.  A stream technique falls back to merge for a pair whose
+// larger set has 2^32 - 1024 elements or more (stream positions are 32-bit).
+__device__ __forceinline__ uint32_t pair_key(const uint32_t* __restrict__ el, const uint64_t* __restrict__ off,
+                                             const uint32_t* __restrict__ pairs, uint64_t p, uint32_t k,
+                                             const TechTable& table, int forced, unsigned char* header,
+                                             uint64_t& cost) {
+    const uint32_t a = pairs[2 * p], b = pairs[2 * p + 1];
+    cost = 0;
+    uint32_t larger = 0;
+    uint8_t t = kMerge;
+    if (a >= k || b >= k) {
+        record_error(reinterpret_cast<uint32_t*>(header), SI_ERR_INVALID_INPUT, 50, static_cast<uint32_t>(p));
+    } else {
+        const PairSets ps = pair_sets(off, a, b);
+        t = forced >= 0 ? static_cast<uint8_t>(forced) : table.t[device_bucket(el, ps)];
+        if (t >= kTechCodes || (is_stream_tech(t) && max(ps.na, ps.nb) >= kMaxStream)) t = kMerge;
+        cost = t == kSearch ? search_cost(min(ps.na, ps.nb), max(ps.na, ps.nb)) : ps.na + ps.nb;
+        larger = ps.na > ps.nb ? a : b;
+    }
+    return uint32_t(t) << 12 | uint32_t(is_stream_tech(t)) << 11 | (127u - cost_class(cost)) << 4 |
+           (larger * 0x9e3779b1u) >> 28;
+}
+__host__ __device__ constexpr uint32_t key_part(uint32_t key) { return (key >> 11) & 1u; }
+
+// Each pair's key, the bins' histogram and the parts' total cost.
 __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
     const uint32_t* __restrict__ el, const uint64_t* __restrict__ off, const uint32_t* __restrict__ pairs,
-    uint64_t npairs, uint32_t k, const __grid_constant__ TechTable table, int forced, uint16_t* __restrict__ bins,
-    uint32_t* __restrict__ hist, unsigned char* header) {
+    uint64_t npairs, uint32_t k, const __grid_constant__ TechTable table, int forced, uint32_t shift,
+    uint16_t* __restrict__ bins, uint32_t* __restrict__ hist, unsigned char* header) {
     __shared__ uint32_t s_hist[kBins];
     __shared__ unsigned long long s_cost[2];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads) s_hist[i] = 0;
+    for (uint32_t i = threadIdx.x; i < kBins >> shift; i += kKeyThreads) s_hist[i] = 0;
     if (threadIdx.x < 2) s_cost[threadIdx.x] = 0;
     __syncthreads();
     const uint64_t p0 = uint64_t(blockIdx.x) * kKeyThreads * kKeyPairs + threadIdx.x;
@@ -194,24 +230,11 @@ __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
     for (uint32_t u = 0; u < kKeyPairs; ++u) {
         const uint64_t p = p0 + u * kKeyThreads;
         if (p >= npairs) continue;
-        const uint32_t a = pairs[2 * p], b = pairs[2 * p + 1];
-        uint64_t cost = 0;
-        uint32_t larger = 0;
-        uint8_t t = kMerge;
-        if (a >= k || b >= k) {
-            record_error(reinterpret_cast<uint32_t*>(header), SI_ERR_INVALID_INPUT, 50, static_cast<uint32_t>(p));
-        } else {
-            const PairSets ps = pair_sets(off, a, b);
-            t = forced >= 0 ? static_cast<uint8_t>(forced) : table.t[device_bucket(el, ps)];
-            if (t >= kTechCodes || (is_stream_tech(t) && max(ps.na, ps.nb) >= kMaxStream)) t = kMerge;
-            cost = t == kSearch ? search_cost(min(ps.na, ps.nb), max(ps.na, ps.nb)) : ps.na + ps.nb;
-            larger = ps.na > ps.nb ? a : b;
-        }
-        const uint32_t part = is_stream_tech(t) ? 1u : 0u;
-        const uint32_t bin = part << 11 | (127u - cost_class(cost)) << 4 | (larger * 0x9e3779b1u) >> 28;
-        bins[p] = static_cast<uint16_t>(bin | uint32_t(t) << 12);
-        atomicAdd(&s_hist[bin], 1u);
-        part_cost[part] += cost;
+        uint64_t cost;
+        const uint32_t key = pair_key(el, off, pairs, p, k, table, forced, header, cost);
+        bins[p] = static_cast<uint16_t>(key);
+        atomicAdd(&s_hist[key_bin(key, shift)], 1u);
+        part_cost[key_part(key)] += cost;
     }
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
@@ -219,16 +242,66 @@ __global__ void __launch_bounds__(kKeyThreads) batch_keys_kernel(
         if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_cost[part], static_cast<unsigned long long>(c));
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads)
+    for (uint32_t i = threadIdx.x; i < kBins >> shift; i += kKeyThreads)
         if (s_hist[i]) atomicAdd(hist + i, s_hist[i]);
     if (threadIdx.x < 2 && s_cost[threadIdx.x])
         atomicAdd(reinterpret_cast<unsigned long long*>(header + kPartCost) + threadIdx.x, s_cost[threadIdx.x]);
 }
 
+// The queue of up to kPlanMost pairs, by one CTA.
+__global__ void __launch_bounds__(kPlanThreads) batch_plan_kernel(
+    const uint32_t* __restrict__ el, const uint64_t* __restrict__ off, const uint32_t* __restrict__ pairs,
+    uint32_t npairs, uint32_t k, const __grid_constant__ TechTable table, int forced, uint64_t* __restrict__ queue,
+    unsigned char* header) {
+    __shared__ __align__(8) uint32_t s_hist[kBins / 2];  // the bins' pairs, then where the next pair of each goes
+    __shared__ uint32_t s_warp[kPlanThreads / 32];
+    __shared__ unsigned long long s_cost[2];
+    constexpr uint32_t kPer = kBins / 2 / kPlanThreads;
+    static_assert(kPer == 2, "a thread scans 8 bytes of the histogram");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint2* h2 = reinterpret_cast<uint2*>(s_hist);
+    h2[tid] = make_uint2(0u, 0u);
+    if (tid < 2) s_cost[tid] = 0;
+    __syncthreads();
+    uint32_t key[kPlanPairs];
+    uint64_t part_cost[2] = {0, 0};
+#pragma unroll
+    for (uint32_t u = 0; u < kPlanPairs; ++u) {
+        const uint32_t p = u * kPlanThreads + tid;
+        key[u] = ~0u;
+        if (p >= npairs) continue;
+        uint64_t cost;
+        key[u] = pair_key(el, off, pairs, p, k, table, forced, header, cost);
+        atomicAdd(&s_hist[key_bin(key[u], 1)], 1u);
+        part_cost[key_part(key[u])] += cost;
+    }
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+        const uint64_t c = warp_sum_u64(part_cost[part]);
+        if (lane == 0 && c) atomicAdd(&s_cost[part], static_cast<unsigned long long>(c));
+    }
+    __syncthreads();
+    const uint2 v = h2[tid];
+    const uint32_t sum = v.x + v.y, incl = warp_inclusive_scan(sum);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t o = incl - sum;
+    for (uint32_t w = 0; w < warp; ++w) o += s_warp[w];
+    h2[tid] = make_uint2(o, o + v.x);
+    if (tid < 2) reinterpret_cast<unsigned long long*>(header + kPartCost)[tid] = s_cost[tid];
+    if (tid == kPlanThreads / 2) *reinterpret_cast<uint32_t*>(header + kNFirst) = o;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t u = 0; u < kPlanPairs; ++u)
+        if (key[u] != ~0u)
+            queue[atomicAdd(&s_hist[key_bin(key[u], 1)], 1u)] = uint64_t(key[u]) << 32 | (u * kPlanThreads + tid);
+}
+
 // The queue: every pair (its key in bits 32.., its index below) at its bin's
 // offset.  A CTA scans the histogram itself and reserves room in each bin once;
 // the order within a bin does not matter.
-__global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t* bins, uint64_t npairs,
+__global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t* bins, uint64_t npairs, uint32_t shift,
                                                                   const uint32_t* hist, uint32_t* __restrict__ cursor,
                                                                   uint64_t* __restrict__ queue,
                                                                   unsigned char* header) {
@@ -236,14 +309,14 @@ __global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t
     __shared__ uint32_t s_count[kBins];  // this CTA's pairs of the bin
     __shared__ uint32_t s_warp[kKeyThreads / 32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads) s_count[i] = 0;
+    for (uint32_t i = threadIdx.x; i < kBins >> shift; i += kKeyThreads) s_count[i] = 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the bins and their histogram
     constexpr uint32_t kPer = kBins / kKeyThreads;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t v[kPer], sum = 0;
 #pragma unroll
     for (uint32_t q = 0; q < kPer; ++q) {
-        v[q] = hist[threadIdx.x * kPer + q];
+        v[q] = threadIdx.x * kPer + q < kBins >> shift ? hist[threadIdx.x * kPer + q] : 0u;
         sum += v[q];
     }
     const uint32_t incl = warp_inclusive_scan(sum);
@@ -262,18 +335,18 @@ __global__ void __launch_bounds__(kKeyThreads) batch_queue_kernel(const uint16_t
     for (uint32_t u = 0; u < kKeyPairs; ++u) {
         const uint64_t p = p0 + u * kKeyThreads;
         key[u] = p < npairs ? bins[p] : ~0u;
-        if (key[u] != ~0u) atomicAdd(&s_count[key_bin(key[u])], 1u);
+        if (key[u] != ~0u) atomicAdd(&s_count[key_bin(key[u], shift)], 1u);
     }
     __syncthreads();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint32_t*>(header + kNFirst) = s_off[kBins / 2];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<uint32_t*>(header + kNFirst) = s_off[(kBins >> shift) / 2];
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < kBins; i += kKeyThreads)
+    for (uint32_t i = threadIdx.x; i < kBins >> shift; i += kKeyThreads)
         if (s_count[i]) s_off[i] += atomicAdd(cursor + i, s_count[i]);
     __syncthreads();
 #pragma unroll
     for (uint32_t u = 0; u < kKeyPairs; ++u)
         if (key[u] != ~0u)
-            queue[atomicAdd(&s_off[key_bin(key[u])], 1u)] = uint64_t(key[u]) << 32 | (p0 + u * kKeyThreads);
+            queue[atomicAdd(&s_off[key_bin(key[u], shift)], 1u)] = uint64_t(key[u]) << 32 | (p0 + u * kKeyThreads);
 }
 
 // ------------------------------------------------------ per-warp techniques --
@@ -899,7 +972,7 @@ si_status batch_launch(const uint32_t* d_elements, const uint64_t* d_offsets, ui
     const BatchLayout L = batch_layout(npairs);
     if (ws_bytes < L.total) return SI_ERR_WORKSPACE_TOO_SMALL;
     unsigned char* w = static_cast<unsigned char*>(ws);
-    SI_CUDA_TRY(cudaMemsetAsync(w, 0, d_subset || npairs == 0 ? kBatchHeader : L.off_bins, stream));
+    SI_CUDA_TRY(cudaMemsetAsync(w, 0, d_subset ? kBatchHeader : L.off_bins, stream));
     if (npairs == 0) return SI_OK;
     uint64_t* queue = reinterpret_cast<uint64_t*>(w + L.off_queue);
     BatchParams prm;
@@ -918,14 +991,20 @@ si_status batch_launch(const uint32_t* d_elements, const uint64_t* d_offsets, ui
         uint32_t* hist = reinterpret_cast<uint32_t*>(w + L.off_hist);
         uint32_t* cursor = reinterpret_cast<uint32_t*>(w + L.off_cursor);
         uint16_t* bins = reinterpret_cast<uint16_t*>(w + L.off_bins);
-        const unsigned g = static_cast<unsigned>((npairs + kKeyThreads * kKeyPairs - 1) / (kKeyThreads * kKeyPairs));
-        batch_keys_kernel<<<g, kKeyThreads, 0, stream>>>(d_elements, d_offsets, d_pairs, npairs, k, table, forced,
-                                                         bins, hist, w);
-        SI_LAUNCH_CHECK("batch_keys_kernel");
-        const si_status st = launch_dependent(batch_queue_kernel, dim3(g), dim3(kKeyThreads), 0, stream,
-                                              static_cast<const uint16_t*>(bins), npairs,
-                                              static_cast<const uint32_t*>(hist), cursor, queue, w);
-        if (st != SI_OK) return st;
+        if (npairs <= kPlanMost) {
+            batch_plan_kernel<<<1, kPlanThreads, 0, stream>>>(d_elements, d_offsets, d_pairs,
+                                                              static_cast<uint32_t>(npairs), k, table, forced, queue, w);
+            SI_LAUNCH_CHECK("batch_plan_kernel");
+        } else {
+            const unsigned g = static_cast<unsigned>((npairs + kKeyThreads * kKeyPairs - 1) / (kKeyThreads * kKeyPairs));
+            batch_keys_kernel<<<g, kKeyThreads, 0, stream>>>(d_elements, d_offsets, d_pairs, npairs, k, table, forced,
+                                                             L.shift, bins, hist, w);
+            SI_LAUNCH_CHECK("batch_keys_kernel");
+            const si_status st = launch_dependent(batch_queue_kernel, dim3(g), dim3(kKeyThreads), 0, stream,
+                                                  static_cast<const uint16_t*>(bins), npairs, L.shift,
+                                                  static_cast<const uint32_t*>(hist), cursor, queue, w);
+            if (st != SI_OK) return st;
+        }
     }
     const BatchOccupancy occ = batch_occupancy();
     const int search_per_sm = occ.search, stream_per_sm = occ.stream;

@@ -285,3 +285,12 @@ def test_misi_workspace_grows_with_the_tile():
             sizes = [L.si_misi_workspace_size(R(0, k // 2 if cross else k), R(k // 2, k) if cross else R(0, k), int(t))
                      for k in (2, 31, 32, 33, 1000, 8192, 16000, 16383, 16384, 16385, 16400, 17000, 40000)]
             assert sizes == sorted(sizes)
+
+
+def test_batch_workspace_is_two_words_a_pair():
+    """A batch's workspace: no more than two 64-bit words a pair and two blocks
+    of 256 bytes, and no less for more pairs."""
+    sizes = [si.lib.si_batch_workspace_size(n) for n in range(20000)]
+    assert sizes == sorted(sizes)
+    for n, size in enumerate(sizes):
+        assert size <= 512 + 2 * ((8 * n + 255) // 256 * 256)

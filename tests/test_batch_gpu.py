@@ -273,3 +273,18 @@ def test_merge_ends_on_padded_sets(cuda, pad):
     col = collection(ds.elements, ds.offsets, top)
     np.testing.assert_array_equal(count(col, pairs, "ip"), want)
     np.testing.assert_array_equal(count(col, pairs[-1:], "ip"), want[-1:])
+
+
+@pytest.mark.parametrize("npairs", [2, 43, 1023, 1024, 1025, 3071, 3072, 3073, 8192, 8193])
+def test_queue_by_one_cta(cuda, npairs):
+    """Batch sizes around the threads of the CTA that orders a small batch and the
+    most pairs it takes: pairs for whole CTAs and for warps, in one and in both
+    parts of the queue."""
+    ds = crafted_pool(7)
+    k = ds.cardinality
+    col = collection(ds.elements, ds.offsets, ds.universe)
+    pairs = np.random.default_rng(npairs).integers(0, k, (npairs, 2)).astype(np.uint32)
+    want = oracle.pairs(ds.elements, ds.offsets, k, pairs)
+    mixed = bytes(np.random.default_rng(5).integers(0, 6, 1024).astype(np.uint8))
+    for tech, table in (("ip", None), ("hi", None), ("auto", None), ("auto", mixed)):
+        np.testing.assert_array_equal(count(col, pairs, tech, table), want)
