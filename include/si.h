@@ -214,8 +214,9 @@ si_status si_validate_sorted(const uint32_t* d_x, uint64_t n, uint32_t* d_flag, 
  * them at once: BITMAP when the values of the tile's sets span at most 2^20
  * (512 sets at a time), 2^21 (256) or 2^22 (128); HI, whose matrix is indexed
  * by a hash table, unless a set holds more than 2^20 elements of a wider span.
- * Other tiles, and up to 128 (HI: 1024) sets of at most 64 elements, are probed
- * pair by pair.
+ * Other tiles, and tiles of sets so small that their pairs take few probes each
+ * (the mean of a pair's smaller size below 2 to 36, by the number of sets), are
+ * probed pair by pair.
  */
 typedef struct si_set_range { uint32_t start, end; } si_set_range;
 size_t si_misi_workspace_size(si_set_range A, si_set_range B, si_technique t);

@@ -204,12 +204,19 @@ __device__ __forceinline__ uint32_t first_not_larger(const uint64_t* keys, uint3
     return lo;
 }
 
+// Adds a warp's partner elements to the tile's; all its lanes make the call.
+__device__ __forceinline__ void add_work(uint64_t work, unsigned char* header) {
+    const uint64_t w = warp_sum_u64(work);
+    if ((threadIdx.x & 31) == 0 && w) atomicAdd(reinterpret_cast<unsigned long long*>(header + kMisiWork), w);
+}
+
 // Per row: where its partners start in the other side's sorted list, and how
 // many work items its partners' elements make.  P: exclusive prefix sums.
 __global__ void misi_rows_kernel(const uint64_t* __restrict__ keys, uint32_t nA, uint32_t nB, bool self,
                                  ItemUnit rule, const uint64_t* __restrict__ P, uint32_t* __restrict__ cs,
-                                 uint64_t* __restrict__ nseg) {
+                                 uint64_t* __restrict__ nseg, unsigned char* header) {
     const uint32_t rows = nA + nB;
+    uint64_t all = 0;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r <= rows; r += gridDim.x * blockDim.x) {
         if (r == rows) {
             nseg[r] = 0;
@@ -237,7 +244,9 @@ __global__ void misi_rows_kernel(const uint64_t* __restrict__ keys, uint32_t nA,
         const uint64_t work = Pt[nt] - Pt[c];
         const uint64_t unit = item_unit(rule, size);
         nseg[r] = work ? (work + unit - 1) / unit : 0;
+        all += work;
     }
+    add_work(all, header);
 }
 
 // The plan of small collections in two kernels.  Every set i compares itself
@@ -347,6 +356,7 @@ __global__ void __launch_bounds__(kOrderThreads) misi_order_kernel(
     const uint32_t n = nA + nB, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t* totals = reinterpret_cast<const uint64_t*>(header + kMisiTotals);
     const uint32_t i = blockIdx.x * kOrderThreads + tid;
+    uint64_t work = 0;
     if (i < n) {
         const bool iA = i < nA;
         const uint32_t local = iA ? i : i - nA, id = (iA ? a_start : b_start) + local;
@@ -361,11 +371,12 @@ __global__ void __launch_bounds__(kOrderThreads) misi_order_kernel(
         if (rank + 1 == (iA ? nA : nB)) Ps[rank + 1] = sum + size;
         // partners: the sets after it of its own side, or the other side's from the first no larger one
         const uint32_t c = self ? rank + 1 : static_cast<uint32_t>(other[i]) & mask;
-        const uint64_t work = self ? totals[0] - sum - size : totals[iA ? 1 : 0] - (other[i] >> kRankBits);
+        work = self ? totals[0] - sum - size : totals[iA ? 1 : 0] - (other[i] >> kRankBits);
         cs[row] = c;
         const uint64_t unit = item_unit(rule, size);
         nseg[row] = work ? (work + unit - 1) / unit : 0;
     }
+    add_work(work, header);
     __syncthreads();
     if (tid == 0) {
         __threadfence();
@@ -833,7 +844,7 @@ si_status misi_tile(const uint32_t* d_elements, const uint64_t* d_offsets, si_te
             SI_CUDA_TRY(cub::DeviceScan::InclusiveSum(cub_tmp, tmp, sizes + L.nA + 1, P + L.nA + 2,
                                                       static_cast<int>(L.nB), stream));
         }
-        misi_rows_kernel<<<g, 256, 0, stream>>>(keys, L.nA, L.nB, L.self, rule, P, cs, nseg);
+        misi_rows_kernel<<<g, 256, 0, stream>>>(keys, L.nA, L.nB, L.self, rule, P, cs, nseg, w);
         SI_LAUNCH_CHECK("misi_rows_kernel");
         tmp = L.cub_bytes;
         SI_CUDA_TRY(cub::DeviceScan::ExclusiveSum(cub_tmp, tmp, nseg, items, static_cast<int>(L.rows + 1), stream));

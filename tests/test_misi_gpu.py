@@ -313,3 +313,30 @@ def test_plan_totals_of_split_warps(cuda, n_a, n_b):
     want = np.array([[len(np.intersect1d(sets[a], sets[n_a + b])) for b in range(n_b)] for a in range(n_a)])
     for tech in ("bitmap", "hi", "obs"):
         np.testing.assert_array_equal(run(col, tech, (0, n_a), (n_a, k)).reshape(n_a, n_b), want)
+
+
+@pytest.mark.parametrize("tech,k,n_a,span,size", [
+    ("bitmap", 128, 0, 1 << 16, 65), ("bitmap", 129, 0, 1 << 16, 6), ("bitmap", 768, 0, 1 << 20, 6),
+    ("bitmap", 769, 0, 1 << 12, 2), ("bitmap", 1025, 0, 1 << 13, 1), ("bitmap", 1025, 0, (1 << 21) + 9, 2),
+    ("bitmap", 2049, 0, (1 << 22) - 9, 2), ("bitmap", 700, 100, 1 << 14, 4), ("bitmap", 16400, 40, 1 << 15, 1),
+    ("hi", 127, 0, 1 << 26, 512), ("hi", 47, 0, 1 << 26, 2048), ("hi", 600, 0, 1 << 14, 36), ("hi", 1024, 0, 1 << 22, 64),
+    ("hi", 1025, 0, 1 << 14, 23), ("hi", 2049, 0, 1 << 30, 8), ("hi", 4097, 0, 1 << 12, 5), ("hi", 800, 300, 1 << 12, 8),
+    ("hi", 16400, 40, 1 << 12, 5),
+])
+def test_matrix_or_probes(cuda, tech, k, n_a, span, size):
+    """Sets whose pairs take as many probes as the rule between the matrix and the
+    probe kernel allows, and one more: one side against itself, and (n_a) two
+    sides; rows sorted as well as ranked."""
+    rng = np.random.default_rng(k + size)
+    for n in (size, size + 1):
+        sets = [np.sort(rng.choice(span, n, replace=False)) if span < 1 << 16 else
+                np.unique(rng.integers(0, span, 2 * n + 8))[:n] for _ in range(k)]
+        ds, col = from_sets([s.astype(np.uint32) for s in sets], span)
+        if n_a:
+            got = run(col, tech, (0, n_a), (n_a, k))
+            pairs = np.stack(np.meshgrid(np.arange(n_a), np.arange(n_a, k), indexing="ij"), -1).reshape(-1, 2)
+            want = oracle.pairs(ds.elements, ds.offsets, k, pairs.astype(np.uint32))
+        else:
+            got = run(col, tech)
+            want = oracle.all_pairs(ds.elements, ds.offsets, k, ds.universe, "std")
+        np.testing.assert_array_equal(got, want)
