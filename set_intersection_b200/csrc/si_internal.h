@@ -95,11 +95,16 @@ si_status bm_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t 
 //   2^27, 1/16            204 (130)    155 (115)    210 (185)
 //   2^27, 1/32            192 (122)    147 (111)    139 (125)
 //   2^27, 1/64            187 (117)    141 (108)    110 (101)
-// A pair of one merge tile is one launch of ip: 3.8 us against 4.2 and more.
+// (uniform values).  A pair of one merge tile is one launch of ip: 3.8 us against
+// 4.2 and more.  Only counted, pairs up to 1.25 x 2^20 elements are merged too:
+// over six distributions (uniform, powers, clusters at twelve scales, runs of
+// 512, fractal) the larger set's 2^18, 2^20 and 3 x 2^19 elements take ip 5.1, 5.6
+// and 6.1 us, obs 5.8, 6.0 and 6.1, the worst distribution 1.4, 1.4 and 1.2 times
+// ip.  With elements out no distribution at these ratios takes obs longer than ip.
 inline si_technique sisi_auto(uint64_t nA, uint64_t nB, bool elements) {
     const uint64_t small = nA < nB ? nA : nB, large = nA < nB ? nB : nA, total = nA + nB;
     const uint64_t ratio = elements && total <= (1ull << 25) ? 16 : total <= (1ull << 27) ? 32 : 64;
-    if (total > (elements ? kIpOneTile : 1ull << 18) && small <= large / ratio) return SI_TECH_OBS;
+    if (total > (elements ? kIpOneTile : 5ull << 18) && small <= large / ratio) return SI_TECH_OBS;
     return total <= (1ull << 24) ? SI_TECH_IP : SI_TECH_BITMAP;
 }
 size_t obs_workspace_size(uint64_t nA, uint64_t nB);

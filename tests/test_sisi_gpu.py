@@ -377,3 +377,30 @@ def test_pair_call_in_a_graph(cuda, tech, n):
         assert int(count.item()) == want.size
         np.testing.assert_array_equal(out[:want.size].cpu().numpy().view(np.uint32), want)
         assert not out[want.size:].any()
+
+
+@pytest.mark.parametrize("total,ratio,spread", [
+    (total, ratio, spread) for total in (5184, 5185, 5 << 18, (5 << 18) + 1) for ratio in (16, 32, 64)
+    for spread in ("clusters", "runs")] + [((1 << 24) + 1, 16, "runs"), ((1 << 25) + 1, 32, "runs")])
+def test_auto_at_its_thresholds(cuda, total, ratio, spread):
+    """Pairs on both sides of the sizes and ratios at which the engine's choice
+    changes, with values that interpolation does not fit: clusters at twelve
+    scales, runs of 512 consecutive values at uneven distances."""
+    rng = np.random.default_rng(total + ratio)
+
+    def values(n):
+        while True:
+            m = n + n // 2 + 4096
+            if spread == "clusters":
+                v = (1 << 32) / 2.0 ** rng.integers(0, 8, m) * (0.8 + 0.19 * rng.random(m) ** 3)
+            else:
+                v = (rng.random(m // 512 + 1)[:, None] ** 2 * ((1 << 32) - 1024)).astype(np.int64) + np.arange(512)
+            v = np.unique(v.astype(np.uint32).ravel())
+            if v.size >= n:
+                return np.sort(rng.permutation(v)[:n])
+
+    small = total // (ratio + 1)
+    large = values(total - small)
+    for n in (small, small + 1):  # at the ratio, and below it
+        a = np.unique(np.concatenate([rng.choice(large, n // 2, replace=False), values(n)[: n - n // 2]]))
+        check(a, large, "auto")
