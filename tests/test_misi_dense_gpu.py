@@ -157,3 +157,35 @@ def test_dense_call_in_a_graph(cuda, dtype):
         out.fill_(3)
         g.replay()
         np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32), want)
+
+
+def wide_tile(k, values, sms):
+    """Whether the tensor-core path takes its 256 x 512 tile: the cheaper of the
+    two schedules, in units of a stage's MMAs."""
+    pairs, panels, stages = sms // 2, -(-k // 256), -(-values // 128)
+    cost = {}
+    for n in (1, 2):
+        columns = -(-panels // n)
+        tiles = sum(columns - i // n for i in range(panels))
+        whole = tiles // pairs * pairs
+        left = tiles - whole
+        cuts = max(1, min(pairs // left, stages // 16)) if left else 1
+        stage, out = (1.25 * stages, 18) if n == 1 else (2.1 * stages, 60)
+        cost[n] = whole // pairs * (stage + out)
+        if left:
+            cost[n] += stage / cuts + (1.5 * out if cuts > 1 else out)
+    return cost[2] < cost[1]
+
+
+@pytest.mark.parametrize("dtype", ["int8", "fp8"])
+@pytest.mark.parametrize("k,values", [(1400, 200001), (2050, 65536), (3601, 10001), (4609, 40010)])
+def test_wide_tile_edges(cuda, k, values, dtype):
+    """The 256 x 512 tile where the sets fill neither a row panel nor a column
+    panel: an odd number of row panels, whose last column panel lies half past
+    the matrix, tiles cut along K in two and six parts, whole tiles, and both; some
+    sets empty, some full, against the popcount kernel and the oracle on sampled
+    pairs.  (4300 sets over 65536 values take the narrow tile.)"""
+    import torch
+    assert wide_tile(k, values, torch.cuda.get_device_properties(0).multi_processor_count)
+    assert not wide_tile(4300, 65536, 148)
+    test_paired_tiles_edges(cuda, k, values, dtype)
