@@ -26,10 +26,12 @@
 //    (ip_group_kernel): once, with a decoupled look-back per group of tiles.
 //
 // A pair of one tile is a single launch of one CTA, which clears the header
-// itself.  Eight CTAs per SM hide each other's staging and searches, so a tile
-// has no warps of its own for them.  What bounds it: shared memory's banks (the
-// threads' reads are kVT / 2 words apart, 2.9 wavefronts a load; 79 % of the
-// LSU's data pipe) and issue slots (77 %) on large pairs, latency on small ones.
+// itself.  Eight CTAs per SM (the group kernel six) hide each other's staging and
+// searches, so a tile has no warps of its own for them.  What bounds it: counting
+// large pairs, shared memory's banks (the threads' reads are kVT / 2 words apart,
+// 2.9 wavefronts a load; 82 % of the LSU's data pipe) and issue slots (80 %); the
+// group kernel, at 57 % and 58 % of those, the latency of global memory; small
+// pairs, latency.
 //
 // Measured, device time with elements out / counts only (in brackets: a
 // persistent kernel with producer, consumer and output warps on tiles cut at
@@ -421,7 +423,8 @@ struct GroupMatches {
     uint16_t i0[kGroup][kIpThreads], before[kGroup][kIpThreads];
     uint32_t count[kGroup];
 };
-__global__ void __launch_bounds__(kIpThreads, kIpCtasPerSm) ip_group_kernel(
+constexpr int kIpGroupCtasPerSm = 6;  // 33 KiB of shared memory each
+__global__ void __launch_bounds__(kIpThreads, kIpGroupCtasPerSm) ip_group_kernel(
     const uint32_t* __restrict__ A, uint64_t nA, const uint32_t* __restrict__ B, uint64_t nB, const uint64_t* split,
     uint64_t nTiles, uint32_t* header, uint64_t* status, uint32_t* __restrict__ out, uint64_t out_cap,
     uint64_t* __restrict__ d_count) {
@@ -466,7 +469,6 @@ __global__ void __launch_bounds__(kIpThreads, kIpCtasPerSm) ip_group_kernel(
         }
         if (g >= gridDim.x) {  // the group before, gd
             const uint64_t gd = g - gridDim.x, td = gd * kGroup;
-            if (gd >= nGroups) break;
             if (warp == 0) {
                 const uint64_t p = gd > 0 ? look_back(status, gd, header) : 0;
                 if (lane == 0) {
