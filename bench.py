@@ -1070,7 +1070,7 @@ def run_ours_batch(args, rank: int, world: int):
         "config": {"workload": args.workload, "desc": w["desc"], "technique": tech, "k": k, "pairs": npairs,
                    "elements": int(el.size), "merge_elements": merge_elems,
                    "l2": f"pool {el.size * 4 >> 20} MiB > 126 MB L2; no flush",
-                   "graph": "one CUDA graph per step: key kernel, radix sort of the queue, the merge/search and "
+                   "graph": "one CUDA graph per step: the queue (a counting sort by its key and queue kernels), the merge/search and "
                             "hash/bitmap batch kernels",
                    "autotune_s": tune_s if table is not None else None,
                    "pairs_per_technique": codes_used,

@@ -208,6 +208,10 @@ si_status si_validate_sorted(const uint32_t* d_x, uint64_t n, uint32_t* d_flag, 
  * intersectPath), src/obs.cu:275-438 (warpBasedOBS / blockBasedOBS),
  * src/hi.cu:295-420 (warpBasedHI / blockBasedHI) and
  * src/bitmap_dynamic.cu:240-319.  t: IP, OBS, HI, BITMAP or AUTO (= BITMAP).
+ * IP and OBS run the same kernel here: merging a pair crosses the larger set at
+ * every element of the smaller one, and each crossing is found by a binary
+ * search of a bucket of the staged set, so the two names' times are one
+ * technique's.
  * MM and BITMAP_NAIVE are served by si_misi_dense (single-tile run only).
  * BITMAP and HI on 32 sets or more keep a value-major bit matrix of up to 512
  * sets in the workspace (64 MiB, HI 72) and count each partner against all of
@@ -326,12 +330,12 @@ si_status si_misi_dense(const uint32_t* d_elements, const uint64_t* d_offsets, u
  * Named cudaEvent pairs around the engine's own kernel launches, recorded on
  * the launching stream while enabled -- the counterpart of the reference's
  * DeviceTimer (include/device_timer.cuh:20-78), which wraps every phase of
- * every executable the same way.  Phase names: single pair "sisi_prepare",
- * "sisi_split", "sisi_tile", and for BITMAP with elements "sisi_scan",
- * "sisi_copy"; dense all pairs "mm_incidence", "mm_gemm",
+ * every executable the same way.  Phase names: single pair "sisi_split",
+ * "sisi_tile", and for BITMAP and HI with elements "sisi_copy"; dense all pairs "mm_incidence", "mm_gemm",
  * "naive_bitmaps", "naive_popcount"; all pairs of a tile "misi_plan",
- * "misi_slab" (bitmap), "misi_probe"; single pair by search "obs_search" and
- * "obs_compact" (adds up the counts, writes the elements); batched pairs "batch_plan", "batch_count".  The events come from a pool that
+ * "misi_slab" (bitmap, hi), "misi_probe"; single pair by search "obs_search" and
+ * "obs_compact" (adds up the counts, writes the elements); batched pairs
+ * "batch_plan", "batch_count"; "degree_stats".  The events come from a pool that
  * si_timer_reset refills, so a timed launch costs two event records.
  * si_timer_read synchronises on the recorded events and returns the summed
  * milliseconds and the number of launches of one phase.

@@ -60,7 +60,7 @@ namespace {
 constexpr int kBThreads = 256;           // 8 warps
 constexpr int kBWarps = kBThreads / 32;
 // Two kernels share the queue: the merge / search one (64 registers a thread,
-// 32 KiB of rings: 4 CTAs, 32 warps per SM; search is latency-bound and wants
+// 32 KiB of windows: 4 CTAs, 32 warps per SM; search is latency-bound and wants
 // the warps) and the stream one for hash and bitmap (80 registers, 8 KiB a
 // warp: 3 CTAs, 24 warps per SM).
 constexpr int kSearchCtasPerSm = 4;
@@ -387,7 +387,8 @@ __device__ __forceinline__ uint32_t window_count_le(const uint32_t* w, uint32_t 
 // A merge step is eight instructions, a round of some 500 elements of sets of
 // similar size about 330.  200000 pairs of 20000 sets of 32 .. 2^18 elements, all
 // merged (most of very different sizes): 1.35 warp instructions per element,
-// bound by issue (83 %) and the shared-memory pipe (88 %), 15.1 ms; rings of
+// 15.1 ms, bound by issue and the shared-memory pipe (100000 pairs of 10000 such
+// sets: 90 % of issue slots, 88 % of the LSU's data pipe); rings of
 // blocks with masked indexes and clamped ends took 2.7 and 21.6 ms.
 constexpr uint32_t kMergeWords = 2 * (kW + 32);  // per set: the window, then end marks that a lane's steps may run into
 __device__ uint32_t merge_pair(const uint32_t* A, uint64_t na, const uint32_t* B, uint64_t nb, uint32_t* win,

@@ -25,10 +25,10 @@
 // smaller sets', as in the probe kernel.
 //
 // Power-law collection (8192 sets, 45.6 M elements, 2^20 values), bitmap: the
-// launch takes 1.88 ms where the probe kernel takes 35.2 ms (builds 0.38 ms,
-// bound by the L2's atomics at 1.4e11 a second; probes 1.35 ms, bound by L2
+// launch takes 1.79 ms where the probe kernel takes 35.2 ms (builds 0.38 ms,
+// bound by the L2's atomics at 1.4e11 a second; probes 1.26 ms, bound by L2
 // gathers in the first groups and by latency in the last; clears 0.15 ms).
-// Hash, a cross tile of 1500 x 1500 of such sets: 0.94 ms against 8.05 ms.
+// Hash, a cross tile of 1500 x 1500 of such sets: 0.94-1.0 ms against 8.05 ms.
 // 64 sets of up to 512 elements: bitmap 46 us a call against 62, hash 60 and 62.
 #include <algorithm>
 
