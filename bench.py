@@ -106,7 +106,7 @@ def auto_engine(small, large, elements):
     through window bitmaps."""
     total = small + large
     ratio = 16 if elements and total <= 1 << 25 else 32 if total <= 1 << 27 else 64
-    if total > (IP_TILE if elements else 5 << 18) and small <= large // ratio:
+    if total > (IP_TILE if elements or small <= 256 else 5 << 18) and small <= large // ratio:
         return "obs"
     return "ip" if total <= 1 << 24 else "bitmap"
 

@@ -86,7 +86,8 @@ const char* si_last_error_string(void);
  * set in the larger one (samples of it in shared memory, then interpolation);
  * AUTO takes OBS when one set is 32 times larger than the other (16 times with
  * elements written and up to 2^25 elements in all, 64 times above 2^27; not for
- * pairs of up to 5184 elements, or 1.25 * 2^20 when only counted), else IP up to 2^24
+ * pairs of up to 5184 elements, nor of up to 1.25 * 2^20 when they are only
+ * counted and both sets have more than 256 elements), else IP up to 2^24
  * elements in all and BITMAP above.
  *
  * d_count: device uint64, receives |A ∩ B|.

@@ -69,6 +69,7 @@ private:
 // ---- one pair ----
 // Intersect path (si_sisi_ip.cu).
 constexpr uint64_t kIpOneTile = 192 * 27;  // a tile of ip: elements of both sets that one CTA merges
+constexpr uint64_t kObsOneChunk = 256;     // obs: elements of the smaller set that one CTA searches
 size_t ip_workspace_size(uint64_t nA, uint64_t nB);
 si_status ip_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t nB, uint64_t* d_count,
                   uint32_t* d_out, uint64_t out_cap, void* ws, size_t ws_bytes, cudaStream_t stream);
@@ -100,11 +101,12 @@ si_status bm_sisi(const uint32_t* dA, uint64_t nA, const uint32_t* dB, uint64_t 
 // over six distributions (uniform, powers, clusters at twelve scales, runs of
 // 512, fractal) the larger set's 2^18, 2^20 and 3 x 2^19 elements take ip 5.1, 5.6
 // and 6.1 us, obs 5.8, 6.0 and 6.1, the worst distribution 1.4, 1.4 and 1.2 times
-// ip.  With elements out no distribution at these ratios takes obs longer than ip.
+// ip; not so when one CTA can search and count (up to 256 elements, 3.0-4.3 us).
+// With elements out no distribution at these ratios takes obs longer than ip.
 inline si_technique sisi_auto(uint64_t nA, uint64_t nB, bool elements) {
     const uint64_t small = nA < nB ? nA : nB, large = nA < nB ? nB : nA, total = nA + nB;
     const uint64_t ratio = elements && total <= (1ull << 25) ? 16 : total <= (1ull << 27) ? 32 : 64;
-    if (total > (elements ? kIpOneTile : 5ull << 18) && small <= large / ratio) return SI_TECH_OBS;
+    if (total > (elements || small <= kObsOneChunk ? kIpOneTile : 5ull << 18) && small <= large / ratio) return SI_TECH_OBS;
     return total <= (1ull << 24) ? SI_TECH_IP : SI_TECH_BITMAP;
 }
 size_t obs_workspace_size(uint64_t nA, uint64_t nB);

@@ -381,7 +381,7 @@ def test_pair_call_in_a_graph(cuda, tech, n):
 
 @pytest.mark.parametrize("total,ratio,spread", [
     (total, ratio, spread) for total in (5184, 5185, 5 << 18, (5 << 18) + 1) for ratio in (16, 32, 64)
-    for spread in ("clusters", "runs")] + [((1 << 24) + 1, 16, "runs"), ((1 << 25) + 1, 32, "runs")])
+    for spread in ("clusters", "runs")] + [(256 * 33, 32, "runs"), (256 * 1025, 1024, "clusters"), ((1 << 24) + 1, 16, "runs"), ((1 << 25) + 1, 32, "runs")])
 def test_auto_at_its_thresholds(cuda, total, ratio, spread):
     """Pairs on both sides of the sizes and ratios at which the engine's choice
     changes, with values that interpolation does not fit: clusters at twelve
